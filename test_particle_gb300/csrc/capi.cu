@@ -188,13 +188,130 @@ bool build_field(int stype, DevField& f)
         f.iBessel = iBessel;
     } else if (stype == TP_SYS_MODESUM) {
         f.nmodes = (int)g.modes.size();
-        f.modes = (const tp_mode*)(f.nmodes ? dd0(g.m_modes, g.modes.data(), sizeof(tp_mode) * f.nmodes, s) : nullptr);
         f.B0 = g.mode_B0;
+        if (!g.fx_modes.empty()) {
+            const std::vector<int4>& tab = cosine_table();
+            f.fxm = (const fx::Mode*)dd0(g.m_fx, g.fx_modes.data(), sizeof(fx::Mode) * g.fx_modes.size(), s);
+            f.ctab = (const int4*)dd0(g.m_ctab, tab.data(), sizeof(int4) * tab.size(), s);
+            f.nfx = (int)g.fx_modes.size();
+            memcpy(f.fxs, g.fx_scale, sizeof(f.fxs));
+            if (!f.fxm || !f.ctab) return false;
+        } else {
+            f.modes = (const tp_mode*)(f.nmodes ? dd0(g.m_modes, g.modes.data(), sizeof(tp_mode) * f.nmodes, s)
+                                                : nullptr);
+        }
     } else if (stype != TP_SYS_TEST) {
         set_error(5, "wrong system type %d", stype);
         return false;
     }
     return g.status == 0;
+}
+
+// ---------------------------------------------------------------- fixed-point mode sum
+namespace {
+
+// Double-double arithmetic for the cosine table (error-free transformations).
+struct DD {
+    double h, l;
+};
+
+DD dd_add(DD a, DD b)
+{
+    const double s = a.h + b.h, v = s - a.h;
+    const double e = (a.h - (s - v)) + (b.h - v) + a.l + b.l;
+    const double h = s + e;
+    return {h, e - (h - s)};
+}
+
+DD dd_mul(DD a, DD b)
+{
+    const double p = a.h * b.h;
+    const double e = std::fma(a.h, b.h, -p) + (a.h * b.l + a.l * b.h);
+    const double h = p + e;
+    return {h, e - (h - p)};
+}
+
+DD dd_div(DD a, double b)
+{
+    const double q = a.h / b;
+    const double r = std::fma(-q, b, a.h) + a.l;
+    const double t = r / b, h = q + t;
+    return {h, t - (h - q)};
+}
+
+// sum of (-1)^k x^(2k + odd) / (2k + odd)!, |x| <= pi / 4
+DD dd_trig(DD x, int odd)
+{
+    const DD x2 = dd_mul(x, x);
+    DD t = odd ? x : DD{1.0, 0.0}, s = t;
+    for (int k = 1; k <= 14; k++) {
+        t = dd_div(dd_mul(t, x2), -(double)((2 * k - 1 + odd) * (2 * k + odd)));
+        s = dd_add(s, t);
+    }
+    return s;
+}
+
+int64_t dd_fixed(DD a, int q)
+{
+    return (int64_t)llrint(std::ldexp(a.h, q)) + (int64_t)llrint(std::ldexp(a.l, q));
+}
+
+}  // namespace
+
+// The cosine table of modesum_fx.cuh.
+const std::vector<int4>& cosine_table()
+{
+    static const std::vector<int4> tab = [] {
+        const DD pi = {3.141592653589793116, 1.2246467991473532e-16};
+        std::vector<int4> t(fx::kTab + 1);
+        for (int i = 0; i <= fx::kTab; i++) {
+            // an angle past pi / 4 from its complement
+            const int j = 2 * i <= fx::kTab ? i : fx::kTab - i;
+            const DD x = dd_div(dd_mul(pi, {(double)j, 0.0}), 2.0 * fx::kTab);
+            DD c = dd_trig(x, 0), s = dd_trig(x, 1);
+            if (j != i) std::swap(c, s);
+            const int64_t C = dd_fixed(c, 62);
+            const int64_t S = dd_fixed(dd_mul({2.0 * pi.h, 2.0 * pi.l}, s), 60);
+            t[i] = make_int4((int)(uint32_t)(C >> 31), (int)(C & 0x7fffffff), (int)(S >> 32),
+                             (int)((uint32_t)S >> 1));
+        }
+        return t;
+    }();
+    return tab;
+}
+
+// The mode table in fixed point: each component in units 2^-k with the sum of
+// its |amplitudes| below 2^62 units.  False where it does not fit: too many
+// modes (their sum would be less exact than in FP64), amplitudes that are not
+// finite or whose scale leaves the normal range.
+bool fixed_modes(const std::vector<tp_mode>& modes, std::vector<fx::Mode>& out, double scale[6])
+{
+    const size_t nm = modes.size();
+    if (nm == 0 || nm > (size_t)fx::kMaxModes) return false;
+    int ex[6];
+    auto amp = [&](size_t m, int k) { return k < 3 ? modes[m].amp_b[k] : modes[m].amp_e[k - 3]; };
+    for (int k = 0; k < 6; k++) {
+        double sum = 0.0;
+        for (size_t m = 0; m < nm; m++) sum += std::fabs(amp(m, k));
+        if (!std::isfinite(sum) || sum > 1e280 || (sum > 0.0 && sum < 1e-280)) return false;
+        int e = 0;
+        std::frexp(sum * (1.0 + 1e-6), &e);  // sum (1 + 1e-6) < 2^e
+        ex[k] = 62 - e;
+        scale[k] = std::ldexp(1.0, 1 - ex[k]);
+    }
+    out.assign((nm + fx::kChunk - 1) / fx::kChunk * fx::kChunk, fx::Mode{});
+    for (size_t m = 0; m < nm; m++) {
+        fx::Mode& o = out[m];
+        for (int k = 0; k < 3; k++) o.n[k] = modes[m].n[k];
+        o.ph = (uint32_t)modes[m].pad;
+        for (int k = 0; k < 6; k++) {
+            const int64_t a = llrint(std::ldexp(amp(m, k), ex[k] - 1));  // pairs of units
+            const int64_t ah = (a + (1ll << 29)) >> 30;
+            o.ah[k] = (int)ah;
+            o.al[k] = (int)(a - (ah << 30));
+        }
+    }
+    return true;
 }
 
 const void* dd0(Mirror& m, const void* h, size_t b, cudaStream_t s)
@@ -411,7 +528,8 @@ extern "C" int tp_set_modes(int nmodes, const tp_mode* modes, double Bz0)
     for (auto& m : g.modes)
         m.pad = (int)(unsigned int)(long long)llround(m.phase / (2.0 * M_PI) * 4294967296.0);
     g.mode_B0 = Bz0;
-    g.m_modes.dirty = true;
+    g.m_modes.dirty = g.m_fx.dirty = true;
+    if (!fixed_modes(g.modes, g.fx_modes, g.fx_scale)) g.fx_modes.clear();
     g.modes_gen++;
     return 0;
 }

@@ -321,8 +321,19 @@ __device__ __forceinline__ uint64_t fixed_frac64(double u)
     return __double2ull_rz(fr * 18446744073709551616.0);
 }
 
-// get_emf, src/emfields.c:32-60, specialised per system type (0..5).
-template <int SYS>
+// The six sums in fixed point (modesum_fx.cuh) as doubles.
+__device__ __forceinline__ void mode_sum_fixed(const DevField& f, const int4* tab, const uint64_t u[3], double e[6])
+{
+    int64_t s[6];
+    fx::mode_sum(f.fxm, f.nfx, tab, u, s);
+#pragma unroll
+    for (int k = 0; k < 6; k++) e[k] = (double)s[k] * f.fxs[k];
+}
+
+// get_emf, src/emfields.c:32-60, specialised per system type (0..5).  TAB: the
+// cosine table of the mode sum lies at the start of the block's dynamic shared
+// memory, else it is read from global memory.
+template <int SYS, bool TAB = false>
 __device__ __forceinline__ void emf64(const DevField& f, double x, double y, double z, double t,
                                       double e[6], int* status)
 {
@@ -399,6 +410,13 @@ __device__ __forceinline__ void emf64(const DevField& f, double x, double y, dou
         uint64_t ux = fixed_frac64((x - f.xmin) / (f.xmax - f.xmin));
         uint64_t uy = fixed_frac64((y - f.ymin) / (f.ymax - f.ymin));
         uint64_t uz = fixed_frac64((z - f.zmin) / (f.zmax - f.zmin));
+        if (f.fxm) {
+            extern __shared__ int4 s_ctab[];
+            const uint64_t u[3] = {ux, uy, uz};
+            mode_sum_fixed(f, TAB ? s_ctab : f.ctab, u, e);
+            e[2] = f.B0 + e[2];
+            return;
+        }
         double b0 = 0.0, b1 = 0.0, b2 = 0.0, e0 = 0.0, e1 = 0.0, e2 = 0.0;
         for (int m = 0; m < f.nmodes; m++) {
             const tp_mode& md = f.modes[m];

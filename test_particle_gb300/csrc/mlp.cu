@@ -80,17 +80,31 @@ __device__ __forceinline__ uint64_t mix64(uint64_t z)
 
 // Uniform positions (32-bit fixed point per axis) and the exact FP64 mode-sum
 // field there (the plane-wave sum of fields_fp64.cuh in the same phase form).
-__global__ void samples_kernel(uint64_t seed, long long first, int n, const tp_mode* __restrict__ modes,
-                               int nmodes, double B0z, uint32_t* __restrict__ U, float* __restrict__ T)
+__global__ void __launch_bounds__(128) samples_kernel(uint64_t seed, long long first, int n, DevField f,
+                                                      uint32_t* __restrict__ U, float* __restrict__ T)
 {
+    __shared__ int4 tab[fx::kTab + 1];
+    if (f.fxm) {
+        for (int k = threadIdx.x; k <= fx::kTab; k += blockDim.x) tab[k] = f.ctab[k];
+        __syncthreads();
+    }
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     uint64_t id = (uint64_t)(first + i);
     uint32_t u[3];
     for (int k = 0; k < 3; k++) u[k] = (uint32_t)(mix64(seed ^ (id * 3 + k) * 0xD1342543DE82EF95ull) >> 32);
     double b[3] = {0, 0, 0}, e[3] = {0, 0, 0};
-    for (int m = 0; m < nmodes; m++) {
-        const tp_mode& md = modes[m];
+    if (f.fxm) {
+        const uint64_t u64[3] = {(uint64_t)u[0] << 32, (uint64_t)u[1] << 32, (uint64_t)u[2] << 32};
+        int64_t s[6];
+        fx::mode_sum(f.fxm, f.nfx, tab, u64, s);
+        for (int k = 0; k < 3; k++) {
+            b[k] = (double)s[k] * f.fxs[k];
+            e[k] = (double)s[3 + k] * f.fxs[3 + k];
+        }
+    }
+    for (int m = 0; m < (f.fxm ? 0 : f.nmodes); m++) {
+        const tp_mode& md = f.modes[m];
         uint64_t ph = (uint64_t)(int64_t)md.n[0] * ((uint64_t)u[0] << 32) +
                       (uint64_t)(int64_t)md.n[1] * ((uint64_t)u[1] << 32) +
                       (uint64_t)(int64_t)md.n[2] * ((uint64_t)u[2] << 32) +
@@ -101,7 +115,7 @@ __global__ void samples_kernel(uint64_t seed, long long first, int n, const tp_m
             e[k] += md.amp_e[k] * c;
         }
     }
-    b[2] += B0z;
+    b[2] += f.B0;
     for (int k = 0; k < 3; k++) {
         U[3 * i + k] = u[k];
         T[6 * i + k] = (float)b[k];
@@ -555,8 +569,7 @@ extern "C" int tp_mlp_train(long long nsamples, int batch, int epochs, double lr
         !cuda_ok(cudaMalloc(&dT, sizeof(float) * 6 * (size_t)nsamples), "train t")) return -1;
     for (long long off = 0; off < nsamples; off += 1 << 22) {
         int cnt = (int)std::min<long long>(1 << 22, nsamples - off);
-        samples_kernel<<<(cnt + 127) / 128, 128, 0, s>>>(seed, off, cnt, f.modes, f.nmodes, f.B0,
-                                                         dU + 3 * off, dT + 6 * off);
+        samples_kernel<<<(cnt + 127) / 128, 128, 0, s>>>(seed, off, cnt, f, dU + 3 * off, dT + 6 * off);
     }
     // output normalisation from the training targets
     {

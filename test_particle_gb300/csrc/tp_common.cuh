@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include "../../include/tp_types.h"
+#include "modesum_fx.cuh"
 
 namespace tp {
 
@@ -36,6 +37,13 @@ struct DevField {
     // plane-wave mode sum
     int nmodes;
     const tp_mode *modes;
+    // the same in fixed point (null: the table is outside its range, and the
+    // sum is taken in FP64): modes padded to whole chunks, the scale of each
+    // component (a power of two), the cosine table
+    const fx::Mode *fxm;
+    int nfx;
+    double fxs[6];
+    const int4 *ctab;
 };
 
 // Output / scratch buffers of one tracking launch.

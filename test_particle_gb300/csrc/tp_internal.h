@@ -41,16 +41,19 @@ struct Ctx {
     int compact_steps = -1;       // open-boundary segment length (0: off, -1: automatic)
     std::vector<tp_mode> modes;
     double mode_B0 = 1.0;
+    // the mode table in fixed point (empty: outside its range) and its scales
+    std::vector<fx::Mode> fx_modes;
+    double fx_scale[6] = {0, 0, 0, 0, 0, 0};
     long modes_gen = 0;
     // mirrors of the reference's host grids
     Mirror m_bc_f, m_ba_f, m_bb_f, m_ec_f, m_ea_f, m_eb_f, m_vc_f, m_va_f, m_vb_f;
     Mirror m_bc_d, m_ba_d, m_bb_d, m_ec_d, m_ea_d, m_eb_d, m_vc_d, m_va_d, m_vb_d;
-    Mirror m_cfg, m_modes;
+    Mirror m_cfg, m_modes, m_fx, m_ctab;
     std::vector<Mirror*> all_mirrors()
     {
         return {&m_bc_f, &m_ba_f, &m_bb_f, &m_ec_f, &m_ea_f, &m_eb_f, &m_vc_f, &m_va_f, &m_vb_f,
                 &m_bc_d, &m_ba_d, &m_bb_d, &m_ec_d, &m_ea_d, &m_eb_d, &m_vc_d, &m_va_d, &m_vb_d,
-                &m_cfg, &m_modes};
+                &m_cfg, &m_modes, &m_fx, &m_ctab};
     }
     // exact energy-bin thresholds on the device
     int thr_nbins = 0;
@@ -77,6 +80,8 @@ bool build_field(int stype, DevField& f);
 bool build_field_points(DevField& f);
 namespace mixed { struct MixField; }
 bool build_mixfield(int stype, mixed::MixField& mf, int* nmodes_out);
+const std::vector<int4>& cosine_table();
+bool fixed_modes(const std::vector<tp_mode>& modes, std::vector<fx::Mode>& out, double scale[6]);
 const void* dd0(Mirror& m, const void* h, size_t b, cudaStream_t s);
 bool ensure_thresholds(int nbins);
 bool compute_thresholds(int nbins, double lmin, double lde, std::vector<double>& thr);

@@ -19,14 +19,14 @@ struct P64 {
 };
 
 // tracking_wirz, src/tracking.c:749-892 (c0_norm = 1)
-template <int SYS>
+template <int SYS, bool TAB = false>
 __device__ __forceinline__ void wirz(const DevField& f, P64& p, double dt, int* status)
 {
     const double cm = f.charge_mass;
     double e[6];
     double t0 = p.t;
     double gama = sqrt(1.0 + p.ux * p.ux + p.uy * p.uy + p.uz * p.uz);
-    emf64<SYS>(f, p.x, p.y, p.z, t0, e, status);
+    emf64<SYS, TAB>(f, p.x, p.y, p.z, t0, e, status);
     double Btot = sqrt(e[0] * e[0] + e[1] * e[1] + e[2] * e[2]);
     double iBtot = 1.0 / Btot;
     double dth = dt * 0.5;
@@ -57,7 +57,7 @@ __device__ __forceinline__ void wirz(const DevField& f, P64& p, double dt, int* 
     double px = p.x + h0 * tmp1 + hp0 * tmp2 + hr0 * tmp3;
     double py = p.y + h1 * tmp1 + hp1 * tmp2 + hr1 * tmp3;
     double pz = p.z + h2 * tmp1 + hp2 * tmp2 + hr2 * tmp3;
-    emf64<SYS>(f, px, py, pz, t0 + dth, e, status);
+    emf64<SYS, TAB>(f, px, py, pz, t0 + dth, e, status);
     Btot = sqrt(e[0] * e[0] + e[1] * e[1] + e[2] * e[2]);
     iBtot = 1.0 / Btot;
     h0 = e[0] * iBtot; h1 = e[1] * iBtot; h2 = e[2] * iBtot;
@@ -145,7 +145,7 @@ __device__ __forceinline__ int energy_bin(const double* thr, int nbins, double u
 
 // calc_diff_coeff, src/diagnostics.c:659-705 (pow(v, 2) taken as v * v).
 // Output order: drr, dxx, dyy, dzz, dpp, duu, daa, dee.
-template <int SYS>
+template <int SYS, bool TAB = false>
 __device__ __forceinline__ void calc_diff(const DevField& f, const P64& p0, const P64& p,
                                           double dt, double o[8], int* status)
 {
@@ -160,8 +160,8 @@ __device__ __forceinline__ void calc_diff(const DevField& f, const P64& p0, cons
     double dg = gamma - gamma0;
     double dee = dg * dg / t;
     double e[6], e0[6];
-    emf64<SYS>(f, p.x, p.y, p.z, p.t, e, status);
-    emf64<SYS>(f, p0.x, p0.y, p0.z, p0.t, e0, status);
+    emf64<SYS, TAB>(f, p.x, p.y, p.z, p.t, e, status);
+    emf64<SYS, TAB>(f, p0.x, p0.y, p0.z, p0.t, e0, status);
     double abs_b = sqrt(e[0] * e[0] + e[1] * e[1] + e[2] * e[2]);
     double abs_u = sqrt(p.ux * p.ux + p.uy * p.uy + p.uz * p.uz);
     double mu = (e[0] * p.ux + e[1] * p.uy + e[2] * p.uz) / (abs_b * abs_u);
@@ -221,10 +221,16 @@ __device__ __forceinline__ void block_diff_sum(const double sg[8], double* red, 
 // (every einterval steps for the spectrum, every 100 for the diffusion sums)
 // are block-uniform and reduce through shared memory.
 template <int SYS>
-__global__ void __launch_bounds__(kBlock) track_kernel(DevField f, TrackBufs b, TrackParams q)
+__global__ void __launch_bounds__(kBlock, SYS == TP_SYS_MODESUM ? 4 : 1) track_kernel(DevField f, TrackBufs b, TrackParams q)
 {
     __shared__ double red[(kBlock / 32) * 8];
     __shared__ unsigned int hist[kMaxSmemBins];
+    constexpr bool kTab = SYS == TP_SYS_MODESUM;
+    if (kTab && f.fxm) {  // the cosine table of the mode sum, once per block
+        extern __shared__ int4 s_ctab[];
+        for (int k = threadIdx.x; k <= fx::kTab; k += blockDim.x) s_ctab[k] = f.ctab[k];
+        __syncthreads();
+    }
     const bool smem_hist = q.nbins <= kMaxSmemBins;
     for (int tile = blockIdx.x; tile < q.ntiles; tile += gridDim.x) {
         const int slot = tile * kBlock + threadIdx.x;
@@ -258,11 +264,11 @@ __global__ void __launch_bounds__(kBlock) track_kernel(DevField f, TrackBufs b, 
         for (int j = q.sstep; j <= q.estep; j++) {
             sg[0] = 0.0; sg[4] = 0.0; sg[5] = 0.0;  // src/tracking.c:334-336
             if (active && (esc_pre == 0 || f.bc_flag == 0)) {
-                wirz<SYS>(f, p, q.dt, b.status);
+                wirz<SYS, kTab>(f, p, q.dt, b.status);
                 particle_bc(f, p, esc_after);
                 nst += 1;
                 if (esc_after == 0 && j % kDiffInterval == 0)
-                    calc_diff<SYS>(f, p0, p, q.dt, sg, b.status);
+                    calc_diff<SYS, kTab>(f, p0, p, q.dt, sg, b.status);
                 if (q.traj_every > 0 && j % q.traj_every == 0) {
                     // trajectory point, src/tracking.c:440-447
                     long off = toff + npts;
@@ -564,11 +570,14 @@ cudaError_t launch_point_interp(const DevField& f, int which, int n, const doubl
     return cudaGetLastError();
 }
 
+// dynamic shared memory of track_kernel: the mode sum's cosine table
+static constexpr size_t track_smem(int sys) { return sys == TP_SYS_MODESUM ? sizeof(int4) * (fx::kTab + 1) : 0; }
+
 template <int SYS>
 static cudaError_t launch_track_sys(const DevField& f, const TrackBufs& b, const TrackParams& q,
                                     int grid, cudaStream_t s)
 {
-    track_kernel<SYS><<<grid, kBlock, 0, s>>>(f, b, q);
+    track_kernel<SYS><<<grid, kBlock, track_smem(SYS), s>>>(f, b, q);
     return cudaGetLastError();
 }
 
@@ -596,7 +605,7 @@ int track_max_blocks_per_sm(int system_type)
     case TP_SYS_FORCEFREE: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, track_kernel<TP_SYS_FORCEFREE>, kBlock, 0); break;
     case TP_SYS_MHD: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, track_kernel<TP_SYS_MHD>, kBlock, 0); break;
     case TP_SYS_PIC: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, track_kernel<TP_SYS_PIC>, kBlock, 0); break;
-    case TP_SYS_MODESUM: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, track_kernel<TP_SYS_MODESUM>, kBlock, 0); break;
+    case TP_SYS_MODESUM: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, track_kernel<TP_SYS_MODESUM>, kBlock, track_smem(TP_SYS_MODESUM)); break;
     default: break;
     }
     return e == cudaSuccess ? nb : 0;
