@@ -12,6 +12,7 @@
 #include <cstring>
 
 #include "../../include/tp_gpu.h"
+#define TP_ELL_FP64_QUOTIENT
 #include "fields_fp64.cuh"
 #include "tp_internal.h"
 
@@ -75,13 +76,13 @@ __device__ __forceinline__ void derivs(const DevField& f, int uform, double t, c
         double cy = y[5] * e[0] - y[3] * e[2];
         double cz = y[3] * e[1] - y[4] * e[0];
         double beta2 = y[3] * y[3] + y[4] * y[4] + y[5] * y[5];
-        double gama = 1.0 / sqrt(1.0 - beta2);
-        double igama3 = 1.0 / (gama * gama * gama);
+        double gama = sd::div(1.0, sd::sqrt_rn(1.0 - beta2));
+        double igama3 = sd::div(1.0, gama * gama * gama);
         yd[3] = igama3 * f.charge_mass * (e[3] + cx);
         yd[4] = igama3 * f.charge_mass * (e[4] + cy);
         yd[5] = igama3 * f.charge_mass * (e[5] + cz);
     } else {
-        double ig = 1.0 / sqrt(1.0 + y[3] * y[3] + y[4] * y[4] + y[5] * y[5]);
+        double ig = sd::div(1.0, sd::sqrt_rn(1.0 + y[3] * y[3] + y[4] * y[4] + y[5] * y[5]));
         double v0 = y[3] * ig, v1 = y[4] * ig, v2 = y[5] * ig;
         yd[0] = v0; yd[1] = v1; yd[2] = v2;
         yd[3] = f.charge_mass * (e[3] + v1 * e[2] - v2 * e[1]);

@@ -136,6 +136,9 @@ bool build_field(int stype, DevField& f)
     f.nx = simul_grid.nx; f.ny = simul_grid.ny; f.nz = simul_grid.nz;
     f.gdx = simul_grid.dx; f.gdy = simul_grid.dy; f.gdz = simul_grid.dz; f.gdt = simul_grid.dt;
     f.charge_mass = charge_mass;
+    f.d_gdx = sd::divisor(f.gdx); f.d_gdy = sd::divisor(f.gdy); f.d_gdz = sd::divisor(f.gdz);
+    f.d_cm = sd::divisor(f.charge_mass);
+    f.d_tenth = sd::divisor(0.1);
     f.xmin = simul_domain.xmin; f.xmax = simul_domain.xmax;
     f.ymin = simul_domain.ymin; f.ymax = simul_domain.ymax;
     f.zmin = simul_domain.zmin; f.zmax = simul_domain.zmax;

@@ -167,6 +167,126 @@ __device__ __forceinline__ void interp_f3(const DevField& f, const Tri64& r, con
     }
 }
 
+// ---------------------------------------------------------------- float grids, filtered
+// The reference's float-grid interpolation rounds v + p w, formed in double
+// from a float v, a float node value p and a double weight w, to a float after
+// every corner.  Those roundings are reproduced in FP32: the weight in two
+// floats (48 of its 53 bits), the product and the sum with their rounding
+// errors (two-product by FMA, two-sum), and a bound d on what is left out.
+// Where v + p w - d and v + p w + d round to the same float, so does the
+// double sum, whatever its own rounding.  Where they do not (about one
+// evaluation in ten thousand), or where an exponent could make an error term
+// inexact, the caller takes the double form.  16 FP32 instructions a term
+// instead of two FP64 ones (64 pipe cycles each) and three conversions.
+
+// v <- RN32(v + p w); bad: the rounding is not certain
+__device__ __forceinline__ void add_term(float& v, float p, float wh, float wl, bool& bad)
+{
+    const float ph = __fmul_rn(p, wh);
+    const float pl = __fmaf_rn(p, wl, __fmaf_rn(p, wh, -ph));
+    const float s = __fadd_rn(v, ph), t = __fsub_rn(s, v);
+    const float e = __fadd_rn(__fsub_rn(v, __fsub_rn(s, t)), __fsub_rn(ph, t));
+    const float rest = __fadd_rn(e, pl);
+    // left out: 2^-45.7 |ph| of the product, 2^-24 |rest| in forming rest,
+    // |rest| <= 2^-24 |s| + 2^-22.4 |ph|, and the double roundings; in all
+    // below 2^-44.9 |ph| + 2^-47.9 |s|
+    const float d = __fadd_rn(fabsf(ph), fabsf(s));
+    const float r = __fadd_rn(s, __fmaf_rn(d, 5.6843418860808015e-14f, rest));   // 2^-44
+    const float q = __fadd_rn(s, __fmaf_rn(d, -5.6843418860808015e-14f, rest));
+    // a node value of 2^-60 or less (not zero) could lose bits of its product
+    bad |= r != q || (__float_as_uint(p) << 1) - 1u < (0x21800000u << 1) - 1u;
+    v = r;
+}
+
+// A weight in [2^-36, 1], or 0, as two floats: its leading 24 bits, and the
+// other 29 rounded to 24.  bad: outside that range.
+__device__ __forceinline__ void split_weight(double w, float& wh, float& wl, bool& bad)
+{
+    const uint32_t hi = (uint32_t)__double2hiint(w), lo = (uint32_t)__double2loint(w);
+    const bool zero = (hi | lo) == 0u;
+    bad |= !zero && hi - (987u << 20) > (36u << 20);
+    const uint32_t b = ((hi - (896u << 20)) << 3) | (lo >> 29);
+    const float scale = __uint_as_float((b & 0x7f800000u) - (52u << 23));
+    wh = zero ? 0.0f : __uint_as_float(b);
+    wl = zero ? 0.0f : __fmul_rn(__uint2float_rn(lo & 0x1fffffffu), scale);
+}
+
+// Index and fraction along one axis inside the box (src/interpolation.c:36-105);
+// false where the reference's wrap branches or the array's end would apply.
+__device__ __forceinline__ bool cell64(double x, double lo, double hi, const sd::Divisor& d, int n, int& i, double& fr)
+{
+    const double q = sd::div(x - lo, d), fl = floor(q);
+    i = (int)fl;
+    fr = q - fl;
+    return !(x > hi) && !(x < lo) && (unsigned)i < (unsigned)(n - 1);
+}
+
+// NF fields on the same float grid at one point, single time frame, filtered.
+// False: not certain, take interp_f3.
+template <int NF>
+__device__ __forceinline__ bool interp_filtered(const DevField& f, double x, double y, double z, const float* const g[NF],
+                                                float out[NF][3])
+{
+    int ix, iy, iz;
+    double dx, dy, dz;
+    const bool in = cell64(x, f.xmin, f.xmax, f.d_gdx, f.nx, ix, dx) &
+                    cell64(y, f.ymin, f.ymax, f.d_gdy, f.ny, iy, dy) &
+                    cell64(z, f.zmin, f.zmax, f.d_gdz, f.nz, iz, dz);
+    if (!in) return false;
+    const size_t base = ((size_t)((size_t)iz * f.ny + iy) * f.nx + ix) * 3;
+    const size_t sy = 3 * (size_t)f.nx, sz = sy * f.ny;
+    const size_t off[8] = {0, sz, sy, 3, 3 + sy, 3 + sz, sy + sz, 3 + sy + sz};  // trilinear64's corner order
+    float p[NF][8][3];
+#pragma unroll
+    for (int a = 0; a < NF; a++)
+#pragma unroll
+        for (int c = 0; c < 8; c++)
+#pragma unroll
+            for (int k = 0; k < 3; k++) p[a][c][k] = __ldg(g[a] + base + off[c] + k);
+    const double ax = 1.0 - dx, ay = 1.0 - dy, az = 1.0 - dz;
+    const double w00 = ax * ay, w10 = dx * ay, w01 = ax * dy, w11 = dx * dy;
+    double w[8] = {w00 * az, w10 * az, w01 * az, w00 * dz, w01 * dz, w10 * dz, w11 * az, w11 * dz};
+    if (f.interp_corrected) {
+        double t = w[1]; w[1] = w[3]; w[3] = t;
+        t = w[4]; w[4] = w[6]; w[6] = t;
+    }
+    bool bad = false;
+#pragma unroll
+    for (int a = 0; a < NF; a++)
+#pragma unroll
+        for (int k = 0; k < 3; k++) out[a][k] = 0.0f;
+#pragma unroll
+    for (int c = 0; c < 8; c++) {
+        float wh, wl;
+        split_weight(w[c], wh, wl, bad);
+#pragma unroll
+        for (int a = 0; a < NF; a++)
+#pragma unroll
+            for (int k = 0; k < 3; k++) add_term(out[a][k], p[a][c][k], wh, wl, bad);
+    }
+    return !bad;
+}
+
+// NF fields on float grids in the reference's own arithmetic (any time frames).
+template <int NF>
+__device__ __noinline__ void interp_exact(const DevField& f, double x, double y, double z, double t, const float* const g[NF],
+                                          const float* const ga[NF], const float* const gb[NF], float out[NF][3],
+                                          int* status)
+{
+    Tri64 r;
+    trilinear64(f, x, y, z, t, r);
+    for (int a = 0; a < NF; a++) interp_f3(f, r, g[a], ga[a], gb[a], out[a], status);
+}
+
+template <int NF>
+__device__ __forceinline__ void interp_grids(const DevField& f, double x, double y, double z, double t,
+                                             const float* const g[NF], const float* const ga[NF],
+                                             const float* const gb[NF], float out[NF][3], int* status)
+{
+    if (f.multi_tframe != 0 || !interp_filtered<NF>(f, x, y, z, g, out))
+        interp_exact<NF>(f, x, y, z, t, g, ga, gb, out, status);
+}
+
 // ---------------------------------------------------------------- WLCS
 // transform / reverse_tran, src/wlcs.c:871-903
 __device__ __forceinline__ void wl_transform(double& ax, double& ay, double& az, double c1,
@@ -193,13 +313,20 @@ __device__ __forceinline__ void wl_reverse(double& ax, double& ay, double& az, d
 
 // ellint, src/wlcs.c:460-809 (Fukushima 2009), coefficient tables recomputed
 // from the mathematics (gen_ellint_coeffs.py)
-__device__ __forceinline__ void ellint64(double k, int corrected, double& elle, double& ellf)
+__device__ __forceinline__ void ellint64(const DevField& f, double k, int corrected, double& elle, double& ellf)
 {
     double m = k * k;
     int i;
     elle = 0.0;
     ellf = 0.0;
+    // (with contraction on, which product the compiler fuses into m - m0 below
+    // depends on the instructions that read m: the adaptive stepper, whose step
+    // counts follow the last bit, keeps the FP64 quotient)
+#ifdef TP_ELL_FP64_QUOTIENT
     if (m < 0.8) i = (int)(m / 0.1);
+#else
+    if (m < 0.8) i = (int)sd::div(m, f.d_tenth);
+#endif
     else if (m >= 0.8 && m < 0.85) i = 8;
     else if (m >= 0.85 && m < 0.9) i = 9;
     else i = 10;
@@ -247,14 +374,16 @@ __device__ __forceinline__ void wl_wire_static(const wlcs& c, double x, double y
 {
     double xp = x - c.x_wr, yp = y - c.y_wr, zp = z - c.z_wr;
     wl_transform(xp, yp, zp, c.costheta_wr, c.sintheta_wr, c.cosphi_wr, c.sinphi_wr);
-    double rho = sqrt(xp * xp + yp * yp);
+    double rho = sd::sqrt_rn(xp * xp + yp * yp);
     if (rho < 0.1) rho = 0.1;
-    double cos_phi0 = xp / rho, phi0;
+    double cos_phi0 = sd::div(xp, rho), phi0;
     if (yp >= 0.0) phi0 = acos(cos_phi0);
     else phi0 = 2.0 * TP_PI - acos(cos_phi0);
-    double bphi = 1.0 / 5.0 * (c.cur_wr * TP_I0) / (rho * TP_L0);
-    B[0] = bphi * cos(phi0 + TP_PI / 2.0);
-    B[1] = bphi * sin(phi0 + TP_PI / 2.0);
+    double bphi = sd::div(1.0 / 5.0 * (c.cur_wr * TP_I0), rho * TP_L0);
+    double sn, cs;
+    sd::sin_cos(phi0 + TP_PI / 2.0, sn, cs);
+    B[0] = bphi * cs;
+    B[1] = bphi * sn;
     B[2] = 0.0;
     wl_reverse(B[0], B[1], B[2], c.costheta_wr, c.sintheta_wr, c.cosphi_wr, c.sinphi_wr);
 }
@@ -285,27 +414,28 @@ __device__ __forceinline__ void wl_wire_bessel(const wlcs& c, double x, double y
 }
 
 // getLoopB, src/wlcs.c:406-449 (NaN Bx, By on the loop axis, as there)
-__device__ __forceinline__ void wl_loop(const wlcs& c, int ell_corr, double x, double y,
+__device__ __forceinline__ void wl_loop(const DevField& f, const wlcs& c, int ell_corr, double x, double y,
                                         double z, double B[3])
 {
     double xp = (x - c.x_lp) * TP_L0, yp = (y - c.y_lp) * TP_L0, zp = (z - c.z_lp) * TP_L0;
     double al = c.r_lp * TP_L0, curI = c.cur_lp * TP_I0;
     wl_transform(xp, yp, zp, c.cosbeta_lp, c.sinbeta_lp, c.cosalpha_lp, c.sinalpha_lp);
     double Irho = 0.2 * curI;
-    double rho_xy = sqrt(xp * xp + yp * yp);
+    double rho_xy = sd::sqrt_rn(xp * xp + yp * yp);
     double al2 = al * al;
     double r2 = rho_xy * rho_xy + zp * zp;
-    double irho1 = 1 / sqrt((al + rho_xy) * (al + rho_xy) + zp * zp);
-    double irho2 = 1 / ((al - rho_xy) * (al - rho_xy) + zp * zp);
-    double k = sqrt(4.0 * al * rho_xy) * irho1, elle, ellk;
-    ellint64(k, ell_corr, elle, ellk);
-    double Brho = Irho * zp * irho1 * (-ellk + (al2 + r2) * elle * irho2) / rho_xy;
+    double irho1 = sd::div(1.0, sd::sqrt_rn((al + rho_xy) * (al + rho_xy) + zp * zp));
+    double irho2 = sd::div(1.0, (al - rho_xy) * (al - rho_xy) + zp * zp);
+    double k = sd::sqrt_rn(4.0 * al * rho_xy) * irho1, elle, ellk;
+    ellint64(f, k, ell_corr, elle, ellk);
+    const sd::Divisor d_rho = sd::divisor(rho_xy);
+    double Brho = sd::div(Irho * zp * irho1 * (-ellk + (al2 + r2) * elle * irho2), d_rho);
     if (rho_xy == 0.0) Brho = 0.0;
     double Bz = Irho * irho1 * (ellk - (r2 - al2) * elle * irho2);
     if (ell_corr && rho_xy == 0.0) {
         B[0] = 0.0; B[1] = 0.0;
     } else {
-        Brho /= rho_xy;
+        Brho = sd::div(Brho, d_rho);
         B[0] = Brho * xp;
         B[1] = Brho * yp;
     }
@@ -343,9 +473,13 @@ __device__ __forceinline__ void emf64(const DevField& f, double x, double y, dou
     } else if (SYS == TP_SYS_FORCEFREE) {
         // getb_ff / gete_ff, src/force_free.c:78-86,138-150
         double l = f.lambda0;
-        double bx = f.ffA * sin(l * z) + f.ffC * cos(l * y);
-        double by = f.ffB * sin(l * x) + f.ffA * cos(l * z);
-        double bz = f.ffC * sin(l * y) + f.ffB * cos(l * x);
+        double sx, cx, sy, cy, sz, cz;
+        sd::sin_cos(l * x, sx, cx);
+        sd::sin_cos(l * y, sy, cy);
+        sd::sin_cos(l * z, sz, cz);
+        double bx = f.ffA * sz + f.ffC * cy;
+        double by = f.ffB * sx + f.ffA * cz;
+        double bz = f.ffC * sy + f.ffB * cx;
         bx *= f.B0;
         by *= f.B0;
         bz *= f.B0;
@@ -380,18 +514,17 @@ __device__ __forceinline__ void emf64(const DevField& f, double x, double y, dou
                 By += B[1]; Ey += E[1];
                 Bz += B[2]; Ez += E[2];
             }
-            wl_loop(c, f.ellint_corrected, x, y, z, B);
+            wl_loop(f, c, f.ellint_corrected, x, y, z, B);
             Bx += B[0]; By += B[1]; Bz += B[2];
         }
         e[0] = Bx; e[1] = By; e[2] = Bz + 0.0;
         e[3] = Ex; e[4] = Ey; e[5] = Ez;
     } else if (SYS == TP_SYS_MHD) {
         // getemf_mhd_test_particle, src/emfields.c:107-120
-        Tri64 r;
-        trilinear64(f, x, y, z, t, r);
-        float v[3], b[3];
-        interp_f3(f, r, f.vc_f, f.va_f, f.vb_f, v, status);
-        interp_f3(f, r, f.bc_f, f.ba_f, f.bb_f, b, status);
+        const float *g[2] = {f.vc_f, f.bc_f}, *ga[2] = {f.va_f, f.ba_f}, *gb[2] = {f.vb_f, f.bb_f};
+        float vb[2][3];
+        interp_grids<2>(f, x, y, z, t, g, ga, gb, vb, status);
+        const float *v = vb[0], *b = vb[1];
         e[0] = b[0]; e[1] = b[1]; e[2] = b[2];
         e[3] = e[1] * v[2] - e[2] * v[1];
         e[4] = e[2] * v[0] - e[0] * v[2];
@@ -399,11 +532,10 @@ __device__ __forceinline__ void emf64(const DevField& f, double x, double y, dou
     } else if (SYS == TP_SYS_PIC) {
         // getemf_pic_test_particle, src/emfields.c:153-166; the reference
         // computes the same corners and weights twice, once is enough
-        Tri64 r;
-        trilinear64(f, x, y, z, t, r);
-        float ev[3], b[3];
-        interp_f3(f, r, f.ec_f, f.ea_f, f.eb_f, ev, status);
-        interp_f3(f, r, f.bc_f, f.ba_f, f.bb_f, b, status);
+        const float *g[2] = {f.ec_f, f.bc_f}, *ga[2] = {f.ea_f, f.ba_f}, *gb[2] = {f.eb_f, f.bb_f};
+        float eb[2][3];
+        interp_grids<2>(f, x, y, z, t, g, ga, gb, eb, status);
+        const float *ev = eb[0], *b = eb[1];
         e[3] = ev[0]; e[4] = ev[1]; e[5] = ev[2];
         e[0] = b[0]; e[1] = b[1]; e[2] = b[2];
     } else if (SYS == TP_SYS_MODESUM) {

@@ -5,6 +5,7 @@
 
 #include "../../include/tp_types.h"
 #include "modesum_fx.cuh"
+#include "soft64.cuh"
 
 namespace tp {
 
@@ -44,6 +45,9 @@ struct DevField {
     int nfx;
     double fxs[6];
     const int4 *ctab;
+    // divisors of every step, prepared (soft64.cuh): the grid spacings, q/m
+    // and the interval of the elliptic-integral tables
+    sd::Divisor d_gdx, d_gdy, d_gdz, d_cm, d_tenth;
 };
 
 // Output / scratch buffers of one tracking launch.

@@ -18,73 +18,73 @@ struct P64 {
     double x, y, z, ux, uy, uz, t, xs, ys, zs;
 };
 
-// tracking_wirz, src/tracking.c:749-892 (c0_norm = 1)
+// tracking_wirz, src/tracking.c:749-892 (c0_norm = 1).  Both field evaluations
+// of a push, at its start and at its midpoint, are followed by the same work
+// (the frame about B, the gyration angle, its sine and cosine): one loop body
+// run twice, in the reference's operations and order.  Inlined twice, the body
+// spills the instruction cache.
 template <int SYS, bool TAB = false>
 __device__ __forceinline__ void wirz(const DevField& f, P64& p, double dt, int* status)
 {
     const double cm = f.charge_mass;
+    const double dth = dt * 0.5;
     double e[6];
-    double t0 = p.t;
-    double gama = sqrt(1.0 + p.ux * p.ux + p.uy * p.uy + p.uz * p.uz);
-    emf64<SYS, TAB>(f, p.x, p.y, p.z, t0, e, status);
-    double Btot = sqrt(e[0] * e[0] + e[1] * e[1] + e[2] * e[2]);
-    double iBtot = 1.0 / Btot;
-    double dth = dt * 0.5;
-    double dm0 = p.ux + cm * dth * e[3];
-    double dm1 = p.uy + cm * dth * e[4];
-    double dm2 = p.uz + cm * dth * e[5];
-    gama = sqrt(1.0 + dm0 * dm0 + dm1 * dm1 + dm2 * dm2);
-    double igama = 1.0 / gama;
-    double vm0 = dm0 * igama, vm1 = dm1 * igama, vm2 = dm2 * igama;
-    double h0 = e[0] * iBtot, h1 = e[1] * iBtot, h2 = e[2] * iBtot;
-    double vdothp = 0.0;
-    vdothp += vm0 * h0;
-    vdothp += vm1 * h1;
-    vdothp += vm2 * h2;
-    double q0 = vm0 - vdothp * h0, q1 = vm1 - vdothp * h1, q2 = vm2 - vdothp * h2;
-    double vperp = sqrt(q0 * q0 + q1 * q1 + q2 * q2);
-    double hp0 = (vm0 - vdothp * h0) / vperp;
-    double hp1 = (vm1 - vdothp * h1) / vperp;
-    double hp2 = (vm2 - vdothp * h2) / vperp;
-    double hr0 = h1 * hp2 - h2 * hp1;
-    double hr1 = h2 * hp0 - h0 * hp2;
-    double hr2 = h0 * hp1 - h1 * hp0;
-    double gyroR = vperp * gama * 1.0 * iBtot / cm;
-    double omegac = cm * Btot * igama;
-    double dtheta = omegac * dt;
-    double sind = sin(dtheta * 0.5), cosd = cos(dtheta * 0.5);
-    double tmp1 = dth * vdothp * 1.0, tmp2 = gyroR * sind, tmp3 = -gyroR * (1.0 - cosd);
-    double px = p.x + h0 * tmp1 + hp0 * tmp2 + hr0 * tmp3;
-    double py = p.y + h1 * tmp1 + hp1 * tmp2 + hr1 * tmp3;
-    double pz = p.z + h2 * tmp1 + hp2 * tmp2 + hr2 * tmp3;
-    emf64<SYS, TAB>(f, px, py, pz, t0 + dth, e, status);
-    Btot = sqrt(e[0] * e[0] + e[1] * e[1] + e[2] * e[2]);
-    iBtot = 1.0 / Btot;
-    h0 = e[0] * iBtot; h1 = e[1] * iBtot; h2 = e[2] * iBtot;
-    vdothp = 0.0;
-    vdothp += vm0 * h0;
-    vdothp += vm1 * h1;
-    vdothp += vm2 * h2;
-    q0 = vm0 - vdothp * h0; q1 = vm1 - vdothp * h1; q2 = vm2 - vdothp * h2;
-    vperp = sqrt(q0 * q0 + q1 * q1 + q2 * q2);
-    hp0 = (vm0 - vdothp * h0) / vperp;
-    hp1 = (vm1 - vdothp * h1) / vperp;
-    hp2 = (vm2 - vdothp * h2) / vperp;
-    hr0 = h1 * hp2 - h2 * hp1;
-    hr1 = h2 * hp0 - h0 * hp2;
-    hr2 = h0 * hp1 - h1 * hp0;
-    omegac = cm * Btot * igama;
-    dtheta = omegac * dt;
-    sind = sin(dtheta);
-    cosd = cos(dtheta);
-    double vp0 = h0 * vdothp + vperp * (cosd * hp0 - sind * hr0);
-    double vp1 = h1 * vdothp + vperp * (cosd * hp1 - sind * hr1);
-    double vp2 = h2 * vdothp + vperp * (cosd * hp2 - sind * hr2);
+    double gama = 1.0, igama = 1.0, vm0 = 0.0, vm1 = 0.0, vm2 = 0.0;
+    double iBtot, h0, h1, h2, vdothp, vperp, hp0, hp1, hp2, hr0, hr1, hr2, sind, cosd;
+    double px = p.x, py = p.y, pz = p.z;
+#pragma unroll 1
+    for (int half = 0;; half++) {
+        emf64<SYS, TAB>(f, px, py, pz, half ? p.t + dth : p.t, e, status);
+        const double Btot = sd::sqrt_rn(e[0] * e[0] + e[1] * e[1] + e[2] * e[2]);
+        iBtot = sd::div(1.0, Btot);
+        if (half == 0) {
+            const double dm0 = p.ux + cm * dth * e[3];
+            const double dm1 = p.uy + cm * dth * e[4];
+            const double dm2 = p.uz + cm * dth * e[5];
+            gama = sd::sqrt_rn(1.0 + dm0 * dm0 + dm1 * dm1 + dm2 * dm2);
+            igama = sd::div(1.0, gama);
+            vm0 = dm0 * igama; vm1 = dm1 * igama; vm2 = dm2 * igama;
+        }
+        h0 = e[0] * iBtot; h1 = e[1] * iBtot; h2 = e[2] * iBtot;
+        vdothp = 0.0;
+        vdothp += vm0 * h0;
+        vdothp += vm1 * h1;
+        vdothp += vm2 * h2;
+        const double q0 = vm0 - vdothp * h0, q1 = vm1 - vdothp * h1, q2 = vm2 - vdothp * h2;
+        vperp = sd::sqrt_rn(q0 * q0 + q1 * q1 + q2 * q2);
+        const sd::Divisor d_vperp = sd::divisor(vperp);
+        hp0 = sd::div(q0, d_vperp);
+        hp1 = sd::div(q1, d_vperp);
+        hp2 = sd::div(q2, d_vperp);
+        hr0 = h1 * hp2 - h2 * hp1;
+        hr1 = h2 * hp0 - h0 * hp2;
+        hr2 = h0 * hp1 - h1 * hp0;
+        const double omegac = cm * Btot * igama;
+        const double dtheta = omegac * dt;
+        const double ang = half ? dtheta : dtheta * 0.5;
+        if (SYS == TP_SYS_MHD || SYS == TP_SYS_PIC) {
+            // the float grids' roundings turn a last-place difference of the
+            // orbit into one of 2^-24 of a field: these systems keep CUDA's
+            sind = sin(ang);
+            cosd = cos(ang);
+        } else {
+            sd::sin_cos(ang, sind, cosd);
+        }
+        if (half) break;
+        const double gyroR = sd::div(vperp * gama * 1.0 * iBtot, f.d_cm);
+        const double tmp1 = dth * vdothp * 1.0, tmp2 = gyroR * sind, tmp3 = -gyroR * (1.0 - cosd);
+        px = p.x + h0 * tmp1 + hp0 * tmp2 + hr0 * tmp3;
+        py = p.y + h1 * tmp1 + hp1 * tmp2 + hr1 * tmp3;
+        pz = p.z + h2 * tmp1 + hp2 * tmp2 + hr2 * tmp3;
+    }
+    const double vp0 = h0 * vdothp + vperp * (cosd * hp0 - sind * hr0);
+    const double vp1 = h1 * vdothp + vperp * (cosd * hp1 - sind * hr1);
+    const double vp2 = h2 * vdothp + vperp * (cosd * hp2 - sind * hr2);
     double bm = 0.0;  // get_delta_vec, src/tracking.c:1066-1078
     bm += vp0 * vp0;
     bm += vp1 * vp1;
     bm += vp2 * vp2;
-    double g2 = 1.0 / sqrt(1.0 - bm);
+    const double g2 = sd::div(1.0, sd::sqrt_rn(1.0 - bm));
     p.ux = g2 * vp0 + cm * dth * e[3];
     p.uy = g2 * vp1 + cm * dth * e[4];
     p.uz = g2 * vp2 + cm * dth * e[5];
@@ -92,12 +92,12 @@ __device__ __forceinline__ void wirz(const DevField& f, P64& p, double dt, int* 
     vdothp += vp0 * h0;
     vdothp += vp1 * h1;
     vdothp += vp2 * h2;
-    q0 = vp0 - vdothp * h0; q1 = vp1 - vdothp * h1; q2 = vp2 - vdothp * h2;
-    vperp = sqrt(q0 * q0 + q1 * q1 + q2 * q2);
-    gyroR = vperp * gama * 1.0 * iBtot / cm;
-    tmp1 = dt * vdothp * 1.0;
-    tmp2 = gyroR * sind;
-    tmp3 = -gyroR * (1.0 - cosd);
+    const double q0 = vp0 - vdothp * h0, q1 = vp1 - vdothp * h1, q2 = vp2 - vdothp * h2;
+    vperp = sd::sqrt_rn(q0 * q0 + q1 * q1 + q2 * q2);
+    const double gyroR = sd::div(vperp * gama * 1.0 * iBtot, f.d_cm);
+    const double tmp1 = dt * vdothp * 1.0;
+    const double tmp2 = gyroR * sind;
+    const double tmp3 = -gyroR * (1.0 - cosd);
     p.x += h0 * tmp1 + hp0 * tmp2 + hr0 * tmp3;
     p.y += h1 * tmp1 + hp1 * tmp2 + hr1 * tmp3;
     p.z += h2 * tmp1 + hp2 * tmp2 + hr2 * tmp3;
@@ -214,6 +214,11 @@ __device__ __forceinline__ void block_diff_sum(const double sg[8], double* red, 
     __syncthreads();
 }
 
+// Resident blocks per SM the kernel is compiled for (3: at most 168 registers,
+// no spills).  Two blocks (up to 228 registers) left the gridded run of 131,072
+// particles 8 % slower, four (128, 120-316 bytes of spills) 4 %.
+constexpr int kTrackMinBlocks = 3;
+
 // Persistent fixed-step tracking, restating particle_tracking_multi_steps_openmp
 // and _single_step_openmp (src/tracking.c:297-462): one thread owns one
 // particle for all estep steps; blocks walk tiles of kBlock particles.  All
@@ -221,7 +226,7 @@ __device__ __forceinline__ void block_diff_sum(const double sg[8], double* red, 
 // (every einterval steps for the spectrum, every 100 for the diffusion sums)
 // are block-uniform and reduce through shared memory.
 template <int SYS>
-__global__ void __launch_bounds__(kBlock, SYS == TP_SYS_MODESUM ? 4 : 1) track_kernel(DevField f, TrackBufs b, TrackParams q)
+__global__ void __launch_bounds__(kBlock, kTrackMinBlocks) track_kernel(DevField f, TrackBufs b, TrackParams q)
 {
     __shared__ double red[(kBlock / 32) * 8];
     __shared__ unsigned int hist[kMaxSmemBins];
@@ -468,12 +473,11 @@ __device__ __forceinline__ void pm_boundary(const DevField& f, double& x, double
 __device__ __forceinline__ void pm_unit_b(const DevField& f, double x, double y, double z, double b[3],
                                           int* status)
 {
-    Tri64 r;
-    trilinear64(f, x, y, z, 0.0, r);
-    float v[3];
-    interp_f3(f, r, f.bc_f, f.ba_f, f.bb_f, v, status);
-    double bx = v[0], by = v[1], bz = v[2];
-    double ib = 1.0 / sqrt(bx * bx + by * by + bz * bz);
+    const float *g[1] = {f.bc_f}, *ga[1] = {f.ba_f}, *gb[1] = {f.bb_f};
+    float v[1][3];
+    interp_grids<1>(f, x, y, z, 0.0, g, ga, gb, v, status);
+    double bx = v[0][0], by = v[0][1], bz = v[0][2];
+    double ib = sd::div(1.0, sd::sqrt_rn(bx * bx + by * by + bz * bz));
     b[0] = bx * ib;
     b[1] = by * ib;
     b[2] = bz * ib;
