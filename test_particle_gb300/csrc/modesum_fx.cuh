@@ -7,9 +7,11 @@
 // in known ranges.  So each term is evaluated and summed in integers and one
 // conversion per component makes the double.  The FP64 cosine and sums took
 // about 2900 cycles a warp and mode; a run of 65,536 particles over 10 steps in
-// a 512-mode field (host buffers in and out) went from 49.8 to 7.8 ms, and a
-// training run on 131,072 samples of such a field from 9.64 to 6.82 ms.  It is
-// bound by the issue of about 90 integer instructions a mode.
+// a 512-mode field (host buffers in and out) went from 49.8 to 5.6 ms, and a
+// training run on 131,072 samples of such a field from 9.64 to 6.60 ms.  It is
+// bound by the issue of 126 instructions a mode (43 multiply-adds, 65 on the
+// half-rate integer pipe) and by four warps on one sub-partition where others
+// have three.
 //
 // Accuracy, against quadruple precision: the cosine is off by 2^-53.9 rms and
 // 2^-51.4 at most, the FP64 form (whose phase rounds before its cosine) by
@@ -42,6 +44,20 @@ struct alignas(16) Mode {
 // (C >> 31, C & (2^31 - 1)), and 2 pi sin phi in Q60 as (>> 32, low word >> 1).
 // int4: x, y the cosine, z, w the sine.
 
+// acc + a b, 32 x 32 + 64 bits, signed.  Spelled out on the device: where the
+// compiler knows a factor not to be negative it widens the two factors
+// differently and multiplies in 64 bits, four instructions for one.
+__host__ __device__ __forceinline__ int64_t mad(int32_t a, int32_t b, int64_t acc)
+{
+#ifdef __CUDA_ARCH__
+    int64_t r;
+    asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(r) : "r"(a), "r"(b), "l"(acc));
+    return r;
+#else
+    return acc + (int64_t)a * b;
+#endif
+}
+
 // High and low parts of cos(2 pi ph / 2^64) = (ch 2^32 + cl 4) / 2^62.
 // The revolution is folded into its first quarter, p = angle * 2^64 / 2 pi in
 // [0, 2^62]; the nearest table point is within d = 2 pi 2^-13, and
@@ -60,10 +76,10 @@ __host__ __device__ __forceinline__ void cosine(uint64_t ph, const int4* tab, in
     const int32_t th = (int32_t)(t >> 20);
     const int32_t tl = (int32_t)((uint32_t)t << 12 >> 1);    // low 20 bits, scaled to 31
     // S d in Q62: (sh 2^32 + sl 2) (th 2^20 + tl 2^-11) 2^-62
-    const int64_t a1 = (int64_t)e.z * th;
-    const int64_t a2 = (int64_t)e.w * th + (int64_t)e.z * tl;
+    const int64_t a1 = mad(e.z, th, 0);
+    const int64_t a2 = mad(e.z, tl, mad(e.w, th, 0));
     // C d^2 / 2 in Q62: z = t^2 2^-71 with the dropped bits of t at their middle
-    const int64_t t2 = (int64_t)th * th + th;
+    const int64_t t2 = mad(th, th, th);
     const uint32_t z = (uint32_t)((uint64_t)(t2 + (1ll << 30)) >> 31);
     const uint32_t zz = (uint32_t)(((uint64_t)z * 2649351758u + (1ull << 30)) >> 31);  // (2 pi)^2 / 2 * 2^27
     const uint64_t quad = (uint64_t)(uint32_t)e.x * zz;
@@ -97,7 +113,7 @@ __host__ __device__ __forceinline__ void mode_sum(const Mode* modes, int nm, con
     int64_t hh[6] = {0, 0, 0, 0, 0, 0}, mid[6] = {0, 0, 0, 0, 0, 0};
     for (int m0 = 0; m0 < nm; m0 += kChunk) {
 #ifdef __CUDA_ARCH__
-#pragma unroll 2
+#pragma unroll 4
 #endif
         for (int m = m0; m < m0 + kChunk; m++) {
             int4 r[4];
@@ -107,9 +123,7 @@ __host__ __device__ __forceinline__ void mode_sum(const Mode* modes, int nm, con
 #else
             for (int q = 0; q < 4; q++) r[q] = reinterpret_cast<const int4*>(modes + m)[q];
 #endif
-            uint64_t ph = (uint64_t)((int64_t)r[0].x * ul[0]);
-            ph += (uint64_t)((int64_t)r[0].y * ul[1]);
-            ph += (uint64_t)((int64_t)r[0].z * ul[2]);
+            uint64_t ph = (uint64_t)mad(r[0].z, ul[2], mad(r[0].y, ul[1], mad(r[0].x, ul[0], 0)));
             const uint32_t hi = (uint32_t)r[0].x * uh[0] + (uint32_t)r[0].y * uh[1] + (uint32_t)r[0].z * uh[2] +
                                 (uint32_t)r[0].w;
             ph += (uint64_t)hi << 32;
@@ -121,9 +135,8 @@ __host__ __device__ __forceinline__ void mode_sum(const Mode* modes, int nm, con
 #pragma unroll
 #endif
             for (int k = 0; k < 6; k++) {
-                hh[k] += (int64_t)ah[k] * ch;
-                mid[k] += (int64_t)ah[k] * cl;
-                mid[k] += (int64_t)al[k] * ch;
+                hh[k] = mad(ah[k], ch, hh[k]);
+                mid[k] = mad(al[k], ch, mad(ah[k], cl, mid[k]));
             }
         }
         // |mid| < 2^63 over a chunk: carry it up
