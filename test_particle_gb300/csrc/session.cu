@@ -32,6 +32,10 @@ static void fill_int(int* p, int n, int v, cudaStream_t s)
     if (n > 0) fill_int_kernel<<<(n + 255) / 256, 256, 0, s>>>(p, n, v);
 }
 
+// Most waves of blocks of a mixed mode-sum run, and the partial sums they may take.
+constexpr int kBlockWaves = 16;
+constexpr size_t kMaxPartialBytes = (size_t)256 << 20;
+
 // ---------------------------------------------------------------- open-boundary segments
 // Between the segments of an open-boundary run the particles still inside the
 // box are compacted into an index list, in list order and independent of
@@ -251,7 +255,18 @@ bool Session::run(const RunSpec& rs, tp_run_info* info)
         return false;
     }
     if (bps < 1) bps = 1;
-    int grid = g.num_sms * bps;
+    // Resident blocks walk the tiles.  The mixed mode sum instead gets a block
+    // per tile, up to kBlockWaves waves: the hardware hands the next block to
+    // the SM that is free, where the walk leaves SMs idle while the blocks with
+    // one tile more finish (262,144 particles, 1.7 waves: 10.06 -> 8.97 ms; the
+    // gridded and analytic fields gain 0 to 1 %, the FP64 gridded path loses
+    // 4 %).  Every block has its own slot of partial sums, so the results do
+    // not depend on the order.
+    const int resident = g.num_sms * bps;
+    int grid = resident;
+    if (is_mixed && system_type == TP_SYS_MODESUM &&
+        (size_t)resident * kBlockWaves * (rs.estep / kDiffInterval + 1) * 64 <= kMaxPartialBytes)
+        grid = resident * kBlockWaves;
     if (grid > ntiles) grid = ntiles;
     if (grid < 1) grid = 1;
     // open boundaries: segments of seg steps with the departed particles
@@ -266,7 +281,7 @@ bool Session::run(const RunSpec& rs, tp_run_info* info)
     seg_ll = (seg_ll + kDiffInterval - 1) / kDiffInterval * kDiffInterval;
     const bool segs = bc_flag == 1 && g.compact_steps != 0 && rs.traj_every == 0 && !is_surr &&
                       rs.sstep == 1 && (long long)rs.estep > seg_ll && n > 0 &&
-                      (!automatic || ntiles > grid);
+                      (!automatic || ntiles > resident);
     const int seg = (int)std::min<long long>(seg_ll, rs.estep);  // < estep whenever segs
     const int nslot = grid + (segs ? 1 : 0);  // the last slot takes the departed particles' rows
     size_t nspec = (size_t)nt_out * nbins;

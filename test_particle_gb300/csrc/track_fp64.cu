@@ -335,13 +335,28 @@ __global__ void __launch_bounds__(kBlock, track_min_blocks(SYS)) track_kernel(De
 }
 
 // Fixed-order sum of the per-block partials: dsum[c * nsdc + s] (component-major).
-__global__ void reduce_dpart_kernel(const double* dpart, int nblocks, int nsdc, double* dsum)
+// A block takes 32 outputs; each of its rows sums every kReduceRows-th tracking
+// block, then the rows are added in order.
+constexpr int kReduceRows = 16;
+__global__ void __launch_bounds__(32 * kReduceRows) reduce_dpart_kernel(const double* dpart, int nblocks, int nsdc,
+                                                                        double* dsum)
 {
-    int k = blockIdx.x * blockDim.x + threadIdx.x;  // k = s * 8 + c
-    if (k >= nsdc * 8) return;
+    __shared__ double part[kReduceRows][32];
+    const int lane = threadIdx.x & 31, row = threadIdx.x >> 5;
+    const int k = blockIdx.x * 32 + lane;  // k = s * 8 + c
     double s = 0.0;
-    for (int bidx = 0; bidx < nblocks; bidx++) s += dpart[(size_t)bidx * nsdc * 8 + k];
-    dsum[(k & 7) * nsdc + (k >> 3)] = s;
+    if (k < nsdc * 8) {
+#pragma unroll 4
+        for (int b = row; b < nblocks; b += kReduceRows) s += dpart[(size_t)b * nsdc * 8 + k];
+    }
+    part[row][lane] = s;
+    __syncthreads();
+    if (row == 0 && k < nsdc * 8) {
+        double t = 0.0;
+#pragma unroll
+        for (int r = 0; r < kReduceRows; r++) t += part[r][lane];
+        dsum[(k & 7) * nsdc + (k >> 3)] = t;
+    }
 }
 
 // ---------------------------------------------------------------- batch utilities
@@ -627,7 +642,7 @@ cudaError_t launch_reduce_dpart(const double* dpart, int nblocks, int nsdc, doub
                                 cudaStream_t s)
 {
     int n = nsdc * 8;
-    reduce_dpart_kernel<<<(n + 127) / 128, 128, 0, s>>>(dpart, nblocks, nsdc, dsum);
+    reduce_dpart_kernel<<<(n + 31) / 32, 32 * kReduceRows, 0, s>>>(dpart, nblocks, nsdc, dsum);
     return cudaGetLastError();
 }
 

@@ -13,6 +13,8 @@
 // rotation form: the perpendicular frame comes from h x u (no cancellation for
 // u nearly along B), 1 - cos(a) is formed as 2 sin^2(a/2), and the momentum is
 // rotated in u-space so gamma is never re-derived from |v| -> 1.
+#include <algorithm>
+
 #include "tp_kernels_mixed.h"
 #include "wirz_f32.cuh"
 
@@ -58,9 +60,9 @@ enum : int { DG_SG = 0, DG_X0 = 8, DG_U0 = 11, DG_T0 = 14, DG_MU0 = 15, DG_G0 = 
 // (Compiled as a separate function, with a cache of its own, this costs the
 // step loop spills at its call site instead of saving registers: measured
 // by -Xptxas -v, 24-32 B at 4 blocks per SM, 132-152 B at 5.)
-template <int SYS>
+template <int SYS, int W>
 __device__ __forceinline__ void diff_singles_body(const MixField& f, const PM& p, const ModePair* smodes,
-                                                  FieldCache& fc, double (*dg)[kBlock], int tx, int done, double qdt)
+                                                  FieldCache& fc, double (*dg)[W], int tx, int done, double qdt)
 {
     double t = dg[DG_T0][tx] + done * qdt;
     double itt = 1.0 / (t * 2 + qdt);
@@ -184,7 +186,7 @@ __global__ void __launch_bounds__(kBlock, SYS == TP_SYS_PIC ? TP_MIXED_PIC_MINBL
                 nst += 1;
                 done += 1;
                 if (esc_after == 0 && at_diff) {
-                    diff_singles_body<SYS>(f, p, smodes, fc, dg, tx, done, q.dt);
+                    diff_singles_body<SYS, kBlock>(f, p, smodes, fc, dg, tx, done, q.dt);
                 }
             }
             if (active && esc_pre == 0 && esc_after == 1 && f.bc_flag == 1 && ntp < q.nt_out)
@@ -251,6 +253,213 @@ __global__ void __launch_bounds__(kBlock, SYS == TP_SYS_PIC ? TP_MIXED_PIC_MINBL
     }
 }
 
+// The same for the mode sum with PPT particles a thread (a tile is PPT * kBlock
+// particles; thread tx owns particles tx, tx + kBlock, ...).  Its loop is bound
+// by issue: the records of the modes are read once for all of a thread's
+// particles, and their chains hide each other's latency: 5.91 -> 5.06 ms for
+// 155,648 particles x 50 steps (host buffers in and out), about 20 cycles a
+// warp, particle and mode against 14 of its multiply-adds alone.  (One kernel
+// for both, with PPT 1 for the other fields, ran the ABC field 7 % slower;
+// three or four particles a thread, at three and two blocks an SM, 3-8 %.)
+template <int PPT>
+__global__ void __launch_bounds__(kBlock, 4) track_modes_kernel(MixField f, TrackBufs b, TrackParams q)
+{
+    constexpr int SYS = TP_SYS_MODESUM, W = PPT * kBlock;
+    __shared__ double red[(kBlock / 32) * 8];
+    __shared__ double dg[DG_ROWS][W];
+    extern __shared__ ModePair smodes[];
+    // the histogram takes the bins it needs, behind the modes
+    unsigned int* hist = (unsigned int*)(smodes + (f.nmodes + 1) / 2);
+    for (int m = threadIdx.x; m < (f.nmodes + 1) / 2; m += blockDim.x) smodes[m] = f.modes[m];
+    __syncthreads();
+    const int tx = threadIdx.x;
+    const bool smem_hist = q.nbins <= kMaxSmemBins;
+    const float dt = (float)q.dt;
+    for (int tile = blockIdx.x; tile < q.ntiles; tile += gridDim.x) {
+        bool active[PPT], esc_pre[PPT], esc_after[PPT];
+        int id[PPT], nst[PPT], done[PPT];
+        PM p[PPT];
+        FieldCache fc;
+#pragma unroll
+        for (int r = 0; r < PPT; r++) {
+            const int slot = tile * W + r * kBlock + tx, tr = r * kBlock + tx;
+            active[r] = slot < q.n;
+            const int i = active[r] && q.idx ? q.idx[slot] : slot;  // the particle of this lane
+            id[r] = i;
+            p[r] = {};
+            nst[r] = 1;
+            bool esc = false;
+#pragma unroll
+            for (int c = 0; c < DG_ROWS; c++) dg[c][tr] = 0.0;
+            if (active[r]) {
+                double xs[3] = {b.x[i], b.y[i], b.z[i]};
+                double sh[3] = {b.xs[i], b.ys[i], b.zs[i]};
+                double x0[3] = {b.x0[i], b.y0[i], b.z0[i]};
+                double u0[3] = {b.ux0[i], b.uy0[i], b.uz0[i]};
+                dg[DG_T0][tr] = b.t[i];
+                nst[r] = b.nsteps_ptl[i];
+#pragma unroll
+                for (int k = 0; k < 3; k++) {
+                    double rr = (xs[k] - f.min[k]) / f.L[k];
+                    double fl = floor(rr);
+                    if (f.bc_flag == 1 && (rr < 0.0 || rr > 1.0)) esc = true;
+                    p[r].X[k] = __double2ull_rz((rr - fl) * 18446744073709551616.0);
+                    p[r].img[k] = (int)fl + (int)llrint(sh[k] / f.L[k]);
+                    dg[DG_X0 + k][tr] = x0[k];
+                    dg[DG_U0 + k][tr] = u0[k];
+                }
+                p[r].u[0] = (float)b.ux[i]; p[r].u[1] = (float)b.uy[i]; p[r].u[2] = (float)b.uz[i];
+                dg[DG_G0][tr] = sqrt(1.0 + u0[0] * u0[0] + u0[1] * u0[1] + u0[2] * u0[2]);
+                // mu of the initial state: the field at the initial position is static
+                uint64_t X0[3];
+                float uf0[3] = {(float)u0[0], (float)u0[1], (float)u0[2]};
+#pragma unroll
+                for (int k = 0; k < 3; k++) {
+                    double rr = (x0[k] - f.min[k]) / f.L[k];
+                    X0[k] = __double2ull_rz((rr - floor(rr)) * 18446744073709551616.0);
+                }
+                dg[DG_MU0][tr] = pitch_mu<SYS>(f, X0, uf0, smodes, fc);
+                if (q.resumed && b.sg_carry) {
+                    // continue exactly where the previous segment stopped: the
+                    // 64-bit fixed-point position and period counts, the start
+                    // time and the steps taken (t = t0 + steps * dt)
+                    const double* cr = b.sg_carry + (size_t)i * kSegCarry;
+#pragma unroll
+                    for (int c = 0; c < 8; c++) dg[DG_SG + c][tr] = cr[c];
+#pragma unroll
+                    for (int k = 0; k < 3; k++) {
+                        p[r].X[k] = (uint64_t)__double_as_longlong(cr[8 + k]);
+                        p[r].img[k] = (int)cr[11 + k];
+                    }
+                    dg[DG_T0][tr] = cr[14];
+                }
+            }
+            esc_pre[r] = esc;
+            esc_after[r] = esc;
+            if (active[r] && esc && !q.resumed) atomicSub(&b.remain[1], 1);
+            done[r] = 0;
+            if (active[r] && q.resumed && b.sg_carry) done[r] = (int)b.sg_carry[(size_t)i * kSegCarry + 15];
+        }
+        int ntp = q.ntp0, tstep = 1 + q.row0;
+        double* slot_base = b.dpart + (size_t)blockIdx.x * q.nsdc * 8;
+        // countdowns to the next diagnostic steps (j % einterval, j % 100)
+        int to_frame = q.einterval - q.sstep % q.einterval;
+        int to_diff = kDiffInterval - q.sstep % kDiffInterval;
+        if (to_frame == q.einterval) to_frame = 0;
+        if (to_diff == kDiffInterval) to_diff = 0;
+        for (int j = q.sstep; j <= q.estep; j++) {
+            const bool at_diff = to_diff == 0, at_frame = to_frame == 0;
+            to_diff = at_diff ? kDiffInterval - 1 : to_diff - 1;
+            to_frame = at_frame ? q.einterval - 1 : to_frame - 1;
+            // every particle of the thread in step; one that does not move
+            // (past the end, or escaped) is sampled and not pushed
+            float E[PPT][3], B[PPT][3];
+            uint64_t X[PPT][3];
+            WirzMid m[PPT];
+#pragma unroll
+            for (int r = 0; r < PPT; r++)
+#pragma unroll
+                for (int k = 0; k < 3; k++) X[r][k] = p[r].X[k];
+            mode_sum_mixed<PPT>(f, X, E, B, smodes);
+#pragma unroll
+            for (int r = 0; r < PPT; r++) wirz_first(f, p[r], dt, E[r], B[r], m[r], X[r]);
+            mode_sum_mixed<PPT>(f, X, E, B, smodes);
+#pragma unroll
+            for (int r = 0; r < PPT; r++) {
+                if (active[r] && (!esc_pre[r] || f.bc_flag == 0)) {
+                    bool e2 = false;
+                    wirz_second(f, p[r], dt, E[r], B[r], m[r], e2);
+                    if (e2) esc_after[r] = true;
+                    nst[r] += 1;
+                    done[r] += 1;
+                }
+            }
+            if (at_diff) {
+#pragma unroll
+                for (int r = 0; r < PPT; r++)
+                    if (active[r] && (!esc_pre[r] || f.bc_flag == 0) && !esc_after[r])
+                        diff_singles_body<SYS, W>(f, p[r], smodes, fc, dg, r * kBlock + tx, done[r], q.dt);
+            }
+#pragma unroll
+            for (int r = 0; r < PPT; r++)
+                if (active[r] && !esc_pre[r] && esc_after[r] && f.bc_flag == 1 && ntp < q.nt_out)
+                    atomicAdd(&b.espect_esc[ntp * q.nbins + energy_bin_f(b.ebin_thr, q.nbins, p[r].u)], 1u);
+            if (at_frame) {
+                if (ntp < q.nt_out) {
+                    if (smem_hist) {
+                        __syncthreads();
+                        for (int k = tx; k < q.nbins; k += blockDim.x) hist[k] = 0u;
+                        __syncthreads();
+#pragma unroll
+                        for (int r = 0; r < PPT; r++)
+                            if (active[r] && !esc_after[r])
+                                atomicAdd(&hist[energy_bin_f(b.ebin_thr, q.nbins, p[r].u)], 1u);
+                        __syncthreads();
+                        for (int k = tx; k < q.nbins; k += blockDim.x)
+                            if (hist[k]) atomicAdd(&b.espect[ntp * q.nbins + k], hist[k]);
+                    } else {
+#pragma unroll
+                        for (int r = 0; r < PPT; r++)
+                            if (active[r] && !esc_after[r])
+                                atomicAdd(&b.espect[ntp * q.nbins + energy_bin_f(b.ebin_thr, q.nbins, p[r].u)], 1u);
+                    }
+                }
+                ntp++;
+            }
+            if (at_diff) {
+                double sg[8] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+                for (int r = 0; r < PPT; r++) {
+                    const int tr = r * kBlock + tx;
+                    // drr, dpp and duu are the only singles the reference clears
+                    // every step (src/tracking.c:334-336); the others keep their
+                    // last values for particles that no longer move
+                    if (!(active[r] && (!esc_pre[r] || f.bc_flag == 0) && !esc_after[r])) {
+                        dg[DG_SG + 0][tr] = 0.0; dg[DG_SG + 4][tr] = 0.0; dg[DG_SG + 5][tr] = 0.0;
+                    }
+#pragma unroll
+                    for (int c = 0; c < 8; c++) sg[c] = r == 0 ? dg[DG_SG + c][tr] : sg[c] + dg[DG_SG + c][tr];
+                }
+                block_diff_sum(sg, red, slot_base + (size_t)tstep * 8);
+                tstep++;
+            }
+#pragma unroll
+            for (int r = 0; r < PPT; r++) {
+                if (active[r] && esc_after[r] && at_diff && tstep < q.nsdc) atomicSub(&b.remain[tstep], 1);
+                esc_pre[r] = esc_after[r];
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < PPT; r++) {
+            if (!active[r]) continue;
+            const int i = id[r], tr = r * kBlock + tx;
+            double xs[3];
+#pragma unroll
+            for (int k = 0; k < 3; k++) xs[k] = f.min[k] + f.L[k] * ((double)p[r].X[k] * 5.421010862427522e-20);
+            b.x[i] = xs[0]; b.y[i] = xs[1]; b.z[i] = xs[2];
+            b.xs[i] = p[r].img[0] * f.L[0]; b.ys[i] = p[r].img[1] * f.L[1]; b.zs[i] = p[r].img[2] * f.L[2];
+            b.ux[i] = p[r].u[0]; b.uy[i] = p[r].u[1]; b.uz[i] = p[r].u[2];
+            b.t[i] = dg[DG_T0][tr] + done[r] * q.dt;
+            b.nsteps_ptl[i] = nst[r];
+            if (b.status && !(isfinite(p[r].u[0]) && isfinite(p[r].u[1]) && isfinite(p[r].u[2])))
+                atomicOr(b.status, ST_NONFINITE);
+            if (b.sg_carry) {
+                double* cr = b.sg_carry + (size_t)i * kSegCarry;
+#pragma unroll
+                for (int c = 0; c < 8; c++) cr[c] = dg[DG_SG + c][tr];
+#pragma unroll
+                for (int k = 0; k < 3; k++) {
+                    cr[8 + k] = __longlong_as_double((long long)p[r].X[k]);
+                    cr[11 + k] = (double)p[r].img[k];
+                }
+                cr[14] = dg[DG_T0][tr];
+                cr[15] = (double)done[r];
+            }
+            if (b.esc_out) b.esc_out[i] = esc_after[r] ? 1 : 0;
+        }
+    }
+}
+
 // The FP32 field of the mixed path at given points (tests and callers that
 // want the field the throughput path sees): each position is turned into
 // 64-bit fixed point exactly as the tracking kernel turns a particle's, and
@@ -291,6 +500,14 @@ cudaError_t launch_emf_batch(const MixField& f, int n, const double* xyz, float*
 }
 
 // --------------------------------------------------------------- launchers
+// The mode sum with two particles a thread: from one 256-particle tile per SM
+// (152 of them) on -- below, half as many warps hide less latency than the
+// shared reads save (32,768 particles: 1.74 against 1.65 ms; 65,536: 2.80
+// against 2.97; 155,648: 5.27 against 5.91) -- and up to the modes whose
+// records leave room for two blocks (1,000 modes, 65,536 particles: 4.73
+// against 5.79 ms).
+constexpr int kPairParticles = 152 * 2 * kBlock;
+constexpr int kPairModes = 1024;
 template <int SYS>
 static cudaError_t launch_sys(const MixField& f, const TrackBufs& b, const TrackParams& q, int grid,
                               cudaStream_t s)
@@ -305,6 +522,19 @@ static cudaError_t launch_sys(const MixField& f, const TrackBufs& b, const Track
     return cudaGetLastError();
 }
 
+static cudaError_t launch_modes(const MixField& f, const TrackBufs& b, const TrackParams& q, int grid,
+                                cudaStream_t s)
+{
+    const size_t smem = sizeof(ModePair) * (size_t)((f.nmodes + 1) / 2) +
+                        sizeof(unsigned int) * (size_t)(q.nbins <= kMaxSmemBins ? q.nbins : 0);
+    cudaError_t e = cudaFuncSetAttribute(track_modes_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    TrackParams qq = q;
+    qq.ntiles = (q.n + 2 * kBlock - 1) / (2 * kBlock);
+    track_modes_kernel<2><<<std::min(grid, qq.ntiles), kBlock, smem, s>>>(f, b, qq);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_track(const MixField& f, const TrackBufs& b, const TrackParams& q, int grid,
                          cudaStream_t s)
 {
@@ -312,7 +542,9 @@ cudaError_t launch_track(const MixField& f, const TrackBufs& b, const TrackParam
     case TP_SYS_TEST: return launch_sys<TP_SYS_TEST>(f, b, q, grid, s);
     case TP_SYS_FORCEFREE: return launch_sys<TP_SYS_FORCEFREE>(f, b, q, grid, s);
     case TP_SYS_PIC: return launch_sys<TP_SYS_PIC>(f, b, q, grid, s);
-    case TP_SYS_MODESUM: return launch_sys<TP_SYS_MODESUM>(f, b, q, grid, s);
+    case TP_SYS_MODESUM:
+        if (f.nmodes <= kPairModes && q.n >= kPairParticles) return launch_modes(f, b, q, grid, s);
+        return launch_sys<TP_SYS_MODESUM>(f, b, q, grid, s);
     default: return cudaErrorInvalidValue;
     }
 }

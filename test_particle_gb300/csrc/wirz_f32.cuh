@@ -42,6 +42,103 @@ __device__ __forceinline__ void advance(uint64_t& X, int& img, float fr)
     X = nx;
 }
 
+// The push in two halves, split at its second field evaluation, for kernels
+// that evaluate the field of several particles at once: the operations of
+// wirz_f32 below in the same order, results bit for bit the same.  (wirz_f32
+// composed of the two ran the ABC field 2 % and the gridded field 0.8 %
+// slower.)
+
+// What the first half of a push hands to its second half.
+struct WirzMid {
+    float um[3];   // momentum after the first half kick
+    float ig;      // 1 / gamma of it
+};
+
+// First half of a Wirz push, from the field E, B at the particle: the half
+// kick and the midpoint Xp where the field is sampled next.
+__device__ __forceinline__ void wirz_first(const MixField& f, const PM& p, float dt, const float E[3],
+                                           const float B[3], WirzMid& m, uint64_t Xp[3])
+{
+    // Norms and their inverses come from one rsqrt each (a single SFU
+    // operation, a few ulp): the FP32 path's error budget is set by FP32
+    // rounding of the push, not by these.
+    const float cm = f.cm, icm = 1.0f / f.cm;
+    float B2 = B[0] * B[0] + B[1] * B[1] + B[2] * B[2];
+    float iB = rsqrtf(B2);
+    float Btot = B2 * iB;
+    float h[3] = {B[0] * iB, B[1] * iB, B[2] * iB};
+    const float hk = 0.5f * cm * dt;
+#pragma unroll
+    for (int k = 0; k < 3; k++) m.um[k] = p.u[k] + hk * E[k];
+    const float* um = m.um;
+    m.ig = rsqrtf(1.0f + um[0] * um[0] + um[1] * um[1] + um[2] * um[2]);  // 1 / gamma
+    // frame at the start point
+    float w[3] = {h[1] * um[2] - h[2] * um[1], h[2] * um[0] - h[0] * um[2], h[0] * um[1] - h[1] * um[0]};
+    float w2 = w[0] * w[0] + w[1] * w[1] + w[2] * w[2];
+    float iu = w2 > 0.0f ? rsqrtf(w2) : 0.0f;
+    float uperp = w2 * iu;
+    float hr[3] = {w[0] * iu, w[1] * iu, w[2] * iu};
+    float hp[3] = {hr[1] * h[2] - hr[2] * h[1], hr[2] * h[0] - hr[0] * h[2], hr[0] * h[1] - hr[1] * h[0]};
+    float upar = um[0] * h[0] + um[1] * h[1] + um[2] * h[2];
+    float theta = cm * Btot * m.ig * dt;
+    float s4, c4;
+    __sincosf(0.25f * theta, &s4, &c4);
+    float sin_h = 2.0f * s4 * c4, omc_h = 2.0f * s4 * s4;  // sin(theta/2), 1 - cos(theta/2)
+    float R = uperp * iB * icm;  // uperp / (cm |B|)
+    float a1 = 0.5f * dt * upar * m.ig, a2 = R * sin_h, a3 = -R * omc_h;
+    float dpre[3];
+#pragma unroll
+    for (int k = 0; k < 3; k++) dpre[k] = (h[k] * a1 + hp[k] * a2 + hr[k] * a3) * f.invL[k];
+    // The midpoint is only sampled, and the field evaluations read the top 32
+    // bits of a position: a 32-bit fixed-point step is enough there.
+#pragma unroll
+    for (int k = 0; k < 3; k++)
+        Xp[k] = (uint64_t)((uint32_t)(p.X[k] >> 32) + (uint32_t)__float2int_rn(dpre[k] * 4294967296.0f)) << 32;
+}
+
+// Second half, from the field at the midpoint: momentum and position.
+__device__ __forceinline__ void wirz_second(const MixField& f, PM& p, float dt, const float E[3], const float B[3],
+                                            const WirzMid& m, bool& escaped)
+{
+    const float cm = f.cm, icm = 1.0f / f.cm;
+    const float hk = 0.5f * cm * dt;
+    const float *um = m.um, ig = m.ig;
+    float B2 = B[0] * B[0] + B[1] * B[1] + B[2] * B[2];
+    float iB = rsqrtf(B2);
+    float Btot = B2 * iB;
+    float h[3] = {B[0] * iB, B[1] * iB, B[2] * iB};
+    float w[3] = {h[1] * um[2] - h[2] * um[1], h[2] * um[0] - h[0] * um[2], h[0] * um[1] - h[1] * um[0]};
+    float w2 = w[0] * w[0] + w[1] * w[1] + w[2] * w[2];
+    float iu = w2 > 0.0f ? rsqrtf(w2) : 0.0f;
+    float uperp = w2 * iu;
+    float hr[3] = {w[0] * iu, w[1] * iu, w[2] * iu};
+    float hp[3] = {hr[1] * h[2] - hr[2] * h[1], hr[2] * h[0] - hr[0] * h[2], hr[0] * h[1] - hr[1] * h[0]};
+    float upar = um[0] * h[0] + um[1] * h[1] + um[2] * h[2];
+    float theta = cm * Btot * ig * dt;
+    float s2, c2;
+    __sincosf(0.5f * theta, &s2, &c2);
+    float sn = 2.0f * s2 * c2, omc = 2.0f * s2 * s2;  // sin(theta), 1 - cos(theta)
+    float cs = 1.0f - omc;
+#pragma unroll
+    for (int k = 0; k < 3; k++) p.u[k] = h[k] * upar + uperp * (cs * hp[k] - sn * hr[k]) + hk * E[k];
+    float R = uperp * iB * icm;
+    float a1 = dt * upar * ig;
+    float a2 = R * sn;
+    float a3 = -R * omc;
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        float d = (h[k] * a1 + hp[k] * a2 + hr[k] * a3) * f.invL[k];
+        if (f.bc_flag == 1) {
+            // open boundary: leaving the box is an escape, not a wrap
+            int before = p.img[k];
+            advance(p.X[k], p.img[k], d);
+            if (p.img[k] != before) escaped = true;
+        } else {
+            advance(p.X[k], p.img[k], d);
+        }
+    }
+}
+
 // One Wirz push; field(X, E, B) evaluates the field at a fixed-point position.
 template <class FieldFn>
 __device__ __forceinline__ void wirz_f32(const MixField& f, PM& p, float dt, FieldFn&& field,
