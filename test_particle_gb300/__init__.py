@@ -236,19 +236,20 @@ def track(ptl_init, dt, nt_out, nbins, precision=PREC_FP64, ptl=None):
     """Fixed-step tracking of all particles on the GPU (host buffers in and out)."""
     L = lib()
     p0 = np.ascontiguousarray(ptl_init, dtype=PARTICLE_DTYPE)
-    p = p0.copy() if ptl is None else np.array(ptl, dtype=PARTICLE_DTYPE, copy=True)
+    start = p0 if ptl is None else np.ascontiguousarray(ptl, dtype=PARTICLE_DTYPE)
     n = len(p0)
+    p = np.empty(n, dtype=PARTICLE_DTYPE)
     estep = int(Domain.in_dll(L, "simul_domain").tmax / dt)
     nsdc = estep // 100 + 1
     esp = np.zeros(nt_out * nbins)
     ese = np.zeros(nt_out * nbins)
     dsum = np.zeros(8 * nsdc)
     rem = np.zeros(nsdc, dtype=np.int32)
-    nst = np.zeros(n, dtype=np.int32)
+    nst = np.empty(n, dtype=np.int32)
     info = RunInfo()
-    check(L.tp_track_host(C.c_int(precision), C.c_int(n), C.c_double(dt), C.c_int(nt_out),
-                          C.c_int(nbins), _ptr(p0), _ptr(p), _ptr(nst), _ptr(esp), _ptr(ese),
-                          _ptr(dsum), _ptr(rem), C.byref(info)), "track")
+    check(L.tp_track_host_to(C.c_int(precision), C.c_int(n), C.c_double(dt), C.c_int(nt_out),
+                             C.c_int(nbins), _ptr(p0), _ptr(start), _ptr(p), _ptr(nst), _ptr(esp), _ptr(ese),
+                             _ptr(dsum), _ptr(rem), C.byref(info)), "track")
     return dict(ptl=p, estep=info.estep, espect=esp.reshape(nt_out, nbins),
                 espect_escape=ese.reshape(nt_out, nbins), dsum=dsum.reshape(8, nsdc),
                 remain=rem, nsteps=nst, info=info)

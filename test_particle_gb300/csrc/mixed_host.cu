@@ -174,6 +174,10 @@ extern "C" int tp_get_emf_mixed_batch(int n, const double* xyz, float* emf6)
     mixed::MixField mf;
     if (!build_mixfield(system_type, mf, nullptr)) return -1;
     if (n <= 0) return 0;
+    if (in_place(xyz, 8) && in_place(emf6, 4)) {
+        if (!cuda_ok(mixed::launch_emf_batch(mf, n, xyz, emf6, g.stream), "emf mixed")) return -1;
+        return cuda_ok(cudaStreamSynchronize(g.stream), "emf mixed sync") ? 0 : -1;
+    }
     double* d_in = (double*)g.s_batch_a.get(sizeof(double) * 3 * (size_t)n);
     float* d_out = (float*)g.s_batch_b.get(sizeof(float) * 6 * (size_t)n);
     if (!d_in || !d_out) return -1;

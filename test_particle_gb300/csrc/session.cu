@@ -4,6 +4,7 @@
 #include <climits>
 #include <cmath>
 #include <cstring>
+#include <unistd.h>
 
 #include "../../include/tp_gpu.h"
 #include "tp_internal.h"
@@ -193,20 +194,29 @@ bool Session::load(const particles* ptl_init, const particles* ptl, int n_)
     if (!reserve(n_)) return false;
     n = n_;
     cudaStream_t s = g.stream;
-    double* a = (double*)aos.ptr;
+    double *S = (double*)soa.ptr, *S0 = (double*)soa0.ptr;
+    auto records = [&](const particles* host, double* to, double* also) {
+        const double* src = (const double*)host;
+        if (!in_place(host, 8)) {
+            if (!cuda_ok(cudaMemcpyAsync(aos.ptr, host, sizeof(particles) * n, cudaMemcpyHostToDevice, s), "load"))
+                return false;
+            src = (const double*)aos.ptr;
+        }
+        aos_to_soa(src, n, to, also, cap, s);
+        return true;
+    };
     if (n > 0) {
-        if (!cuda_ok(cudaMemcpyAsync(a, ptl_init, sizeof(particles) * n, cudaMemcpyHostToDevice, s),
-                     "load init")) return false;
-        aos_to_soa(a, n, (double*)soa0.ptr, cap, s);
-        if (!cuda_ok(cudaMemcpyAsync(a, ptl, sizeof(particles) * n, cudaMemcpyHostToDevice, s),
-                     "load ptl")) return false;
-        aos_to_soa(a, n, (double*)soa.ptr, cap, s);
+        if (ptl == ptl_init) {
+            if (!records(ptl, S, S0)) return false;
+        } else if (!records(ptl_init, S0, nullptr) || !records(ptl, S, nullptr)) {
+            return false;
+        }
     }
     loaded = true;
     return cuda_ok(cudaGetLastError(), "load");
 }
 
-bool Session::run(const RunSpec& rs, tp_run_info* info)
+bool Session::run(const RunSpec& rs, tp_run_info* info, const std::function<void()>& meanwhile)
 {
     if (!loaded) {
         set_error(1, "session: particles not loaded");
@@ -359,6 +369,7 @@ bool Session::run(const RunSpec& rs, tp_run_info* info)
     cudaEventRecord(ev0, s);
     if (!segs) {
         if (!cuda_ok(launch(q, grid), "track launch")) return false;
+        if (meanwhile) meanwhile();
     } else {
         b.sg_carry = c_sg;
         b.esc_out = c_esc;
@@ -381,6 +392,7 @@ bool Session::run(const RunSpec& rs, tp_run_info* info)
             if (qs.resumed) qs.ntp0 = q.ntp0 + (s0 - 1) / rs.einterval;
             if (!cuda_ok(launch(qs, std::min(grid, qs.ntiles)), "track launch")) return false;
             launches++;
+            if (meanwhile && !qs.resumed) meanwhile();
             if (e0 >= rs.estep) break;
             const int nblk = (n_act + kCmpBlock - 1) / kCmpBlock;
             seg_count_kernel<<<nblk, kCmpBlock, 0, s>>>(cur, n_act, c_esc, c_sg, c_cnt, c_part);
@@ -431,8 +443,9 @@ bool Session::fetch(particles* ptl, int* nsteps_ptl, double* espect, double* esp
 {
     cudaStream_t s = g.stream;
     if (ptl && n > 0) {
-        soa_to_aos((const double*)soa.ptr, n, cap, (double*)aos.ptr, s);
-        cudaMemcpyAsync(ptl, aos.ptr, sizeof(particles) * n, cudaMemcpyDeviceToHost, s);
+        const bool direct = in_place(ptl, 8);
+        soa_to_aos((const double*)soa.ptr, n, cap, direct ? (double*)ptl : (double*)aos.ptr, s);
+        if (!direct) cudaMemcpyAsync(ptl, aos.ptr, sizeof(particles) * n, cudaMemcpyDeviceToHost, s);
     }
     if (nsteps_ptl && n > 0)
         cudaMemcpyAsync(nsteps_ptl, nsteps.ptr, sizeof(int) * n, cudaMemcpyDeviceToHost, s);
@@ -528,7 +541,7 @@ extern "C" void tp_session_destroy(tp_session* s) { delete s; }
 
 extern "C" int tp_session_load(tp_session* s, const particles* ptl_init, const particles* ptl)
 {
-    return s && s->s.load(ptl_init, ptl, s->s.cap) ? 0 : -1;
+    return s && s->s.load(ptl_init, ptl, s->s.cap) && cuda_ok(cudaStreamSynchronize(g.stream), "load") ? 0 : -1;
 }
 
 extern "C" int tp_session_track(tp_session* s, int precision, double dt, int nt_out, int nbins,
@@ -550,10 +563,19 @@ extern "C" int tp_session_fetch(tp_session* s, particles* ptl, int* nsteps_ptl, 
     return s && s->s.fetch(ptl, nsteps_ptl, espect, espect_escape, dsum, remain) ? 0 : -1;
 }
 
-extern "C" int tp_track_host(int precision, int nptl, double dt, int nt_out, int nbins,
-                             const particles* ptl_init, particles* ptl, int* nsteps_ptl,
-                             double* espect, double* espect_escape, double* dsum, int* remain,
-                             tp_run_info* info)
+// Maps the pages of a buffer that is about to be written: a fresh allocation's
+// pages are zeroed one by one at their first touch, 10 GB/s on one core, which
+// the tracking kernel's time hides.
+static void touch_pages(void* p, size_t bytes)
+{
+    const size_t page = (size_t)sysconf(_SC_PAGESIZE);
+    for (size_t i = 0; i < bytes; i += page) ((volatile char*)p)[i] = 0;
+}
+
+extern "C" int tp_track_host_to(int precision, int nptl, double dt, int nt_out, int nbins,
+                                const particles* ptl_init, const particles* ptl, particles* ptl_out,
+                                int* nsteps_ptl, double* espect, double* espect_escape, double* dsum,
+                                int* remain, tp_run_info* info)
 {
     Session& s = cached_session();
     RunSpec rs;
@@ -563,9 +585,25 @@ extern "C" int tp_track_host(int precision, int nptl, double dt, int nt_out, int
     rs.nt_out = nt_out;
     rs.nbins = nbins;
     if (!s.load(ptl_init, ptl, nptl)) return -1;
-    if (!s.run(rs, info)) return -1;
-    if (!s.fetch(ptl, nsteps_ptl, espect, espect_escape, dsum, remain)) return -1;
+    auto meanwhile = [&] {
+        if (nptl > 0 && ptl_out != ptl && ptl_out != ptl_init) touch_pages(ptl_out, sizeof(particles) * (size_t)nptl);
+        if (nptl > 0 && nsteps_ptl) touch_pages(nsteps_ptl, sizeof(int) * (size_t)nptl);
+    };
+    if (!s.run(rs, info, meanwhile)) {
+        cudaStreamSynchronize(g.stream);  // the records may still be read in place
+        return -1;
+    }
+    if (!s.fetch(ptl_out, nsteps_ptl, espect, espect_escape, dsum, remain)) return -1;
     if (remain)  // the kernel counts departures; the reference starts from nptl
         for (int k = 0; k < s.nsdc; k++) remain[k] += nptl;
     return 0;
+}
+
+extern "C" int tp_track_host(int precision, int nptl, double dt, int nt_out, int nbins,
+                             const particles* ptl_init, particles* ptl, int* nsteps_ptl,
+                             double* espect, double* espect_escape, double* dsum, int* remain,
+                             tp_run_info* info)
+{
+    return tp_track_host_to(precision, nptl, dt, nt_out, nbins, ptl_init, ptl, ptl, nsteps_ptl, espect,
+                            espect_escape, dsum, remain, info);
 }

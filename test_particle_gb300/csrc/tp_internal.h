@@ -30,6 +30,7 @@ struct Ctx {
     bool inited = false;
     int device = 0;
     int num_sms = 0;
+    bool direct = false;     // kernels may address the host's memory (shared page tables)
     cudaStream_t stream = nullptr;
     int* d_status = nullptr;
     int status = 0;
@@ -85,7 +86,12 @@ bool fixed_modes(const std::vector<tp_mode>& modes, std::vector<fx::Mode>& out, 
 const void* dd0(Mirror& m, const void* h, size_t b, cudaStream_t s);
 bool ensure_thresholds(int nbins);
 bool compute_thresholds(int nbins, double lmin, double lde, std::vector<double>& thr);
-void aos_to_soa(const double* d_aos, int n, double* d_soa, long stride, cudaStream_t s);
-void soa_to_aos(const double* d_soa, int n, long stride, double* d_aos, cudaStream_t s);
+// A host buffer that kernels may read or write in place: the device walks the
+// host's page tables, and elements are aligned.  Work on it has to be waited
+// for before the caller gets its buffer back.
+inline bool in_place(const void* host, size_t align) { return g.direct && ((uintptr_t)host & (align - 1)) == 0; }
+// particles records to columns (both when soa2 is given) and back
+void aos_to_soa(const double* aos, int n, double* d_soa, double* d_soa2, long stride, cudaStream_t s);
+void soa_to_aos(const double* d_soa, int n, long stride, double* aos, cudaStream_t s);
 
 }  // namespace tp

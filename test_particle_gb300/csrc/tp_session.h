@@ -1,5 +1,7 @@
 // tp_session.h -- the device-resident tracking session behind the C ABI.
 #pragma once
+#include <functional>
+
 #include "../../include/tp_gpu.h"
 #include "tp_internal.h"
 
@@ -32,8 +34,11 @@ struct Session {
     float last_ms = 0.f;
     ~Session();
     bool reserve(int n);
+    // (may read the host's records in place: wait for the stream before the
+    // caller may change them)
     bool load(const particles* ptl_init, const particles* ptl, int n);
-    bool run(const RunSpec& rs, tp_run_info* info);
+    // meanwhile: host work done once the first kernel is launched
+    bool run(const RunSpec& rs, tp_run_info* info, const std::function<void()>& meanwhile = nullptr);
     // remain: departures counted on the device (negative numbers)
     bool fetch(particles* ptl, int* nsteps_ptl, double* espect, double* espect_escape,
                double* dsum, int* remain);
