@@ -99,9 +99,10 @@ __host__ __device__ __forceinline__ void cosine(uint64_t ph, const int4* tab, in
 
 // The six components at the point with box fractions u (64-bit fixed point),
 // as integers to be multiplied with the components' scales.  nm is a multiple
-// of kChunk (tables are padded with zero amplitudes).
+// of kChunk (tables are padded with zero amplitudes).  Chunks first, first +
+// step, ... only: the sums of all of them add up exactly.
 __host__ __device__ __forceinline__ void mode_sum(const Mode* modes, int nm, const int4* tab, const uint64_t u[3],
-                                                  int64_t out[6])
+                                                  int64_t out[6], int first = 0, int step = 1)
 {
     // u = uh 2^32 + ul with signed ul, so that n u mod 2^64 takes signed products
     int32_t ul[3];
@@ -111,7 +112,7 @@ __host__ __device__ __forceinline__ void mode_sum(const Mode* modes, int nm, con
         uh[k] = (uint32_t)(u[k] >> 32) + (uint32_t)(ul[k] < 0);
     }
     int64_t hh[6] = {0, 0, 0, 0, 0, 0}, mid[6] = {0, 0, 0, 0, 0, 0};
-    for (int m0 = 0; m0 < nm; m0 += kChunk) {
+    for (int m0 = first * kChunk; m0 < nm; m0 += step * kChunk) {
 #ifdef __CUDA_ARCH__
 #pragma unroll 4
 #endif

@@ -279,6 +279,17 @@ bool Session::run(const RunSpec& rs, tp_run_info* info, const std::function<void
         grid = resident * kBlockWaves;
     if (grid > ntiles) grid = ntiles;
     if (grid < 1) grid = 1;
+    // FP64 runs too small to fill the machine: four lanes a particle.  (Not
+    // where segments are asked for; and with contraction the two kernels agree
+    // to rounding only, so that open-boundary runs, whose segments have to
+    // continue exactly, keep the one.)
+    int small = 0;
+    const bool contracted = rs.precision == TP_PREC_FP64_FAST;
+    if (!is_mixed && !is_surr && rs.traj_every == 0 && !(bc_flag == 1 && (contracted || g.compact_steps > 0))) {
+        small = rs.precision == TP_PREC_FP64 ? fp64::track_small_blocks(f, n, g.num_sms)
+                                                : fp64fast::track_small_blocks(f, n, g.num_sms);
+        if (small > 0) grid = small;
+    }
     // open boundaries: segments of seg steps with the departed particles
     // dropped.  Automatic mode: only when the tiles take more than one wave of
     // the grid (within one wave an idle lane costs nothing), about 8 segments
@@ -290,7 +301,7 @@ bool Session::run(const RunSpec& rs, tp_run_info* info, const std::function<void
                                   : (long long)std::max(kDiffInterval, rs.estep / (is_mixed ? 8 : 32));
     seg_ll = (seg_ll + kDiffInterval - 1) / kDiffInterval * kDiffInterval;
     const bool segs = bc_flag == 1 && g.compact_steps != 0 && rs.traj_every == 0 && !is_surr &&
-                      rs.sstep == 1 && (long long)rs.estep > seg_ll && n > 0 &&
+                      rs.sstep == 1 && (long long)rs.estep > seg_ll && n > 0 && small == 0 &&
                       (!automatic || ntiles > resident);
     const int seg = (int)std::min<long long>(seg_ll, rs.estep);  // < estep whenever segs
     const int nslot = grid + (segs ? 1 : 0);  // the last slot takes the departed particles' rows
@@ -360,6 +371,9 @@ bool Session::run(const RunSpec& rs, tp_run_info* info, const std::function<void
     q.traj_every = rs.traj_every;
     q.dt = rs.dt;
     auto launch = [&](const TrackParams& qq, int gr) {
+        if (small > 0)
+            return rs.precision == TP_PREC_FP64 ? fp64::launch_track_small(f, b, qq, g.num_sms, s)
+                                                : fp64fast::launch_track_small(f, b, qq, g.num_sms, s);
         return rs.precision == TP_PREC_FP64 ? fp64::launch_track(f, b, qq, gr, s)
              : is_mixed ? mixed::launch_track(mf, b, qq, gr, s)
              : is_surr  ? mlp::launch_track_surrogate(mf, md, b, qq, gr, s)

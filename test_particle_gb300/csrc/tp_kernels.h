@@ -9,6 +9,9 @@ namespace tp {
     cudaError_t launch_track(const DevField& f, const TrackBufs& b, const TrackParams& q,      \
                              int grid, cudaStream_t s);                                        \
     int track_max_blocks_per_sm(int system_type);                                              \
+    int track_small_blocks(const DevField& f, int n, int num_sms);                             \
+    cudaError_t launch_track_small(const DevField& f, const TrackBufs& b, const TrackParams& q, \
+                                   int num_sms, cudaStream_t s);                               \
     cudaError_t launch_reduce_dpart(const double* dpart, int nblocks, int nsdc, double* dsum,  \
                                     cudaStream_t s);                                           \
     cudaError_t launch_emf_batch(const DevField& f, int n, const double* xyzt, double* out,    \

@@ -4,6 +4,8 @@
 //
 // Built twice: with -fmad=false as the parity path (TP_FP64_NS = fp64) and
 // with -fmad=true as the fast FP64 path (TP_FP64_NS = fp64fast, -DTP_FAST).
+#include <algorithm>
+
 #include "fields_fp64.cuh"
 #include "tp_kernels.h"
 
@@ -358,6 +360,8 @@ __global__ void __launch_bounds__(32 * kReduceRows) reduce_dpart_kernel(const do
         dsum[(k & 7) * nsdc + (k >> 3)] = t;
     }
 }
+
+#include "track_small.cuh"
 
 // ---------------------------------------------------------------- batch utilities
 __global__ void emf_batch_kernel(DevField f, int n, const double* xyzt, double* out, int* status)
