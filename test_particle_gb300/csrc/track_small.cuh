@@ -12,8 +12,8 @@
 // sum), and one wire or loop a warp for the block's 32 particles (current
 // systems), through shared memory; gridded fields are evaluated by every lane.
 // Every particle's operations and their order are those of track_kernel.
-// 256 particles x 200 steps, ABC: 3.05 -> @ABC@ ms; 4,096 x 200, two wires and
-// loops: 23.1 -> @WLCS@ ms.
+// Whole runs: 256 particles x 200 steps, ABC, 3.11 -> 1.79 ms; 4,096 x 200, two
+// wires and loops, 23.2 -> 9.2 ms.
 #pragma once
 
 constexpr int kSmallTile = 32;      // particles a block
@@ -209,19 +209,17 @@ __global__ void __launch_bounds__(128) track_small_kernel(DevField f, TrackBufs 
     const int i = blockIdx.x * kSmallTile + (threadIdx.x >> 2);
     const int c = (threadIdx.x & 3) == 3 ? 0 : threadIdx.x & 3;
     const bool active = i < q.n, lead = (threadIdx.x & 3) == 0;
-    double x = 0.0, u = 0.0, xs = 0.0, t = 0.0;
-    int nst = 1;
-    if (active) {
-        x = (c == 0 ? b.x : c == 1 ? b.y : b.z)[i];
-        u = (c == 0 ? b.ux : c == 1 ? b.uy : b.uz)[i];
-        xs = (c == 0 ? b.xs : c == 1 ? b.ys : b.zs)[i];
-        t = b.t[i];
-        nst = b.nsteps_ptl[i];
-    }
+    // groups past the end follow the last particle and write nothing (a group
+    // at rest would divide zeros by zeros and take the FP64 instructions for it)
+    const int il = min(i, q.n - 1);
+    double x = (c == 0 ? b.x : c == 1 ? b.y : b.z)[il];
+    double u = (c == 0 ? b.ux : c == 1 ? b.uy : b.uz)[il];
+    double xs = (c == 0 ? b.xs : c == 1 ? b.ys : b.zs)[il];
+    double t = b.t[il];
+    int nst = b.nsteps_ptl[il];
     // a group's escape: any of its lanes out of the box
     auto group_any = [&](bool v) { return (__ballot_sync(0xffffffffu, v) >> (threadIdx.x & 28) & 7u) != 0u; };
-    bool out = false;
-    if (active) out = small_bc(f, c, x, xs);
+    const bool out = small_bc(f, c, x, xs);
     bool esc_pre = group_any(out), esc_after = esc_pre;
     int ntp = q.ntp0, tstep = 1;
     double sg[8] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
@@ -234,7 +232,7 @@ __global__ void __launch_bounds__(128) track_small_kernel(DevField f, TrackBufs 
         const bool diff = to_diff == 0, frame = to_frame == 0;
         to_diff = diff ? kDiffInterval - 1 : to_diff - 1;
         to_frame = frame ? q.einterval - 1 : to_frame - 1;
-        const bool moves = active && (!esc_pre || f.bc_flag == 0);
+        const bool moves = !esc_pre || f.bc_flag == 0;
         sg[0] = 0.0; sg[4] = 0.0; sg[5] = 0.0;  // src/tracking.c:334-336
         double xn = x, un = u, tn = t, xsn = xs;
         small_wirz<SYS>(f, c, xn, un, tn, q.dt, sh, active ? b.status : nullptr);
@@ -292,8 +290,7 @@ static cudaError_t launch_small_sys(const DevField& f, const TrackBufs& b, const
     const int blocks = (q.n + kSmallTile - 1) / kSmallTile;
     size_t smem = SYS == TP_SYS_MODESUM ? sizeof(int4) * (fx::kTab + 1) : 0;
     // up to one block an SM, each asks for more than half of an SM's shared
-    // memory: the hardware otherwise puts two on one SM when it has 32 to 94
-    // to place, whose warps then share FP64 pipes (ABC: 2.98 against 1.70 ms)
+    // memory, so that no two share one's FP64 pipes
     if (blocks <= num_sms) smem = std::max(smem, (size_t)120 * 1024);
     if (smem > 0) {
         cudaError_t e = cudaFuncSetAttribute(track_small_kernel<SYS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -305,14 +302,16 @@ static cudaError_t launch_small_sys(const DevField& f, const TrackBufs& b, const
 }
 
 // Blocks of a small run of this field, or 0: track_kernel is the better or the
-// only one for it.  One block an SM for the push-bound fields (ABC, 200 steps:
-// 4,864 particles 1.70 against 3.05 ms, 5,000 particles 3.53 against 3.15;
-// 256^3 grid, 50 steps: 0.86 against 1.10, 1.61 against 1.15); two for the
-// current systems (9,728 particles x 40 steps: 2.39 against 4.60 ms; 16,000:
-// slower); three for the mode sum (16,000 x 10 steps: 1.69 against 2.30 ms).
+// only one for it.  Whole runs, host buffers in and out: ABC, 200 steps, 3.0 ms
+// in track_kernel up to its first full wave against 1.8 with one block an SM
+// here, 2.1 with two, 2.8 with three; 256^3 grid, 50 steps, 1.24 against 0.95,
+// 1.25 and 1.64 (every lane evaluates the grid); two wires and loops, 40 steps,
+// 4.6 against 1.8 and 2.4; mode sum, 10 steps, 2.3 against 0.7, 1.0 and 1.7
+// with four.
 int track_small_blocks(const DevField& f, int n, int num_sms)
 {
-    const int per_sm = f.system_type == TP_SYS_MODESUM ? 3 : f.system_type == TP_SYS_WLCS ? 2 : 1;
+    const bool grids = f.system_type == TP_SYS_PIC || f.system_type == TP_SYS_MHD;
+    const int per_sm = f.system_type == TP_SYS_MODESUM ? 4 : grids ? 2 : 3;
     const int blocks = (n + kSmallTile - 1) / kSmallTile;
     if (n < 1 || blocks > per_sm * num_sms) return 0;
     if (f.system_type == TP_SYS_WLCS && f.nwlcs > kSmallSystems) return 0;

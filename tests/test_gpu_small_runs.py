@@ -11,7 +11,7 @@ tp = pytest.importorskip("test_particle_gb300")
 import test_particle_gb300.workloads as wl  # noqa: E402
 
 SC = mg.scenarios()
-LARGE = 3 * 152 * 32 + 1  # more particles than any small run takes
+LARGE = 4 * 152 * 32 + 1  # more particles than any small run takes
 
 
 def _configure(name, bc):
