@@ -50,3 +50,25 @@ def test_small_matches_large(name, bc, n):
     assert np.array_equal(few["remain"] - n, sum(r["remain"] - 1 for r in parts))
     total = sum(r["dsum"] for r in parts)
     assert np.all(np.abs(few["dsum"] - total) <= n * 2.0 ** -52 * np.abs(total))
+
+
+@pytest.mark.parametrize("n,off", [(1, 0.0), (9, 0.0), (257, -0.75)])
+def test_few_field_lines_match_many(n, off):
+    """Field lines of few seeds (four lanes a seed) against the same seeds in a
+    map of more than 16,384, and seeds outside the box as the reference wraps them."""
+    g = tp.Grids()
+    g.nx, g.ny, g.nz, g.nt = 17, 13, 15, 1
+    g.dx, g.dy, g.dz = 0.25, 0.3, 0.2
+    dom = tp.Domain()
+    dom.xmin, dom.ymin, dom.zmin = off, 0.0, 0.0
+    dom.xmax, dom.ymax, dom.zmax = off + 16 * 0.25, 12 * 0.3, 14 * 0.2
+    rng = np.random.default_rng(11)
+    b = (rng.normal(0, 0.4, (17 * 13 * 15, 3)) + [0.0, 0.0, 1.0]).astype(np.float32)
+    tp.configure(system_type=tp.SYS_PIC, dom=dom, grd=g, bgrid=b, egrid=np.zeros_like(b))
+    seeds = [off, 0.0, 0.0] + rng.random((16385, 3)) * [4.0, 3.6, 2.8]
+    seeds[:, 2] = 1.4
+    seeds[0] = [off + 5.0, 1.0, 1.4]
+    many = tp.poincare_trace(seeds, 2, 0.05, 20.0, 3)
+    few = tp.poincare_trace(seeds[:n], 2, 0.05, 20.0, 3)
+    for m, w in zip(many, few):
+        assert m[:n].tobytes() == w.tobytes()
