@@ -191,6 +191,19 @@ bool build_field(int stype, DevField& f)
         }
         g.m_cfg.dirty = true;  // tiny; always refreshed
         f.cfg = (const wlcs*)(nwlcs > 0 ? dd0(g.m_cfg, config, sizeof(wlcs) * nwlcs, s) : nullptr);
+        g.loop_pre.resize(nwlcs > 0 ? nwlcs : 0);
+        for (int i = 0; i < nwlcs; i++) {
+            const wlcs& w = config[i];
+            LoopPre& o = g.loop_pre[i];
+            const double cur = w.cur_lp * TP_I0;
+            o.al = w.r_lp * TP_L0;
+            o.al2 = o.al * o.al;
+            o.al4 = 4.0 * o.al;
+            o.Irho = 0.2 * cur;
+            o.flat = w.cosbeta_lp == 1.0 && w.sinbeta_lp == 0.0 && w.cosalpha_lp == 1.0 && w.sinalpha_lp == 0.0;
+        }
+        g.m_pre.dirty = true;
+        f.pre = (const LoopPre*)(nwlcs > 0 ? dd0(g.m_pre, g.loop_pre.data(), sizeof(LoopPre) * nwlcs, s) : nullptr);
         f.nwlcs = nwlcs;
         f.iBessel = iBessel;
     } else if (stype == TP_SYS_MODESUM) {

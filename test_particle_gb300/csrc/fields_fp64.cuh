@@ -313,6 +313,21 @@ __device__ __forceinline__ void wl_reverse(double& ax, double& ay, double& az, d
 
 // ellint, src/wlcs.c:460-809 (Fukushima 2009), coefficient tables recomputed
 // from the mathematics (gen_ellint_coeffs.py)
+// The division and square root of the loop's field as calls and its series
+// rolled (TP_SOFT_CALLS), or all inline.  The adaptive stepper, whose warps sit
+// at different points of a long loop body, calls them: inlined it waited for
+// code 38 % of the time (65,536 particles: 433 -> 389 ms).  The fixed-step
+// kernels, whose warps run in step, are 3 % faster inline.
+#ifdef TP_SOFT_CALLS
+constexpr int kEllUnroll = 4;
+static __device__ __noinline__ double soft_div(double a, double b) { return sd::div(a, b); }
+static __device__ __noinline__ double soft_sqrt(double x) { return sd::sqrt_rn(x); }
+#else
+constexpr int kEllUnroll = 20;
+__device__ __forceinline__ double soft_div(double a, double b) { return sd::div(a, b); }
+__device__ __forceinline__ double soft_sqrt(double x) { return sd::sqrt_rn(x); }
+#endif
+
 __device__ __forceinline__ void ellint64(const DevField& f, double k, int corrected, double& elle, double& ellf)
 {
     double m = k * k;
@@ -336,7 +351,7 @@ __device__ __forceinline__ void ellint64(const DevField& f, double k, int correc
         // sums are those of the interval's own length while the lanes of a
         // warp, whatever their intervals, take the same loop
         double m1 = m - __ldg(&tp_ell_m0[i]), powj = 1.0;
-#pragma unroll
+#pragma unroll kEllUnroll
         for (int j = 0; j < TP_ELL_NK_MAX; j++) {
             double kc = __ldg(&tp_ell_k[i][j]);
             if (!corrected && i == 9 && j == 19) kc = TP_ELL_K9_19_REF;
@@ -346,26 +361,27 @@ __device__ __forceinline__ void ellint64(const DevField& f, double k, int correc
         }
         return;
     }
+    // the powers of the third series, in 0.95 - m, are those of the first up to
+    // sign (the reference's first series runs in m - 0.95): one chain for both,
+    // the sign on the coefficient's bits
     double ellf1 = 0.0, q1 = 0.0, hm = 0.0, powj = 1.0;
-    double m1 = corrected ? (0.95 - m) : (m - 0.95);
+    const double m1 = corrected ? (0.95 - m) : (m - 0.95), mq = 1.0 - m;
+    double powq = mq;
+    const uint64_t flip = corrected ? 0ull : 0x8000000000000000ull;
+#pragma unroll kEllUnroll
     for (int j = 0; j <= 10; j++) {
+        const uint64_t h = (uint64_t)__double_as_longlong(__ldg(&tp_ell_h[j])) ^ (j & 1 ? flip : 0ull);
         ellf1 += __ldg(&tp_ell_k[0][j]) * powj;
+        hm += __longlong_as_double((long long)h) * powj;
         powj *= m1;
     }
-    m1 = 1.0 - m;
-    powj = m1;
+#pragma unroll kEllUnroll
     for (int j = 1; j <= 14; j++) {
-        q1 += __ldg(&tp_ell_q[j]) * powj;
-        powj *= m1;
+        q1 += __ldg(&tp_ell_q[j]) * powq;
+        powq *= mq;
     }
-    powj = 1.0;
-    m1 = 0.95 - m;
-    for (int j = 0; j <= 10; j++) {
-        hm += __ldg(&tp_ell_h[j]) * powj;
-        powj *= m1;
-    }
-    ellf = -log(q1) * (ellf1 / TP_PI);
-    elle = 1.0 / ellf1 * (TP_PI / 2.0 + ellf * hm);
+    ellf = -log(q1) * soft_div(ellf1, TP_PI);
+    elle = soft_div(1.0, ellf1) * (TP_PI / 2.0 + ellf * hm);
 }
 
 // getWireB, src/wlcs.c:361-401
@@ -414,33 +430,30 @@ __device__ __forceinline__ void wl_wire_bessel(const wlcs& c, double x, double y
 }
 
 // getLoopB, src/wlcs.c:406-449 (NaN Bx, By on the loop axis, as there)
-__device__ __forceinline__ void wl_loop(const DevField& f, const wlcs& c, int ell_corr, double x, double y,
-                                        double z, double B[3])
+__device__ __forceinline__ void wl_loop(const DevField& f, const wlcs& c, const LoopPre& pre, int ell_corr, double x,
+                                        double y, double z, double B[3])
 {
     double xp = (x - c.x_lp) * TP_L0, yp = (y - c.y_lp) * TP_L0, zp = (z - c.z_lp) * TP_L0;
-    double al = c.r_lp * TP_L0, curI = c.cur_lp * TP_I0;
-    wl_transform(xp, yp, zp, c.cosbeta_lp, c.sinbeta_lp, c.cosalpha_lp, c.sinalpha_lp);
-    double Irho = 0.2 * curI;
-    double rho_xy = sd::sqrt_rn(xp * xp + yp * yp);
-    double al2 = al * al;
+    const double al = pre.al, al2 = pre.al2, Irho = pre.Irho;
+    if (!pre.flat) wl_transform(xp, yp, zp, c.cosbeta_lp, c.sinbeta_lp, c.cosalpha_lp, c.sinalpha_lp);
+    double rho_xy = soft_sqrt(xp * xp + yp * yp);
     double r2 = rho_xy * rho_xy + zp * zp;
-    double irho1 = sd::div(1.0, sd::sqrt_rn((al + rho_xy) * (al + rho_xy) + zp * zp));
-    double irho2 = sd::div(1.0, (al - rho_xy) * (al - rho_xy) + zp * zp);
-    double k = sd::sqrt_rn(4.0 * al * rho_xy) * irho1, elle, ellk;
+    double irho1 = soft_div(1.0, soft_sqrt((al + rho_xy) * (al + rho_xy) + zp * zp));
+    double irho2 = soft_div(1.0, (al - rho_xy) * (al - rho_xy) + zp * zp);
+    double k = soft_sqrt(pre.al4 * rho_xy) * irho1, elle, ellk;
     ellint64(f, k, ell_corr, elle, ellk);
-    const sd::Divisor d_rho = sd::divisor(rho_xy);
-    double Brho = sd::div(Irho * zp * irho1 * (-ellk + (al2 + r2) * elle * irho2), d_rho);
+    double Brho = soft_div(Irho * zp * irho1 * (-ellk + (al2 + r2) * elle * irho2), rho_xy);
     if (rho_xy == 0.0) Brho = 0.0;
     double Bz = Irho * irho1 * (ellk - (r2 - al2) * elle * irho2);
     if (ell_corr && rho_xy == 0.0) {
         B[0] = 0.0; B[1] = 0.0;
     } else {
-        Brho = sd::div(Brho, d_rho);
-        B[0] = Brho * xp;
-        B[1] = Brho * yp;
+        Brho = soft_div(Brho, rho_xy);
+        B[0] = __dmul_rn(Brho, xp);
+        B[1] = __dmul_rn(Brho, yp);
     }
     B[2] = Bz;
-    wl_reverse(B[0], B[1], B[2], c.cosbeta_lp, c.sinbeta_lp, c.cosalpha_lp, c.sinalpha_lp);
+    if (!pre.flat) wl_reverse(B[0], B[1], B[2], c.cosbeta_lp, c.sinbeta_lp, c.cosalpha_lp, c.sinalpha_lp);
 }
 
 // ---------------------------------------------------------------- mode sum
@@ -514,7 +527,7 @@ __device__ __forceinline__ void emf64(const DevField& f, double x, double y, dou
                 By += B[1]; Ey += E[1];
                 Bz += B[2]; Ez += E[2];
             }
-            wl_loop(f, c, f.ellint_corrected, x, y, z, B);
+            wl_loop(f, c, f.pre[i], f.ellint_corrected, x, y, z, B);
             Bx += B[0]; By += B[1]; Bz += B[2];
         }
         e[0] = Bx; e[1] = By; e[2] = Bz + 0.0;

@@ -9,6 +9,15 @@
 
 namespace tp {
 
+// Values of a current system that do not depend on the position: its loop's
+// radius in cm, the radius squared and times four, 0.2 times its current, and
+// whether its axes are the box's, so that its rotations multiply by one and
+// add zeros.
+struct LoopPre {
+    double al, al2, al4, Irho;
+    int flat;
+};
+
 // Field description handed to every kernel by value.  Pointers are device
 // addresses; grids are the reference's AoS {x,y,z} records, x fastest
 // (src/magnetic_field.c:31-35, src/electric_field.c:31-35).
@@ -35,6 +44,7 @@ struct DevField {
     // wire-loop current systems
     int nwlcs, iBessel;
     const wlcs *cfg;
+    const LoopPre *pre;
     // plane-wave mode sum
     int nmodes;
     const tp_mode *modes;

@@ -49,12 +49,13 @@ struct Ctx {
     // mirrors of the reference's host grids
     Mirror m_bc_f, m_ba_f, m_bb_f, m_ec_f, m_ea_f, m_eb_f, m_vc_f, m_va_f, m_vb_f;
     Mirror m_bc_d, m_ba_d, m_bb_d, m_ec_d, m_ea_d, m_eb_d, m_vc_d, m_va_d, m_vb_d;
-    Mirror m_cfg, m_modes, m_fx, m_ctab;
+    Mirror m_cfg, m_pre, m_modes, m_fx, m_ctab;
+    std::vector<LoopPre> loop_pre;
     std::vector<Mirror*> all_mirrors()
     {
         return {&m_bc_f, &m_ba_f, &m_bb_f, &m_ec_f, &m_ea_f, &m_eb_f, &m_vc_f, &m_va_f, &m_vb_f,
                 &m_bc_d, &m_ba_d, &m_bb_d, &m_ec_d, &m_ea_d, &m_eb_d, &m_vc_d, &m_va_d, &m_vb_d,
-                &m_cfg, &m_modes, &m_fx, &m_ctab};
+                &m_cfg, &m_pre, &m_modes, &m_fx, &m_ctab};
     }
     // exact energy-bin thresholds on the device
     int thr_nbins = 0;

@@ -101,7 +101,7 @@ __device__ __forceinline__ void small_field(const DevField& f, int c, double x, 
         for (int p = threadIdx.x >> 5; p < 2 * f.nwlcs; p += 4) {
             const wlcs w = f.cfg[p >> 1];
             double b[3] = {0.0, 0.0, 0.0}, e[3] = {0.0, 0.0, 0.0};
-            if (p & 1) wl_loop(f, w, f.ellint_corrected, px, py, pz, b);
+            if (p & 1) wl_loop(f, w, f.pre[p >> 1], f.ellint_corrected, px, py, pz, b);
             else if (f.iBessel != 0) wl_wire_bessel(w, px, py, pz, pt, b, e);
             else if (w.cur_wr != 0.0) wl_wire_static(w, px, py, pz, b);
 #pragma unroll
