@@ -1,5 +1,6 @@
 // capi.cu -- the C ABI of libtpgpu.so: the reference's tracking entry points
 // and globals, device mirrors of the host field arrays, tracking sessions.
+#include <algorithm>
 #include <cfloat>
 #include <climits>
 #include <cmath>
@@ -10,6 +11,8 @@
 #include <vector>
 
 #include "../../include/tp_gpu.h"
+#include "ellint_coeffs.h"
+#include "ellint_fx.cuh"
 #include "tp_kernels.h"
 #include "tp_internal.h"
 
@@ -204,6 +207,8 @@ bool build_field(int stype, DevField& f)
         }
         g.m_pre.dirty = true;
         f.pre = (const LoopPre*)(nwlcs > 0 ? dd0(g.m_pre, g.loop_pre.data(), sizeof(LoopPre) * nwlcs, s) : nullptr);
+        const std::vector<uint64_t>& ell = ellint_table();
+        f.ell = (const uint64_t*)dd0(g.m_ell, ell.data(), sizeof(uint64_t) * ell.size(), s);
         f.nwlcs = nwlcs;
         f.iBessel = iBessel;
     } else if (stype == TP_SYS_MODESUM) {
@@ -295,6 +300,28 @@ const std::vector<int4>& cosine_table()
             t[i] = make_int4((int)(uint32_t)(C >> 31), (int)(C & 0x7fffffff), (int)(S >> 32),
                              (int)((uint32_t)S >> 1));
         }
+        return t;
+    }();
+    return tab;
+}
+
+// The elliptic integrals' table: magnitudes in 2^-61, scaled by 16^-j for the
+// argument 16 |m - m0| (the nome's by 8^-j); centres in 2^-63.
+const std::vector<uint64_t>& ellint_table()
+{
+    static const std::vector<uint64_t> tab = [] {
+        using namespace ellfx;
+        std::vector<uint64_t> t(kSize, 0);
+        auto put = [&](int at, double c, int shift) { t[at] = (uint64_t)llrint(std::ldexp(std::fabs(c), 61 - shift)); };
+        for (int r = 0; r < kRows; r++) {
+            const int i = std::min(r, TP_ELL_NCASE - 1);
+            for (int j = 0; j < kK; j++)
+                put(r * kK + j, r == kRows - 1 && j == 19 ? TP_ELL_K9_19_REF : tp_ell_k[i][j], 4 * j);
+            for (int j = 0; j < kE; j++)
+                put(kOffE + r * kE + j, r < kRows - 1 ? tp_ell_e[i][j] : j <= 10 ? tp_ell_h[j] : 0.0, 4 * j);
+            t[kOffC + r] = (uint64_t)llrint(std::ldexp(r < kRows - 1 ? tp_ell_m0[i] : 0.95, 63));
+        }
+        for (int j = 0; j < kQ; j++) put(kOffQ + j, tp_ell_q[j + 1], 3 * j);
         return t;
     }();
     return tab;

@@ -6,6 +6,7 @@
 // results differ from the reference only where CUDA's sin/cos/acos/log differ
 // from glibc's by an ulp.
 #pragma once
+#include "ellint_fx.cuh"
 #include "tp_common.cuh"
 
 // In global memory, read through L1: the lanes of a warp index different
@@ -441,7 +442,12 @@ __device__ __forceinline__ void wl_loop(const DevField& f, const wlcs& c, const 
     double irho1 = soft_div(1.0, soft_sqrt((al + rho_xy) * (al + rho_xy) + zp * zp));
     double irho2 = soft_div(1.0, (al - rho_xy) * (al - rho_xy) + zp * zp);
     double k = soft_sqrt(pre.al4 * rho_xy) * irho1, elle, ellk;
-    ellint64(f, k, ell_corr, elle, ellk);
+#ifndef TP_SOFT_CALLS
+    // (the adaptive stepper, whose step counts follow the last bit, keeps the
+    // FP64 series; its calls are those of this macro)
+    if (!ellfx::integrals(f.ell, k * k, ell_corr, elle, ellk))
+#endif
+        ellint64(f, k, ell_corr, elle, ellk);
     double Brho = soft_div(Irho * zp * irho1 * (-ellk + (al2 + r2) * elle * irho2), rho_xy);
     if (rho_xy == 0.0) Brho = 0.0;
     double Bz = Irho * irho1 * (ellk - (r2 - al2) * elle * irho2);
@@ -453,7 +459,9 @@ __device__ __forceinline__ void wl_loop(const DevField& f, const wlcs& c, const 
         B[1] = __dmul_rn(Brho, yp);
     }
     B[2] = Bz;
-    if (!pre.flat) wl_reverse(B[0], B[1], B[2], c.cosbeta_lp, c.sinbeta_lp, c.cosalpha_lp, c.sinalpha_lp);
+    // (a component that is not finite, as on the axis, spreads through the rotation)
+    const uint32_t e0 = (uint32_t)__double2hiint(B[0]) & 0x7ff00000u, e1 = (uint32_t)__double2hiint(B[1]) & 0x7ff00000u;
+    if (!pre.flat || e0 == 0x7ff00000u || e1 == 0x7ff00000u) wl_reverse(B[0], B[1], B[2], c.cosbeta_lp, c.sinbeta_lp, c.cosalpha_lp, c.sinalpha_lp);
 }
 
 // ---------------------------------------------------------------- mode sum

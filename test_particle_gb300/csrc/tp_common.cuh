@@ -45,6 +45,7 @@ struct DevField {
     int nwlcs, iBessel;
     const wlcs *cfg;
     const LoopPre *pre;
+    const uint64_t *ell;      // the elliptic integrals' table (ellint_fx.cuh)
     // plane-wave mode sum
     int nmodes;
     const tp_mode *modes;

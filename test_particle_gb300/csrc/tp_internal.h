@@ -49,13 +49,13 @@ struct Ctx {
     // mirrors of the reference's host grids
     Mirror m_bc_f, m_ba_f, m_bb_f, m_ec_f, m_ea_f, m_eb_f, m_vc_f, m_va_f, m_vb_f;
     Mirror m_bc_d, m_ba_d, m_bb_d, m_ec_d, m_ea_d, m_eb_d, m_vc_d, m_va_d, m_vb_d;
-    Mirror m_cfg, m_pre, m_modes, m_fx, m_ctab;
+    Mirror m_cfg, m_pre, m_ell, m_modes, m_fx, m_ctab;
     std::vector<LoopPre> loop_pre;
     std::vector<Mirror*> all_mirrors()
     {
         return {&m_bc_f, &m_ba_f, &m_bb_f, &m_ec_f, &m_ea_f, &m_eb_f, &m_vc_f, &m_va_f, &m_vb_f,
                 &m_bc_d, &m_ba_d, &m_bb_d, &m_ec_d, &m_ea_d, &m_eb_d, &m_vc_d, &m_va_d, &m_vb_d,
-                &m_cfg, &m_pre, &m_modes, &m_fx, &m_ctab};
+                &m_cfg, &m_pre, &m_ell, &m_modes, &m_fx, &m_ctab};
     }
     // exact energy-bin thresholds on the device
     int thr_nbins = 0;
@@ -83,6 +83,7 @@ bool build_field_points(DevField& f);
 namespace mixed { struct MixField; }
 bool build_mixfield(int stype, mixed::MixField& mf, int* nmodes_out);
 const std::vector<int4>& cosine_table();
+const std::vector<uint64_t>& ellint_table();
 bool fixed_modes(const std::vector<tp_mode>& modes, std::vector<fx::Mode>& out, double scale[6]);
 const void* dd0(Mirror& m, const void* h, size_t b, cudaStream_t s);
 bool ensure_thresholds(int nbins);

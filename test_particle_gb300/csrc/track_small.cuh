@@ -13,7 +13,7 @@
 // systems), through shared memory; gridded fields are evaluated by every lane.
 // Every particle's operations and their order are those of track_kernel.
 // Whole runs: 256 particles x 200 steps, ABC, 3.11 -> 1.79 ms; 4,096 x 200, two
-// wires and loops, 23.2 -> 9.2 ms.
+// wires and loops, 23.2 -> 9.2 ms (4.5 with the integrals of ellint_fx.cuh).
 #pragma once
 
 constexpr int kSmallTile = 32;      // particles a block
@@ -305,8 +305,8 @@ static cudaError_t launch_small_sys(const DevField& f, const TrackBufs& b, const
 // only one for it.  Whole runs, host buffers in and out: ABC, 200 steps, 3.0 ms
 // in track_kernel up to its first full wave against 1.8 with one block an SM
 // here, 2.1 with two, 2.8 with three; 256^3 grid, 50 steps, 1.24 against 0.95,
-// 1.25 and 1.64 (every lane evaluates the grid); two wires and loops, 40 steps,
-// 4.6 against 1.8 and 2.4; mode sum, 10 steps, 2.3 against 0.7, 1.0 and 1.7
+// 1.25 and 1.64 (every lane evaluates the grid); two wires and loops, 40 steps
+// (before ellint_fx.cuh), 4.6 against 1.8 and 2.4; mode sum, 10 steps, 2.3 against 0.7, 1.0 and 1.7
 // with four.
 int track_small_blocks(const DevField& f, int n, int num_sms)
 {
