@@ -11,6 +11,7 @@
 // then 128 -> 256 -> 256 -> 256 -> 256 -> 6 with SiLU.  Outputs are trained
 // on normalised components (zero mean, unit variance per component).
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -27,20 +28,20 @@ namespace mlp {
 
 // ---------------------------------------------------------------- features
 // X[b][j] = sin(2 pi f_j . u_b), X[b][64 + j] = cos(...) with u in 32-bit fixed
-// point, as BF16 [n][128]; with XT, also transposed [128][n] (the
-// weight-gradient operand).  Eight features at a time: the row is written in
-// 16-byte pieces, the transposed copy one column at a time (a warp writes 32
-// consecutive samples of a column).
-__global__ void features_kernel(const uint32_t* __restrict__ U, int n, const int* __restrict__ freq,
-                                __nv_bfloat16* __restrict__ X, __nv_bfloat16* __restrict__ XT = nullptr)
+// point, as BF16 [n][128] in the GEMMs' blocks (tctrain::tile_offset).  A thread
+// takes a sample, eight features at a time; a warp's 32 rows of both blocks are
+// put together in shared memory (4 KB each, the global layout) and written 512
+// bytes a store: 8.1 us for 65,536 samples (12.8 row by row with a transposed copy).
+__global__ void __launch_bounds__(128) features_kernel(const uint32_t* __restrict__ U, int n,
+                                                       const int* __restrict__ freq, unsigned char* __restrict__ X)
 {
     __shared__ int fs[3 * kFeat];
+    __shared__ uint4 strip[4][2][256];  // of a warp: sines, cosines
     for (int k = threadIdx.x; k < 3 * kFeat; k += blockDim.x) fs[k] = freq[k];
     __syncthreads();
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const uint32_t U0 = U[3 * i], U1 = U[3 * i + 1], U2 = U[3 * i + 2];
-    uint4* row = reinterpret_cast<uint4*>(X + (size_t)i * kIn);
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const uint32_t U0 = i < n ? U[3 * i] : 0u, U1 = i < n ? U[3 * i + 1] : 0u, U2 = i < n ? U[3 * i + 2] : 0u;
 #pragma unroll 1
     for (int j0 = 0; j0 < kFeat; j0 += 8) {
         uint32_t sp[4], cp[4];
@@ -56,17 +57,17 @@ __global__ void features_kernel(const uint32_t* __restrict__ U, int n, const int
             sp[q / 2] = pack_bf16(s0, s1);
             cp[q / 2] = pack_bf16(c0, c1);
         }
-        row[j0 / 8] = make_uint4(sp[0], sp[1], sp[2], sp[3]);
-        row[(kFeat + j0) / 8] = make_uint4(cp[0], cp[1], cp[2], cp[3]);
-        if (XT) {
-            unsigned short* xt = reinterpret_cast<unsigned short*>(XT);
-#pragma unroll
-            for (int q = 0; q < 8; q++) {
-                xt[(size_t)(j0 + q) * n + i] = (unsigned short)(sp[q / 2] >> (16 * (q & 1)));
-                xt[(size_t)(kFeat + j0 + q) * n + i] = (unsigned short)(cp[q / 2] >> (16 * (q & 1)));
-            }
-        }
+        const int at = lane * 8 + ((j0 / 8) ^ (lane & 7));
+        strip[w][0][at] = make_uint4(sp[0], sp[1], sp[2], sp[3]);
+        strip[w][1][at] = make_uint4(cp[0], cp[1], cp[2], cp[3]);
     }
+    __syncwarp();
+    // rows 32 w.. of the two blocks of this 128-sample tile
+    uint4* dst = reinterpret_cast<uint4*>(X + (size_t)blockIdx.x * 32768u) + w * 256;
+#pragma unroll
+    for (int b = 0; b < 2; b++)
+#pragma unroll
+        for (int k = 0; k < 8; k++) dst[b * 1024 + k * 32 + lane] = strip[w][b][k * 32 + lane];
 }
 
 // ---------------------------------------------------------------- samples
@@ -125,13 +126,13 @@ __global__ void __launch_bounds__(128) samples_kernel(uint64_t seed, long long f
 
 // ---------------------------------------------------------------- loss, biases, AdamW
 // dY = 2 (y - t_n) / (n * 6) with t_n the normalised target; BF16 dY padded with
-// zeros to kDYld columns (one k-atom of the output layer's data-gradient GEMM);
-// the kernel writes the first 8, the rest are zeroed once
+// zeros to kDYld columns (one k-atom of the output layer's data-gradient GEMM), in
+// the GEMMs' blocks; the kernel writes the first 8, the rest are zeroed once
 constexpr int kDYld = 64;
 constexpr int kWgradSplits = 80;  // most split-K parts of a weight-gradient GEMM
 __global__ void loss_kernel(const float* __restrict__ Y, const float* __restrict__ T, int n,
                             const float* __restrict__ mean, const float* __restrict__ istd,
-                            __nv_bfloat16* __restrict__ dY, float* __restrict__ dYf,
+                            unsigned char* __restrict__ dY, float* __restrict__ dYf,
                             double* __restrict__ loss)
 {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -146,39 +147,22 @@ __global__ void loss_kernel(const float* __restrict__ Y, const float* __restrict
             if (dYf) dYf[(size_t)i * kOut + c] = g[c];
         }
         // columns 8.. of dY stay zero from its allocation (mlp_reserve)
-        *reinterpret_cast<uint4*>(dY + (size_t)i * kDYld) =
+        *reinterpret_cast<uint4*>(dY + tctrain::tile_offset(i, 0, 1)) =
             make_uint4(pack_bf16(g[0], g[1]), pack_bf16(g[2], g[3]), pack_bf16(g[4], g[5]), pack_bf16(g[6], g[7]));
     }
     for (int off = 16; off > 0; off >>= 1) l += __shfl_down_sync(0xffffffffu, l, off);
     if ((threadIdx.x & 31) == 0) atomicAdd(loss, (double)l);
 }
 
-// db[c] += sum_rows G[row][c] (BF16 rows of width ld)
-// db[c] += sum over the n samples of GT[c][*] (the gradient transposed, one row
-// per feature, so every block reads one contiguous row); one block per
-// feature, a fixed summation order.
-__global__ void bias_grad_kernel(const __nv_bfloat16* __restrict__ GT, int n, float* __restrict__ db)
+// db[c] = the sum of the blocks' column sums part[block][c]
+__global__ void __launch_bounds__(kHid) bias_grad_kernel(const float* __restrict__ part, int blocks,
+                                                         float* __restrict__ db)
 {
-    __shared__ float red[8];
-    const uint4* row = reinterpret_cast<const uint4*>(GT + (size_t)blockIdx.x * n);
+    const int c = threadIdx.x;
     float s = 0.f;
-    for (int i = threadIdx.x; i < n / 8; i += blockDim.x) {  // 8 values per 16-byte load
-        const uint4 v = row[i];
-        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-        for (int q = 0; q < 4; q++) {
-            const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w[q]));
-            s += f.x + f.y;
-        }
-    }
-    for (int off = 16; off > 0; off >>= 1) s += __shfl_down_sync(0xffffffffu, s, off);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        float t = 0.f;
-        for (int w = 0; w < (int)(blockDim.x >> 5); w++) t += red[w];
-        db[blockIdx.x] += t;
-    }
+#pragma unroll 8
+    for (int k = 0; k < blocks; k++) s += part[(size_t)k * kHid + c];
+    db[c] = s;
 }
 
 // The output layer's gradients from the FP32 loss gradient dYf [n][6] and the
@@ -188,7 +172,7 @@ __global__ void bias_grad_kernel(const __nv_bfloat16* __restrict__ GT, int n, fl
 // block's partial sums.
 constexpr int kOutRows = 128;
 __global__ void __launch_bounds__(256) out_grad_kernel(const float* __restrict__ dYf,
-                                                       const __nv_bfloat16* __restrict__ H3, int n,
+                                                       const unsigned char* __restrict__ H3, int n,
                                                        float* __restrict__ dW4, float* __restrict__ db4)
 {
     __shared__ float dy[kOutRows * kOut];
@@ -198,7 +182,8 @@ __global__ void __launch_bounds__(256) out_grad_kernel(const float* __restrict__
     const int k = threadIdx.x;
     float acc[kOut] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     for (int r = 0; r < nr; r++) {
-        const float h = __bfloat162float(H3[(size_t)(r0 + r) * kHid + k]);
+        const float h = __bfloat162float(
+            *reinterpret_cast<const __nv_bfloat16*>(H3 + tctrain::tile_offset(r0 + r, k, kHid / 64)));
 #pragma unroll
         for (int o = 0; o < kOut; o++) acc[o] = fmaf(dy[r * kOut + o], h, acc[o]);
     }
@@ -229,26 +214,20 @@ __global__ void adamw_kernel(float* __restrict__ p, const float* __restrict__ gr
     p[i] = p[i] - a.lr * (upd + a.wd * p[i]);
 }
 
-// BF16 copies of layer weights: W [out_pad][in] and its transpose [in][out_pad]
+// BF16 copies of layer weights: W [out_pad][in] row-major (wb), as the forward
+// GEMM's k-atoms of out_pad rows (wk), and transposed, as the data gradient's
+// k-atoms of `in` rows (wn); the latter's columns past out_pad stay zero.
 __global__ void to_bf16_kernel(const float* __restrict__ w, int out, int out_pad, int in,
-                               __nv_bfloat16* __restrict__ wb, __nv_bfloat16* __restrict__ wt)
+                               __nv_bfloat16* __restrict__ wb, unsigned char* __restrict__ wk,
+                               unsigned char* __restrict__ wn)
 {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= out_pad * in) return;
     int o = i / in, k = i % in;
     __nv_bfloat16 v = __float2bfloat16(o < out ? w[(size_t)o * in + k] : 0.f);
     wb[i] = v;
-    if (wt) wt[(size_t)k * out_pad + o] = v;
-}
-
-// The output layer's weights transposed and padded to one k-atom: WT4 [256][64],
-// WT4[k][o] = W4[o][k] for o < kOut, zero beyond.
-__global__ void wt4_pad_kernel(const __nv_bfloat16* __restrict__ wt4, __nv_bfloat16* __restrict__ wt4p)
-{
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= kHid * kDYld) return;
-    int k = i / kDYld, o = i % kDYld;
-    wt4p[i] = o < kOutPad ? wt4[(size_t)k * kOutPad + o] : __float2bfloat16(0.f);
+    *reinterpret_cast<__nv_bfloat16*>(wk + tc::sw128_offset(out_pad, o, k)) = v;
+    if (wn) *reinterpret_cast<__nv_bfloat16*>(wn + tc::sw128_offset(in, k, o)) = v;
 }
 
 }  // namespace mlp
@@ -263,8 +242,8 @@ struct MlpState {
     size_t nparam = 0;
     size_t woff[kLayers], boff[kLayers];
     float *p = nullptr, *gr = nullptr, *m = nullptr, *v = nullptr;
-    __nv_bfloat16 *wb[kLayers] = {}, *wt[kLayers] = {};
-    __nv_bfloat16* wt4p = nullptr;          // [256][64] output weights transposed, padded
+    __nv_bfloat16* wb[kLayers] = {};        // [out_pad][in]
+    unsigned char *wk[kLayers] = {}, *wn[kLayers] = {};  // the GEMMs' operands: W, its transpose (not layer 0)
     unsigned char* wpack = nullptr;         // kPackBytes, tensor-core inference layout
     int* freq = nullptr;
     float out_mean[kOut] = {0}, out_std[kOut] = {1, 1, 1, 1, 1, 1};
@@ -272,13 +251,12 @@ struct MlpState {
     long step = 0;
     // batch workspaces
     int cap = 0;
-    __nv_bfloat16* X = nullptr;             // [cap][128]
-    __nv_bfloat16 *Z[4] = {}, *H[4] = {};   // [cap][256]
-    __nv_bfloat16 *G0 = nullptr, *G1 = nullptr;  // [cap][256] backward scratch
-    __nv_bfloat16* dY = nullptr;            // [cap][kDYld]
-    __nv_bfloat16* XT = nullptr;            // [128][n] features transposed
-    __nv_bfloat16* HT[4] = {};              // [256][n] activations transposed
-    __nv_bfloat16* GT = nullptr;            // [256][n] pre-activation gradient transposed
+    // samples x columns, BF16 in the GEMMs' blocks
+    unsigned char* X = nullptr;             // [cap][128]
+    unsigned char *Z[4] = {}, *H[4] = {};   // [cap][256]
+    unsigned char *G0 = nullptr, *G1 = nullptr;  // [cap][256] backward scratch
+    unsigned char* dY = nullptr;            // [cap][kDYld]
+    float* bpart = nullptr;                 // bias gradients by block of the data-gradient GEMM
     float* partial = nullptr;               // split-K partial weight gradients
     float* Y = nullptr;                     // [cap][6]
     float* dYf = nullptr;                   // [cap][6]
@@ -305,11 +283,17 @@ static bool mlp_alloc_params()
     for (int l = 0; l < kLayers; l++) {
         size_t e = (size_t)layer_out_pad(l) * layer_in(l);
         if (!cuda_ok(cudaMalloc(&M.wb[l], sizeof(__nv_bfloat16) * e), "mlp wb") ||
-            !cuda_ok(cudaMalloc(&M.wt[l], sizeof(__nv_bfloat16) * e), "mlp wt"))
+            !cuda_ok(cudaMalloc(&M.wk[l], sizeof(__nv_bfloat16) * e), "mlp wk"))
+            return false;
+        if (l == 0) continue;
+        const size_t t = sizeof(__nv_bfloat16) * (size_t)layer_in(l) * (l == kLayers - 1 ? kDYld : kHid);
+        if (!cuda_ok(cudaMalloc(&M.wn[l], t), "mlp wn") ||
+            !cuda_ok(cudaMemsetAsync(M.wn[l], 0, t, g.stream), "mlp wn zero"))
             return false;
     }
     return cuda_ok(cudaMalloc(&M.wpack, kPackBytes), "mlp wpack") &&
-           cuda_ok(cudaMalloc(&M.wt4p, sizeof(__nv_bfloat16) * kHid * kDYld), "mlp wt4p") &&
+           cuda_ok(cudaMalloc(&M.bpart, sizeof(float) * (size_t)tctrain::layer_blocks(INT_MAX / 128 * 128) * kHid),
+                   "mlp bias partial") &&
            cuda_ok(cudaMalloc(&M.partial, sizeof(float) * (size_t)kWgradSplits * kHid * kHid), "mlp partial") &&
            cuda_ok(cudaMalloc(&M.freq, sizeof(int) * 3 * kFeat), "mlp freq") &&
            cuda_ok(cudaMalloc(&M.d_mean, sizeof(float) * kOut), "mlp mean") &&
@@ -323,19 +307,16 @@ static bool mlp_reserve(int n)
     n = (n + 127) / 128 * 128;
     if (n <= M.cap) return true;
     auto fr = [](void* p) { if (p) cudaFree(p); };
-    fr(M.X); fr(M.G0); fr(M.G1); fr(M.dY); fr(M.Y); fr(M.dYf); fr(M.XT); fr(M.GT);
-    for (int l = 0; l < 4; l++) { fr(M.Z[l]); fr(M.H[l]); fr(M.HT[l]); }
+    fr(M.X); fr(M.G0); fr(M.G1); fr(M.dY); fr(M.Y); fr(M.dYf);
+    for (int l = 0; l < 4; l++) { fr(M.Z[l]); fr(M.H[l]); }
     size_t h = sizeof(__nv_bfloat16) * (size_t)n * kHid;
     bool ok = cuda_ok(cudaMalloc(&M.X, sizeof(__nv_bfloat16) * (size_t)n * kIn), "X") &&
-              cuda_ok(cudaMalloc(&M.XT, sizeof(__nv_bfloat16) * (size_t)n * kIn), "XT") &&
               cuda_ok(cudaMalloc(&M.G0, h), "G0") && cuda_ok(cudaMalloc(&M.G1, h), "G1") &&
-              cuda_ok(cudaMalloc(&M.GT, h), "GT") &&
               cuda_ok(cudaMalloc(&M.dY, sizeof(__nv_bfloat16) * (size_t)n * kDYld), "dY") &&
               cuda_ok(cudaMalloc(&M.Y, sizeof(float) * (size_t)n * kOut), "Y") &&
               cuda_ok(cudaMalloc(&M.dYf, sizeof(float) * (size_t)n * kOut), "dYf");
     for (int l = 0; l < 4 && ok; l++)
-        ok = cuda_ok(cudaMalloc(&M.Z[l], h), "Z") && cuda_ok(cudaMalloc(&M.H[l], h), "H") &&
-             cuda_ok(cudaMalloc(&M.HT[l], h), "HT");
+        ok = cuda_ok(cudaMalloc(&M.Z[l], h), "Z") && cuda_ok(cudaMalloc(&M.H[l], h), "H");
     // the padding columns of dY (beyond the 8 the loss kernel writes) stay zero
     if (ok) ok = cuda_ok(cudaMemsetAsync(M.dY, 0, sizeof(__nv_bfloat16) * (size_t)n * kDYld, g.stream), "dY zero");
     if (ok) M.cap = n;
@@ -348,9 +329,8 @@ static bool mlp_refresh_bf16()
     for (int l = 0; l < kLayers; l++) {
         int e = layer_out_pad(l) * layer_in(l);
         to_bf16_kernel<<<(e + 255) / 256, 256, 0, s>>>(M.p + M.woff[l], layer_out(l), layer_out_pad(l),
-                                                       layer_in(l), M.wb[l], M.wt[l]);
+                                                       layer_in(l), M.wb[l], M.wk[l], M.wn[l]);
     }
-    wt4_pad_kernel<<<(kHid * kDYld + 255) / 256, 256, 0, s>>>(M.wt[kLayers - 1], M.wt4p);
     if (!cuda_ok(pack_weights(M.wb, M.wpack, s), "pack weights")) return false;
     float istd[kOut];
     for (int c = 0; c < kOut; c++) istd[c] = 1.0f / M.out_std[c];
@@ -360,22 +340,20 @@ static bool mlp_refresh_bf16()
 }
 
 // forward of n samples from features X (rows up to the next multiple of 128
-// are computed too and ignored): fills Z/H (and H transposed) and Y
+// are computed too and ignored): fills Z/H and Y
 // (normalised outputs), on the tensor cores
 static bool mlp_forward(int n)
 {
     cudaStream_t s = g.stream;
     const int np = (n + 127) / 128 * 128;
-    const __nv_bfloat16* in = M.X;
-    int ldin = kIn;
+    const unsigned char* in = M.X;
     for (int l = 0; l < 4; l++) {
-        if (!cuda_ok(tctrain::forward_hidden(in, ldin, M.wb[l], layer_in(l), np, M.p + M.boff[l], M.Z[l],
-                                             M.H[l], M.HT[l], g.d_status, s),
+        if (!cuda_ok(tctrain::forward_hidden(in, layer_in(l), M.wk[l], np, M.p + M.boff[l], M.Z[l], M.H[l],
+                                             g.d_status, s),
                      "fwd gemm")) return false;
         in = M.H[l];
-        ldin = kHid;
     }
-    return cuda_ok(tctrain::forward_out(in, M.wb[4], np, M.p + M.boff[4], M.Y, g.d_status, s), "out gemm");
+    return cuda_ok(tctrain::forward_out(in, M.wk[4], np, M.p + M.boff[4], M.Y, g.d_status, s), "out gemm");
 }
 
 // backward of n samples (a multiple of 128) after mlp_forward and the loss
@@ -390,30 +368,25 @@ static bool mlp_backward(int n)
     {
         out_grad_kernel<<<(n + kOutRows - 1) / kOutRows, 256, 0, s>>>(M.dYf, M.H[3], n, M.gr + M.woff[4],
                                                                        M.gr + M.boff[4]);
-        if (!cuda_ok(tctrain::backward_data(M.dY, kDYld, M.wt4p, kDYld, n, M.Z[3], M.G0, M.GT, g.d_status, s),
+        if (!cuda_ok(tctrain::backward_data(M.dY, kDYld, M.wn[4], n, M.Z[3], M.G0, M.bpart, g.d_status, s),
                      "dH3"))
             return false;
     }
-    __nv_bfloat16 *gcur = M.G0, *gnext = M.G1;
+    unsigned char *gcur = M.G0, *gnext = M.G1;
+    // split the samples so that the two 128-row tiles fill the SMs, at least
+    // four steps of 64 per split
+    const int splits = std::max(1, std::min({kWgradSplits, 76, n / 256}));
     for (int l = 3; l >= 0; l--) {
-        const __nv_bfloat16* xt = l == 0 ? M.XT : M.HT[l - 1];
-        const int kin = layer_in(l);
-        // split K (the samples) so that the two 128-row tiles fill the SMs, at
-        // least four k-atoms per split
-        const int splits = std::max(1, std::min({kWgradSplits, 76, n / 256}));
-        if (!cuda_ok(tctrain::backward_weights(M.GT, xt, kin, n, M.partial, splits, M.gr + M.woff[l], g.d_status,
-                                               s),
+        bias_grad_kernel<<<1, kHid, 0, s>>>(M.bpart, tctrain::layer_blocks(n), M.gr + M.boff[l]);
+        if (!cuda_ok(tctrain::backward_weights(gcur, l == 0 ? M.X : M.H[l - 1], layer_in(l), n, M.partial, splits,
+                                               M.gr + M.woff[l], g.d_status, s),
                      "dW"))
             return false;
-        bias_grad_kernel<<<kHid, 256, 0, s>>>(M.GT, n, M.gr + M.boff[l]);
         if (l > 0) {
-            if (!cuda_ok(tctrain::backward_data(gcur, kHid, M.wt[l], kHid, n, M.Z[l - 1], gnext, M.GT, g.d_status,
-                                                s),
+            if (!cuda_ok(tctrain::backward_data(gcur, kHid, M.wn[l], n, M.Z[l - 1], gnext, M.bpart, g.d_status, s),
                          "dH"))
                 return false;
-            __nv_bfloat16* tmp = gcur;
-            gcur = gnext;
-            gnext = tmp;
+            std::swap(gcur, gnext);
         }
     }
     return true;
@@ -528,7 +501,7 @@ extern "C" int tp_mlp_grad(int n, const unsigned int* u, const float* t, double*
         !cuda_ok(cudaMalloc(&dT, sizeof(float) * 6 * n), "t")) return -1;
     cudaMemcpyAsync(dU, u, sizeof(uint32_t) * 3 * n, cudaMemcpyHostToDevice, s);
     cudaMemcpyAsync(dT, t, sizeof(float) * 6 * n, cudaMemcpyHostToDevice, s);
-    features_kernel<<<(n + 127) / 128, 128, 0, s>>>(dU, n, M.freq, M.X, M.XT);
+    features_kernel<<<(n + 127) / 128, 128, 0, s>>>(dU, n, M.freq, M.X);
     bool ok = mlp_forward(n) && mlp_loss(n, dT, loss) && mlp_backward(n);
     if (ok) {
         if (y) cudaMemcpyAsync(y, M.Y, sizeof(float) * 6 * n, cudaMemcpyDeviceToHost, s);
@@ -599,7 +572,7 @@ extern "C" int tp_mlp_train(long long nsamples, int batch, int epochs, double lr
     bool ok = mlp_refresh_bf16();
     for (long long it = 0; it < total && ok; it++) {
         long long bi = it % nb;
-        features_kernel<<<(batch + 127) / 128, 128, 0, s>>>(dU + 3 * bi * batch, batch, M.freq, M.X, M.XT);
+        features_kernel<<<(batch + 127) / 128, 128, 0, s>>>(dU + 3 * bi * batch, batch, M.freq, M.X);
         const bool last = it == total - 1;
         ok = mlp_forward(batch) && mlp_loss(batch, dT + 6 * bi * batch, last ? &loss : nullptr) &&
              mlp_backward(batch);

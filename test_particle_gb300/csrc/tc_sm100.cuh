@@ -45,6 +45,21 @@ __device__ __forceinline__ uint64_t desc_sw128(uint32_t saddr)
     return d;
 }
 
+// The same for an operand whose rows (128 bytes) run along M or N and follow one
+// another along K: the leading byte offset leads from 64 of M or N to the next 64,
+// the stride byte offset 1024 from 8 of K to the next 8.
+__device__ __forceinline__ uint64_t desc_sw128_mn(uint32_t saddr, uint32_t lead)
+{
+    uint64_t d = 0;
+    d |= (uint64_t)((saddr >> 4) & 0x3FFFu);
+    d |= (uint64_t)(lead >> 4) << 16;
+    d |= (uint64_t)(1024u >> 4) << 32;
+    d |= (uint64_t)1u << 46;
+    d |= (uint64_t)2u << 61;
+    return d;
+}
+constexpr uint32_t kIdescMnMajorAB = (1u << 15) | (1u << 16);  // instruction descriptor: A and B MN-major
+
 // Instruction descriptor of kind::f16: D F32, A and B BF16, both K-major, M x N.
 __host__ __device__ constexpr uint32_t idesc_bf16_f32(int M, int N)
 {
@@ -108,6 +123,17 @@ __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void* src, uint32_t
         "l"(src), "r"(bytes), "r"(bar)
         : "memory");
 }
+
+// ---- 1-D bulk async copy shared -> global (after fence_async_smem), in bulk groups of
+// the issuing thread; bulk_wait_read: the shared memory may be written again
+__device__ __forceinline__ void bulk_s2g(void* dst, uint32_t src, uint32_t bytes)
+{
+    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(src), "r"(bytes)
+                 : "memory");
+}
+__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+__device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 
 // ---- fences
 __device__ __forceinline__ void fence_async_smem()  // generic-proxy smem writes -> async proxy

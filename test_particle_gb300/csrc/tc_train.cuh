@@ -3,36 +3,41 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include "tc_sm100.cuh"
+
 namespace tp {
-namespace tct {
-size_t smem_bytes(int n, int ring);
-}
 namespace tctrain {
 
-// Z, H = silu(X W^T + b) of a hidden layer: X [M][kin] (row stride lda), W [256][kin];
-// Z, H row-major [M][256], H also transposed into HT [256][M].  M a multiple of 128.
-cudaError_t forward_hidden(const __nv_bfloat16* X, int lda, const __nv_bfloat16* W, int kin, int M,
-                           const float* b, __nv_bfloat16* Z, __nv_bfloat16* H, __nv_bfloat16* HT, int* status,
-                           cudaStream_t s);
+// Byte offset of element (m, c) of a matrix of samples [M][64 atoms] in BF16: 16 KB
+// blocks of 128 samples x 64 columns, swizzled rows of 128 bytes (M a multiple of 128).
+__host__ __device__ __forceinline__ size_t tile_offset(size_t m, int c, int atoms)
+{
+    return (m >> 7) * (size_t)atoms * 16384u + tc::sw128_offset(128, (int)(m & 127), c);
+}
 
-// Y = H3 W4^T + b: H3 [M][256], W4 [16][256] (rows past the 6 outputs zero); Y FP32 [M][6].
-cudaError_t forward_out(const __nv_bfloat16* H3, const __nv_bfloat16* W4, int M, const float* b, float* Y,
-                        int* status, cudaStream_t s);
+// Weights are k-atoms of all rows: element (n, k) of [N][K] at sw128_offset(N, n, k).
 
-// G = (Gin WT^T) * silu'(Zprev): Gin [M][kout] (row stride ldg), WT [256][kout] (the
-// layer's weights transposed); G row-major [M][256] and transposed into GT [256][M].
-cudaError_t backward_data(const __nv_bfloat16* Gin, int ldg, const __nv_bfloat16* WT, int kout, int M,
-                          const __nv_bfloat16* Zprev, __nv_bfloat16* G, __nv_bfloat16* GT, int* status,
-                          cudaStream_t s);
+// Blocks of a layer kernel over M samples (the rows of backward_data's bpart).
+int layer_blocks(int M);
 
-// gr[256][kin] += GT XT^T over nsamp samples: GT [256][nsamp], XT [kin][nsamp]; split-K
-// partial sums in `partial` (splits x 256 x kin FP32) reduced into gr.
-cudaError_t backward_weights(const __nv_bfloat16* GT, const __nv_bfloat16* XT, int kin, int nsamp,
-                             float* partial, int splits, float* gr, int* status, cudaStream_t s);
+// Z, H = silu(X W^T + b) of a hidden layer: X [M][kin], W [256][kin]; Z, H [M][256].
+// M a multiple of 128.
+cudaError_t forward_hidden(const void* X, int kin, const void* W, int M, const float* b, void* Z, void* H,
+                           int* status, cudaStream_t s);
 
-// D[M][N] = A[M][K] B[N][K]^T in FP32 (self-check).
-cudaError_t gemm_f32(const __nv_bfloat16* A, const __nv_bfloat16* B, int M, int N, int K, float* D, int* status,
-                     cudaStream_t s);
+// Y = H3 W4^T + b: H3 [M][256], W4 [16][256] (rows past the 6 outputs zero); Y FP32 [M][6], row-major.
+cudaError_t forward_out(const void* H3, const void* W4, int M, const float* b, float* Y, int* status,
+                        cudaStream_t s);
+
+// G = (Gin WT^T) * silu'(Zprev): Gin [M][kout], WT [256][kout] (the layer's weights
+// transposed); G [M][256], its column sums over a block's samples in bpart [layer_blocks(M)][256].
+cudaError_t backward_data(const void* Gin, int kout, const void* WT, int M, const void* Zprev, void* G,
+                          float* bpart, int* status, cudaStream_t s);
+
+// gr[256][kin] = G^T X over nsamp samples: G [nsamp][256], X [nsamp][kin]; `splits`
+// (at most nsamp / 64) partial sums in `partial` (splits x 256 x kin FP32), summed into gr.
+cudaError_t backward_weights(const void* G, const void* X, int kin, int nsamp, float* partial, int splits,
+                             float* gr, int* status, cudaStream_t s);
 
 }  // namespace tctrain
 }  // namespace tp
