@@ -1,9 +1,10 @@
 // mlp.cu -- training and inference of the learned field model: the forward,
 // data-gradient and hidden weight-gradient GEMMs on the 5th-generation tensor
 // cores (tc_train.cu: tcgen05.mma, FP32 accumulation in tensor memory, fused
-// bias / SiLU / SiLU-derivative epilogues), Fourier features, MSE loss, the
-// bias gradients and the output layer's 6 x 256 weight gradient as
-// reductions on the CUDA cores, AdamW.
+// bias / SiLU / SiLU-derivative / bias-gradient epilogues), Fourier features, MSE
+// loss, the output layer's 6 x 256 weight gradient as a reduction on the CUDA
+// cores, and one kernel a batch that sums the partial gradients and takes the
+// AdamW step.
 //
 // The model maps a position u in the periodic box (u = (x - min) / L) to the
 // six field components: 64 integer-lattice frequencies f_j give the features
@@ -124,7 +125,7 @@ __global__ void __launch_bounds__(128) samples_kernel(uint64_t seed, long long f
     }
 }
 
-// ---------------------------------------------------------------- loss, biases, AdamW
+// ---------------------------------------------------------------- loss, output layer, AdamW
 // dY = 2 (y - t_n) / (n * 6) with t_n the normalised target; BF16 dY padded with
 // zeros to kDYld columns (one k-atom of the output layer's data-gradient GEMM), in
 // the GEMMs' blocks; the kernel writes the first 8, the rest are zeroed once
@@ -154,45 +155,71 @@ __global__ void loss_kernel(const float* __restrict__ Y, const float* __restrict
     if ((threadIdx.x & 31) == 0) atomicAdd(loss, (double)l);
 }
 
-// db[c] = the sum of the blocks' column sums part[block][c]
-__global__ void __launch_bounds__(kHid) bias_grad_kernel(const float* __restrict__ part, int blocks,
-                                                         float* __restrict__ db)
-{
-    const int c = threadIdx.x;
-    float s = 0.f;
-#pragma unroll 8
-    for (int k = 0; k < blocks; k++) s += part[(size_t)k * kHid + c];
-    db[c] = s;
-}
-
-// The output layer's gradients from the FP32 loss gradient dYf [n][6] and the
-// last hidden activations H3 [n][256]: dW4[o][k] += sum_r dYf[r][o] H3[r][k],
-// db4[o] += sum_r dYf[r][o].  A block takes kOutRows consecutive samples:
-// thread k owns column k of H3 and keeps six sums; FP32 atomics add the
-// block's partial sums.
-constexpr int kOutRows = 128;
+// Partial sums of the output layer's gradients from the FP32 loss gradient dYf
+// [n][6] and the last hidden activations H3 [n][256]: part[block] holds
+// dW4[o][k] = sum_r dYf[r][o] H3[r][k] and, behind, db4[o] = sum_r dYf[r][o] over
+// the block's 128-sample tiles.  Thread (g, c) takes columns 8 c.. of the 16
+// rows 16 g.. of a tile: a warp reads a row's 512 bytes, 48 FMAs a thread and
+// 16-byte load; the eight groups of rows are added in shared memory at the end.
+// 17 us for 65,536 samples (32 MB, from HBM); with a column a thread, 2-byte loads
+// and 128 samples a block added with atomics 25 us (39 from the blocks).
+constexpr int kOutGrad = kOut * kHid + kOut;
 __global__ void __launch_bounds__(256) out_grad_kernel(const float* __restrict__ dYf,
-                                                       const unsigned char* __restrict__ H3, int n,
-                                                       float* __restrict__ dW4, float* __restrict__ db4)
+                                                       const unsigned char* __restrict__ H3, int ntiles,
+                                                       float* __restrict__ part)
 {
-    __shared__ float dy[kOutRows * kOut];
-    const int r0 = blockIdx.x * kOutRows, nr = min(kOutRows, n - r0);
-    for (int i = threadIdx.x; i < nr * kOut; i += blockDim.x) dy[i] = dYf[(size_t)r0 * kOut + i];
-    __syncthreads();
-    const int k = threadIdx.x;
-    float acc[kOut] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    for (int r = 0; r < nr; r++) {
-        const float h = __bfloat162float(
-            *reinterpret_cast<const __nv_bfloat16*>(H3 + tctrain::tile_offset(r0 + r, k, kHid / 64)));
+    __shared__ float4 dy[128 * 2];  // rows padded to eight values
+    __shared__ float red[8][kHid + 1];
+    const int c = threadIdx.x & 31, gr = threadIdx.x >> 5;
+    float acc[kOut][8] = {}, accb = 0.f;
+    float* dys = reinterpret_cast<float*>(dy);
+    for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
+        __syncthreads();
+        for (int i = threadIdx.x; i < 128 * kOut; i += 256)
+            dys[(i / kOut) * 8 + i % kOut] = dYf[(size_t)t * 128 * kOut + i];
+        const unsigned char* src = H3 + (size_t)t * 4 * 16384u + (size_t)(c >> 3) * 16384u;
+        uint4 h[16];
 #pragma unroll
-        for (int o = 0; o < kOut; o++) acc[o] = fmaf(dy[r * kOut + o], h, acc[o]);
+        for (int r = 0; r < 16; r++)
+            h[r] = *reinterpret_cast<const uint4*>(src + tc::sw128_offset(128, 16 * gr + r, 8 * (c & 7)));
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < 16; r++) {
+            const float4 a = dy[2 * (16 * gr + r)];
+            const float2 b = *reinterpret_cast<const float2*>(&dy[2 * (16 * gr + r) + 1]);
+            const float d[kOut] = {a.x, a.y, a.z, a.w, b.x, b.y};
+            const uint32_t w[4] = {h[r].x, h[r].y, h[r].z, h[r].w};
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w[j]));
+#pragma unroll
+                for (int o = 0; o < kOut; o++) {
+                    acc[o][2 * j] = fmaf(d[o], f.x, acc[o][2 * j]);
+                    acc[o][2 * j + 1] = fmaf(d[o], f.y, acc[o][2 * j + 1]);
+                }
+            }
+        }
+        if (threadIdx.x < 8 * kOut)  // sixteen rows of one output
+            for (int r = 0; r < 16; r++) accb += dys[((threadIdx.x / kOut) * 16 + r) * 8 + threadIdx.x % kOut];
     }
+    float* dst = part + (size_t)blockIdx.x * kOutGrad;
 #pragma unroll
-    for (int o = 0; o < kOut; o++) atomicAdd(&dW4[o * kHid + k], acc[o]);
-    if (k < kOut) {
-        float t = 0.f;
-        for (int r = 0; r < nr; r++) t += dy[r * kOut + k];
-        atomicAdd(&db4[k], t);
+    for (int o = 0; o < kOut; o++) {
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < 8; j++) red[gr][8 * c + j] = acc[o][j];
+        __syncthreads();
+        float s = 0.f;
+        for (int g8 = 0; g8 < 8; g8++) s += red[g8][threadIdx.x];
+        dst[o * kHid + threadIdx.x] = s;
+    }
+    __syncthreads();
+    if (threadIdx.x < 8 * kOut) red[threadIdx.x / kOut][threadIdx.x % kOut] = accb;
+    __syncthreads();
+    if (threadIdx.x < kOut) {
+        float s = 0.f;
+        for (int g8 = 0; g8 < 8; g8++) s += red[g8][threadIdx.x];
+        dst[kOut * kHid + threadIdx.x] = s;
     }
 }
 
@@ -200,34 +227,134 @@ struct Adam {
     float lr, b1, b2, eps, wd, c1, c2;  // c1 = 1 / (1 - b1^t), c2 = 1 / (1 - b2^t)
 };
 
-__global__ void adamw_kernel(float* __restrict__ p, const float* __restrict__ gr, float* __restrict__ m,
-                             float* __restrict__ v, int n, Adam a)
+// BF16 copies of the weights: as the forward GEMM's k-atoms of out_pad rows (wk),
+// transposed, as the data gradient's k-atoms of `in` rows (wn, not layer 0; the
+// output layer's columns past kOut stay zero) and in the tracking kernel's chunks.
+struct Copies {
+    unsigned char *wk[kLayers], *wn[kLayers], *pack;
+};
+
+__device__ __forceinline__ void store_weight(const Copies& c, int l, int o, int k, float w)
 {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    float g = gr[i];
-    float mi = a.b1 * m[i] + (1.f - a.b1) * g;
-    float vi = a.b2 * v[i] + (1.f - a.b2) * g * g;
-    m[i] = mi;
-    v[i] = vi;
-    float upd = (mi * a.c1) / (sqrtf(vi * a.c2) + a.eps);
-    p[i] = p[i] - a.lr * (upd + a.wd * p[i]);
+    const __nv_bfloat16 v = __float2bfloat16(w);
+    *reinterpret_cast<__nv_bfloat16*>(c.wk[l] + tc::sw128_offset(layer_out_pad(l), o, k)) = v;
+    if (l > 0) *reinterpret_cast<__nv_bfloat16*>(c.wn[l] + tc::sw128_offset(layer_in(l), k, o)) = v;
+    *reinterpret_cast<__nv_bfloat16*>(c.pack + pack_offset(l, o, k)) = v;
 }
 
-// BF16 copies of layer weights: W [out_pad][in] row-major (wb), as the forward
-// GEMM's k-atoms of out_pad rows (wk), and transposed, as the data gradient's
-// k-atoms of `in` rows (wn); the latter's columns past out_pad stay zero.
-__global__ void to_bf16_kernel(const float* __restrict__ w, int out, int out_pad, int in,
-                               __nv_bfloat16* __restrict__ wb, unsigned char* __restrict__ wk,
-                               unsigned char* __restrict__ wn)
+// First parameter of layer l (weights [out][in], then biases) in the flat layout
+__host__ __device__ constexpr int param_offset(int l)
+{
+    int off = 0;
+    for (int k = 0; k < l; k++) off += layer_out(k) * (layer_in(k) + 1);
+    return off;
+}
+constexpr int kParams = param_offset(kLayers);
+
+__global__ void copies_kernel(const float* __restrict__ p, const __grid_constant__ Copies cp)
 {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= out_pad * in) return;
-    int o = i / in, k = i % in;
-    __nv_bfloat16 v = __float2bfloat16(o < out ? w[(size_t)o * in + k] : 0.f);
-    wb[i] = v;
-    *reinterpret_cast<__nv_bfloat16*>(wk + tc::sw128_offset(out_pad, o, k)) = v;
-    if (wn) *reinterpret_cast<__nv_bfloat16*>(wn + tc::sw128_offset(in, k, o)) = v;
+    for (int l = 0; l < kLayers; l++) {
+        const int nw = layer_out(l) * layer_in(l);
+        if (i < nw) {
+            store_weight(cp, l, i / layer_in(l), i % layer_in(l), p[param_offset(l) + i]);
+            return;
+        }
+        i -= nw;
+    }
+}
+
+// Partial sums of the gradients: the hidden layers' weights by split
+// (backward_weights), their biases by block of the data-gradient GEMM, the
+// output layer by block of out_grad_kernel.
+struct Partials {
+    const float *w[4], *b[4], *out;
+    int splits, bblocks, oblocks;
+};
+
+// The end of a batch in one launch: every gradient is summed from its partial
+// sums, in a fixed order, and either stored (gr) or used at once for the AdamW
+// step, the new weights going out as FP32 and in their three BF16 copies.
+// A block takes 32 x 8 of a hidden layer's weights (thread = one, 128-byte reads
+// of every split, turned through shared memory for the row-major parameters), 32
+// biases, or 32 of the output layer's parameters (eight threads each).  17.8
+// us for 76 splits (68 MB read); a kernel per layer and purpose (four sums of
+// splits, four of biases, AdamW, six of copies) took 137 us.
+constexpr int kPatches0 = (kHid / 32) * (kIn / 8), kPatches = (kHid / 32) * (kHid / 8);
+constexpr int kBiasBlocks = 4 * kHid / 32, kOutBlocks = (kOutGrad + 31) / 32;
+constexpr int kUpdateBlocks = kPatches0 + 3 * kPatches + kBiasBlocks + kOutBlocks;
+
+template <bool STEP>
+__global__ void __launch_bounds__(256) update_kernel(const __grid_constant__ Partials ps, float* __restrict__ gr,
+                                                     float* __restrict__ p, float* __restrict__ m,
+                                                     float* __restrict__ v, Adam a, const __grid_constant__ Copies cp)
+{
+    __shared__ float red[8][33];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    int blk = blockIdx.x, l, o, k, idx;
+    float g;
+    if (blk < kPatches0 + 3 * kPatches) {
+        l = blk < kPatches0 ? 0 : 1 + (blk - kPatches0) / kPatches;
+        const int i = blk < kPatches0 ? blk : (blk - kPatches0) % kPatches;
+        const int in = layer_in(l), m0 = (i & 7) * 32, n0 = (i >> 3) * 8;
+        const float* src = ps.w[l] + ((size_t)(m0 >> 7) * in + n0 + w) * 128 + (m0 & 127) + lane;
+        const size_t step = (size_t)(kHid / 128) * in * 128;
+        float s = 0.f;
+#pragma unroll 8
+        for (int q = 0; q < ps.splits; q++) s += src[q * step];
+        red[w][lane] = s;
+        __syncthreads();
+        o = m0 + (threadIdx.x >> 3);
+        k = n0 + (threadIdx.x & 7);
+        g = red[threadIdx.x & 7][threadIdx.x >> 3];
+        idx = param_offset(l) + o * in + k;
+    } else {
+        blk -= kPatches0 + 3 * kPatches;
+        const bool bias = blk < kBiasBlocks;
+        const float* src;
+        int stride, n;
+        bool in_range = true;
+        if (bias) {
+            l = blk / (kHid / 32);
+            const int e = (blk % (kHid / 32)) * 32 + lane;
+            src = ps.b[l] + e;
+            stride = kHid;
+            n = ps.bblocks;
+            idx = param_offset(l) + kHid * layer_in(l) + e;
+            o = k = -1;
+        } else {
+            l = kLayers - 1;
+            const int e = (blk - kBiasBlocks) * 32 + lane;
+            in_range = e < kOutGrad;
+            src = ps.out + (in_range ? e : 0);
+            stride = kOutGrad;
+            n = ps.oblocks;
+            idx = param_offset(l) + e;
+            o = e < kOut * kHid ? e / kHid : -1;
+            k = e % kHid;
+        }
+        float s = 0.f;
+#pragma unroll 8
+        for (int q = w; q < n; q += 8) s += src[(size_t)q * stride];
+        red[w][lane] = s;
+        __syncthreads();
+        if (w > 0 || !in_range) return;
+        g = 0.f;
+#pragma unroll
+        for (int q = 0; q < 8; q++) g += red[q][lane];
+    }
+    if (!STEP) {
+        gr[idx] = g;
+        return;
+    }
+    const float mi = a.b1 * m[idx] + (1.f - a.b1) * g;
+    const float vi = a.b2 * v[idx] + (1.f - a.b2) * g * g;
+    m[idx] = mi;
+    v[idx] = vi;
+    const float upd = (mi * a.c1) / (sqrtf(vi * a.c2) + a.eps);
+    const float pn = p[idx] - a.lr * (upd + a.wd * p[idx]);
+    p[idx] = pn;
+    if (o >= 0) store_weight(cp, l, o, k, pn);
 }
 
 }  // namespace mlp
@@ -242,9 +369,7 @@ struct MlpState {
     size_t nparam = 0;
     size_t woff[kLayers], boff[kLayers];
     float *p = nullptr, *gr = nullptr, *m = nullptr, *v = nullptr;
-    __nv_bfloat16* wb[kLayers] = {};        // [out_pad][in]
-    unsigned char *wk[kLayers] = {}, *wn[kLayers] = {};  // the GEMMs' operands: W, its transpose (not layer 0)
-    unsigned char* wpack = nullptr;         // kPackBytes, tensor-core inference layout
+    Copies cp{};                            // BF16 copies of the weights
     int* freq = nullptr;
     float out_mean[kOut] = {0}, out_std[kOut] = {1, 1, 1, 1, 1, 1};
     float *d_mean = nullptr, *d_istd = nullptr;
@@ -256,14 +381,17 @@ struct MlpState {
     unsigned char *Z[4] = {}, *H[4] = {};   // [cap][256]
     unsigned char *G0 = nullptr, *G1 = nullptr;  // [cap][256] backward scratch
     unsigned char* dY = nullptr;            // [cap][kDYld]
-    float* bpart = nullptr;                 // bias gradients by block of the data-gradient GEMM
-    float* partial = nullptr;               // split-K partial weight gradients
+    // partial gradients: hidden weights by split, biases and output layer by block
+    float *wpart[4] = {}, *bpart[4] = {}, *opart = nullptr;
     float* Y = nullptr;                     // [cap][6]
     float* dYf = nullptr;                   // [cap][6]
     double* loss = nullptr;
 };
 
 static MlpState M;
+
+// most blocks of a kernel whose partial sums are kept by block
+static int max_blocks() { return 2 * tctrain::layer_blocks(INT_MAX / 128 * 128); }
 
 static bool mlp_alloc_params()
 {
@@ -275,26 +403,28 @@ static bool mlp_alloc_params()
         M.boff[l] = off;
         off += layer_out(l);
     }
-    M.nparam = off;
+    M.nparam = off;  // = kParams
     size_t b = sizeof(float) * off;
     if (!cuda_ok(cudaMalloc(&M.p, b), "mlp params") || !cuda_ok(cudaMalloc(&M.gr, b), "mlp grads") ||
         !cuda_ok(cudaMalloc(&M.m, b), "mlp m") || !cuda_ok(cudaMalloc(&M.v, b), "mlp v"))
         return false;
+    // the rows and columns that pad the output layer's copies stay zero
+    auto zeroed = [](unsigned char*& d, size_t n, const char* what) {
+        return cuda_ok(cudaMalloc(&d, n), what) && cuda_ok(cudaMemsetAsync(d, 0, n, g.stream), what);
+    };
     for (int l = 0; l < kLayers; l++) {
-        size_t e = (size_t)layer_out_pad(l) * layer_in(l);
-        if (!cuda_ok(cudaMalloc(&M.wb[l], sizeof(__nv_bfloat16) * e), "mlp wb") ||
-            !cuda_ok(cudaMalloc(&M.wk[l], sizeof(__nv_bfloat16) * e), "mlp wk"))
+        if (!zeroed(M.cp.wk[l], sizeof(__nv_bfloat16) * layer_out_pad(l) * layer_in(l), "mlp wk") ||
+            (l > 0 && !zeroed(M.cp.wn[l],
+                              sizeof(__nv_bfloat16) * (size_t)layer_in(l) * (l == kLayers - 1 ? kDYld : kHid), "mlp wn")))
             return false;
-        if (l == 0) continue;
-        const size_t t = sizeof(__nv_bfloat16) * (size_t)layer_in(l) * (l == kLayers - 1 ? kDYld : kHid);
-        if (!cuda_ok(cudaMalloc(&M.wn[l], t), "mlp wn") ||
-            !cuda_ok(cudaMemsetAsync(M.wn[l], 0, t, g.stream), "mlp wn zero"))
+        if (l == kLayers - 1) continue;
+        if (!cuda_ok(cudaMalloc(&M.wpart[l], sizeof(float) * (size_t)kWgradSplits * kHid * layer_in(l)),
+                     "mlp weight partial") ||
+            !cuda_ok(cudaMalloc(&M.bpart[l], sizeof(float) * (size_t)max_blocks() * kHid), "mlp bias partial"))
             return false;
     }
-    return cuda_ok(cudaMalloc(&M.wpack, kPackBytes), "mlp wpack") &&
-           cuda_ok(cudaMalloc(&M.bpart, sizeof(float) * (size_t)tctrain::layer_blocks(INT_MAX / 128 * 128) * kHid),
-                   "mlp bias partial") &&
-           cuda_ok(cudaMalloc(&M.partial, sizeof(float) * (size_t)kWgradSplits * kHid * kHid), "mlp partial") &&
+    return zeroed(M.cp.pack, kPackBytes, "mlp wpack") &&
+           cuda_ok(cudaMalloc(&M.opart, sizeof(float) * (size_t)max_blocks() * kOutGrad), "mlp output partial") &&
            cuda_ok(cudaMalloc(&M.freq, sizeof(int) * 3 * kFeat), "mlp freq") &&
            cuda_ok(cudaMalloc(&M.d_mean, sizeof(float) * kOut), "mlp mean") &&
            cuda_ok(cudaMalloc(&M.d_istd, sizeof(float) * kOut), "mlp std") &&
@@ -323,20 +453,16 @@ static bool mlp_reserve(int n)
     return ok;
 }
 
-static bool mlp_refresh_bf16()
+// the BF16 copies and the output normalisation on the device
+static bool mlp_refresh()
 {
     cudaStream_t s = g.stream;
-    for (int l = 0; l < kLayers; l++) {
-        int e = layer_out_pad(l) * layer_in(l);
-        to_bf16_kernel<<<(e + 255) / 256, 256, 0, s>>>(M.p + M.woff[l], layer_out(l), layer_out_pad(l),
-                                                       layer_in(l), M.wb[l], M.wk[l], M.wn[l]);
-    }
-    if (!cuda_ok(pack_weights(M.wb, M.wpack, s), "pack weights")) return false;
+    copies_kernel<<<(kParams + 255) / 256, 256, 0, s>>>(M.p, M.cp);
     float istd[kOut];
     for (int c = 0; c < kOut; c++) istd[c] = 1.0f / M.out_std[c];
     cudaMemcpyAsync(M.d_mean, M.out_mean, sizeof(float) * kOut, cudaMemcpyHostToDevice, s);
     cudaMemcpyAsync(M.d_istd, istd, sizeof(float) * kOut, cudaMemcpyHostToDevice, s);
-    return cuda_ok(cudaGetLastError(), "bf16 refresh");
+    return cuda_ok(cudaGetLastError(), "weights refresh");
 }
 
 // forward of n samples from features X (rows up to the next multiple of 128
@@ -348,48 +474,51 @@ static bool mlp_forward(int n)
     const int np = (n + 127) / 128 * 128;
     const unsigned char* in = M.X;
     for (int l = 0; l < 4; l++) {
-        if (!cuda_ok(tctrain::forward_hidden(in, layer_in(l), M.wk[l], np, M.p + M.boff[l], M.Z[l], M.H[l],
+        if (!cuda_ok(tctrain::forward_hidden(in, layer_in(l), M.cp.wk[l], np, M.p + M.boff[l], M.Z[l], M.H[l],
                                              g.d_status, s),
                      "fwd gemm")) return false;
         in = M.H[l];
     }
-    return cuda_ok(tctrain::forward_out(in, M.wk[4], np, M.p + M.boff[4], M.Y, g.d_status, s), "out gemm");
+    return cuda_ok(tctrain::forward_out(in, M.cp.wk[4], np, M.p + M.boff[4], M.Y, g.d_status, s), "out gemm");
 }
 
 // backward of n samples (a multiple of 128) after mlp_forward and the loss
-// kernel: fills M.gr.  Data gradients and the hidden layers' weight gradients
-// on the tensor cores; bias gradients and the output layer's weight gradient
-// as reductions.
-static bool mlp_backward(int n)
+// kernel: the gradients into M.gr, or, with `step`, one AdamW step from them.
+// Data gradients and the hidden layers' weight gradients on the tensor cores;
+// bias gradients in the former's epilogue, the output layer's on the CUDA cores.
+static bool mlp_backward(int n, const Adam* step)
 {
     cudaStream_t s = g.stream;
-    cudaMemsetAsync(M.gr, 0, sizeof(float) * M.nparam, s);
-    // output layer: dW4 = dY^T H3, db4 = sum dY, dH3 = dY W4 (times silu'(Z3))
-    {
-        out_grad_kernel<<<(n + kOutRows - 1) / kOutRows, 256, 0, s>>>(M.dYf, M.H[3], n, M.gr + M.woff[4],
-                                                                       M.gr + M.boff[4]);
-        if (!cuda_ok(tctrain::backward_data(M.dY, kDYld, M.wn[4], n, M.Z[3], M.G0, M.bpart, g.d_status, s),
-                     "dH3"))
-            return false;
-    }
-    unsigned char *gcur = M.G0, *gnext = M.G1;
+    const int oblocks = std::min(n / 128, max_blocks());
+    out_grad_kernel<<<oblocks, 256, 0, s>>>(M.dYf, M.H[3], n / 128, M.opart);
     // split the samples so that the two 128-row tiles fill the SMs, at least
     // four steps of 64 per split
     const int splits = std::max(1, std::min({kWgradSplits, 76, n / 256}));
+    const unsigned char* gin = M.dY;
+    unsigned char *gcur = M.G0, *gnext = M.G1;
+    Partials ps;
     for (int l = 3; l >= 0; l--) {
-        bias_grad_kernel<<<1, kHid, 0, s>>>(M.bpart, tctrain::layer_blocks(n), M.gr + M.boff[l]);
-        if (!cuda_ok(tctrain::backward_weights(gcur, l == 0 ? M.X : M.H[l - 1], layer_in(l), n, M.partial, splits,
-                                               M.gr + M.woff[l], g.d_status, s),
+        if (!cuda_ok(tctrain::backward_data(gin, l == 3 ? kDYld : kHid, M.cp.wn[l + 1], n, M.Z[l], gcur, M.bpart[l],
+                                            g.d_status, s),
+                     "dH") ||
+            !cuda_ok(tctrain::backward_weights(gcur, l == 0 ? M.X : M.H[l - 1], layer_in(l), n, M.wpart[l], splits,
+                                               g.d_status, s),
                      "dW"))
             return false;
-        if (l > 0) {
-            if (!cuda_ok(tctrain::backward_data(gcur, kHid, M.wn[l], n, M.Z[l - 1], gnext, M.bpart, g.d_status, s),
-                         "dH"))
-                return false;
-            std::swap(gcur, gnext);
-        }
+        ps.w[l] = M.wpart[l];
+        ps.b[l] = M.bpart[l];
+        gin = gcur;
+        std::swap(gcur, gnext);
     }
-    return true;
+    ps.out = M.opart;
+    ps.splits = splits;
+    ps.bblocks = tctrain::layer_blocks(n);
+    ps.oblocks = oblocks;
+    if (step)
+        update_kernel<true><<<kUpdateBlocks, 256, 0, s>>>(ps, nullptr, M.p, M.m, M.v, *step, M.cp);
+    else
+        update_kernel<false><<<kUpdateBlocks, 256, 0, s>>>(ps, M.gr, nullptr, nullptr, nullptr, Adam{}, M.cp);
+    return cuda_ok(cudaGetLastError(), "update");
 }
 
 static bool mlp_loss(int n, const float* T, double* loss_out)
@@ -411,12 +540,9 @@ bool mlp::mlp_model(Model& md)
         set_error(12, "the learned field model is not trained (tp_mlp_train)");
         return false;
     }
-    for (int l = 0; l < kLayers; l++) {
-        md.w[l] = M.wb[l];
-        md.b[l] = M.p + M.boff[l];
-    }
+    for (int l = 0; l < kLayers; l++) md.b[l] = M.p + M.boff[l];
     md.freq = M.freq;
-    md.wpack = M.wpack;
+    md.wpack = M.cp.pack;
     for (int c = 0; c < kOut; c++) {
         md.out_scale[c] = M.out_std[c];
         md.out_shift[c] = M.out_mean[c];
@@ -457,7 +583,7 @@ extern "C" int tp_mlp_init(const int* freq, const float* weights, unsigned long 
     cudaMemsetAsync(M.v, 0, sizeof(float) * M.nparam, g.stream);
     M.step = 0;
     M.ready = true;
-    return mlp_refresh_bf16() && cuda_ok(cudaStreamSynchronize(g.stream), "mlp init") ? 0 : -1;
+    return mlp_refresh() && cuda_ok(cudaStreamSynchronize(g.stream), "mlp init") ? 0 : -1;
 }
 
 extern "C" int tp_mlp_param_count(void)
@@ -473,7 +599,7 @@ extern "C" int tp_mlp_set_output_norm(const float* mean, const float* stdv)
         M.out_mean[c] = mean[c];
         M.out_std[c] = stdv[c];
     }
-    return M.ready && mlp_refresh_bf16() ? 0 : -1;
+    return M.ready && mlp_refresh() ? 0 : -1;
 }
 
 extern "C" int tp_mlp_get_weights(float* weights)
@@ -502,7 +628,7 @@ extern "C" int tp_mlp_grad(int n, const unsigned int* u, const float* t, double*
     cudaMemcpyAsync(dU, u, sizeof(uint32_t) * 3 * n, cudaMemcpyHostToDevice, s);
     cudaMemcpyAsync(dT, t, sizeof(float) * 6 * n, cudaMemcpyHostToDevice, s);
     features_kernel<<<(n + 127) / 128, 128, 0, s>>>(dU, n, M.freq, M.X);
-    bool ok = mlp_forward(n) && mlp_loss(n, dT, loss) && mlp_backward(n);
+    bool ok = mlp_forward(n) && mlp_loss(n, dT, loss) && mlp_backward(n, nullptr);
     if (ok) {
         if (y) cudaMemcpyAsync(y, M.Y, sizeof(float) * 6 * n, cudaMemcpyDeviceToHost, s);
         if (grads) cudaMemcpyAsync(grads, M.gr, sizeof(float) * M.nparam, cudaMemcpyDeviceToHost, s);
@@ -569,15 +695,12 @@ extern "C" int tp_mlp_train(long long nsamples, int batch, int epochs, double lr
     long long nb = nsamples / batch;
     long long total = nb * epochs;
     double loss = 0.0;
-    bool ok = mlp_refresh_bf16();
+    bool ok = mlp_refresh();
     for (long long it = 0; it < total && ok; it++) {
         long long bi = it % nb;
         features_kernel<<<(batch + 127) / 128, 128, 0, s>>>(dU + 3 * bi * batch, batch, M.freq, M.X);
         const bool last = it == total - 1;
-        ok = mlp_forward(batch) && mlp_loss(batch, dT + 6 * bi * batch, last ? &loss : nullptr) &&
-             mlp_backward(batch);
-        if (!ok) break;
-        M.step++;
+        const long step = M.step + 1;
         Adam a;
         double frac = (double)it / (double)total;
         a.lr = (float)(lr * 0.5 * (1.0 + std::cos(M_PI * frac)));
@@ -585,10 +708,11 @@ extern "C" int tp_mlp_train(long long nsamples, int batch, int epochs, double lr
         a.b2 = 0.999f;
         a.eps = 1e-8f;
         a.wd = (float)wd;
-        a.c1 = (float)(1.0 / (1.0 - std::pow(0.9, (double)M.step)));
-        a.c2 = (float)(1.0 / (1.0 - std::pow(0.999, (double)M.step)));
-        adamw_kernel<<<(int)((M.nparam + 255) / 256), 256, 0, s>>>(M.p, M.gr, M.m, M.v, (int)M.nparam, a);
-        ok = mlp_refresh_bf16();
+        a.c1 = (float)(1.0 / (1.0 - std::pow(0.9, (double)step)));
+        a.c2 = (float)(1.0 / (1.0 - std::pow(0.999, (double)step)));
+        ok = mlp_forward(batch) && mlp_loss(batch, dT + 6 * bi * batch, last ? &loss : nullptr) &&
+             mlp_backward(batch, &a);
+        if (ok) M.step = step;
     }
     cudaEventRecord(e1, s);
     ok = ok && cuda_ok(cudaStreamSynchronize(s), "train");

@@ -5,6 +5,8 @@
 #include <cuda_bf16.h>
 #include <cstdint>
 
+#include "tc_sm100.cuh"
+
 namespace tp {
 namespace mlp {
 
@@ -21,7 +23,6 @@ __host__ __device__ constexpr int layer_out_pad(int l) { return l == kLayers - 1
 
 // Device view of the trained model used for inference.
 struct Model {
-    const __nv_bfloat16* w[kLayers];  // [out_pad][in] row-major, BF16
     const float* b[kLayers];          // [out] FP32
     const int* freq;                  // [kFeat][3] integer lattice frequencies
     const unsigned char* wpack;       // weights in the tensor-core chunk layout (kPackBytes)
@@ -34,8 +35,14 @@ constexpr size_t kPackBytes = 466944;
 // Device view of the trained model (host side; false and an error if untrained).
 bool mlp_model(Model& md);
 
-// Packs the BF16 weights of every layer for the tensor-core inference.
-cudaError_t pack_weights(const __nv_bfloat16* const w[kLayers], unsigned char* pack, cudaStream_t s);
+// byte offset in the pack of weight (n, k) of layer l (n < padded outputs)
+__host__ __device__ __forceinline__ uint32_t pack_offset(int l, int n, int k)
+{
+    if (l == kLayers - 1) return 458752u + (uint32_t)(k >> 6) * 2048u + tc::sw128_offset(16, n, k & 63);
+    const int h = n >> 7, a = k >> 6;
+    const uint32_t base = l == 0 ? 0u : 65536u + (uint32_t)(l - 1) * 131072u;
+    return base + (uint32_t)(2 * a + h) * 16384u + tc::sw128_offset(128, n & 127, k & 63);
+}
 
 __device__ __forceinline__ float silu(float z)
 {

@@ -577,26 +577,6 @@ __global__ void __launch_bounds__(kDwThreads, 1)
     if (warp == 1) tc::tmem_dealloc(tmem, cols);
 }
 
-// D[m][n] (row length ncol) = the sum over the splits of P[split][m / 128][n][m % 128]
-// (nrow rows of tiles, npad columns held): a block takes 32 m x 8 n, read 128
-// bytes at a time and written through shared memory in 32-byte pieces.
-__global__ void __launch_bounds__(256) sum_splits_kernel(const float* __restrict__ P, int splits, int mtiles,
-                                                         int npad, int ncol, float* __restrict__ D)
-{
-    __shared__ float tile[8][33];
-    const int m0 = blockIdx.x * 32, n0 = blockIdx.y * 8;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const float* src = P + ((size_t)(m0 >> 7) * npad + n0 + w) * 128 + (m0 & 127) + lane;
-    const size_t step = (size_t)mtiles * npad * 128;
-    float s = 0.f;
-#pragma unroll 8
-    for (int k = 0; k < splits; k++) s += src[k * step];
-    tile[w][lane] = s;
-    __syncthreads();
-    const int m = threadIdx.x >> 3, n = threadIdx.x & 7;
-    if (n0 + n < ncol) D[(size_t)(m0 + m) * ncol + n0 + n] = tile[n][m];
-}
-
 static cudaError_t launch_weights(const void* G, int mtiles, const void* X, int xatoms, int nsteps, float* P,
                                   int splits, int* status, cudaStream_t s)
 {
@@ -607,6 +587,15 @@ static cudaError_t launch_weights(const void* G, int mtiles, const void* X, int 
         static_cast<const unsigned char*>(G), 2 * mtiles, static_cast<const unsigned char*>(X), xatoms, nsteps, P,
         status);
     return cudaGetLastError();
+}
+
+// Self-check: D[m][n] of one split of P
+__global__ void from_split_kernel(const float* __restrict__ P, int M, int N, int npad, float* __restrict__ D)
+{
+    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= (size_t)M * N) return;
+    const int m = (int)(i / N), n = (int)(i % N);
+    D[i] = P[((size_t)(m >> 7) * npad + n) * 128 + (m & 127)];
 }
 
 // Self-check: row-major A [rows][K] into blocks (kind 0), k-atoms of R rows
@@ -655,13 +644,10 @@ cudaError_t backward_data(const void* Gin, int kout, const void* WT, int M, cons
     return launch_layer<256>(Gin, WT, M, kout, e, status, s);
 }
 
-cudaError_t backward_weights(const void* G, const void* X, int kin, int nsamp, float* partial, int splits,
-                             float* gr, int* status, cudaStream_t s)
+cudaError_t backward_weights(const void* G, const void* X, int kin, int nsamp, float* P, int splits, int* status,
+                             cudaStream_t s)
 {
-    cudaError_t e = launch_weights(G, mlp::kHid / 128, X, kin / 64, nsamp / 64, partial, splits, status, s);
-    if (e != cudaSuccess) return e;
-    sum_splits_kernel<<<dim3(mlp::kHid / 32, kin / 8), 256, 0, s>>>(partial, splits, mlp::kHid / 128, kin, kin, gr);
-    return cudaGetLastError();
+    return launch_weights(G, mlp::kHid / 128, X, kin / 64, nsamp / 64, P, splits, status, s);
 }
 
 // the shapes of the layer GEMMs go through the kernel those use, the others
@@ -679,7 +665,7 @@ static cudaError_t gemm_f32(const __nv_bfloat16* A, const __nv_bfloat16* B, int 
     float* P = reinterpret_cast<float*>(wb + 2 * (size_t)npad * kpad);
     cudaError_t e = launch_weights(wa, M / 128, wb, npad / 64, K / 64, P, 1, status, s);
     if (e != cudaSuccess) return e;
-    sum_splits_kernel<<<dim3(M / 32, npad / 8), 256, 0, s>>>(P, 1, M / 128, npad, N, D);
+    from_split_kernel<<<grid((size_t)M * N), 256, 0, s>>>(P, M, N, npad, D);
     return cudaGetLastError();
 }
 

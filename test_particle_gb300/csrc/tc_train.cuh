@@ -34,10 +34,10 @@ cudaError_t forward_out(const void* H3, const void* W4, int M, const float* b, f
 cudaError_t backward_data(const void* Gin, int kout, const void* WT, int M, const void* Zprev, void* G,
                           float* bpart, int* status, cudaStream_t s);
 
-// gr[256][kin] = G^T X over nsamp samples: G [nsamp][256], X [nsamp][kin]; `splits`
-// (at most nsamp / 64) partial sums in `partial` (splits x 256 x kin FP32), summed into gr.
-cudaError_t backward_weights(const void* G, const void* X, int kin, int nsamp, float* partial, int splits,
-                             float* gr, int* status, cudaStream_t s);
+// The gradient G^T X [256][kin] over nsamp samples, G [nsamp][256], X [nsamp][kin],
+// as `splits` (at most nsamp / 64) partial sums: P[split][m / 128][k][m % 128] FP32.
+cudaError_t backward_weights(const void* G, const void* X, int kin, int nsamp, float* P, int splits,
+                             int* status, cudaStream_t s);
 
 }  // namespace tctrain
 }  // namespace tp
