@@ -252,19 +252,21 @@ static bool run_range(int nptl, const RunSpec& rs, particles* ptl_init, particle
                       RunOut& o, double* wall_ms)
 {
     Session& s = cached_session();
-    if (!s.load(ptl_init, ptl, nptl)) return false;
-    if (rs.traj_every > 0 && !s.set_traj(ntraj_accum, ptl_time, traj_points)) return false;
+    // the caller's records may still be read or written in place when a call fails
+    auto fail = [] { return cudaStreamSynchronize(g.stream), false; };
+    if (!s.load(ptl_init, ptl, nptl)) return fail();
+    if (rs.traj_every > 0 && !s.set_traj(ntraj_accum, ptl_time, traj_points)) return fail();
     if (!rs.reset_nsteps && nsteps_ptl && nptl > 0)
         cudaMemcpyAsync(s.nsteps.ptr, nsteps_ptl, sizeof(int) * nptl, cudaMemcpyHostToDevice, g.stream);
     tp_run_info info;
-    if (!s.run(rs, &info)) return false;
+    if (!s.run(rs, &info)) return fail();
     size_t nspec = (size_t)rs.nt_out * rs.nbins;
     o.espect.assign(nspec, 0.0);
     o.espect_esc.assign(nspec, 0.0);
     o.dsum.assign((size_t)8 * s.nsdc, 0.0);
     o.remain.assign(s.nsdc, 0);
     if (!s.fetch(ptl, nsteps_ptl, o.espect.data(), o.espect_esc.data(), o.dsum.data(),
-                 o.remain.data())) return false;
+                 o.remain.data())) return fail();
     if (rs.traj_every > 0 && !s.get_traj(ptl_time, traj_points)) return false;
     if (wall_ms) *wall_ms = info.kernel_ms;
     return true;
