@@ -161,34 +161,8 @@ __global__ void __launch_bounds__(128) moments_kernel(const float* __restrict__ 
 }
 
 // ---------------------------------------------------------------- loss, output layer, AdamW
-// dY = 2 (y - t_n) / (n * 6) with t_n the normalised target; BF16 dY padded with
-// zeros to kDYld columns (one k-atom of the output layer's data-gradient GEMM), in
-// the GEMMs' blocks; the kernel writes the first 8, the rest are zeroed once
-constexpr int kDYld = 64;
+constexpr int kDYld = 64;         // columns of dY: one k-atom of the output layer's data-gradient GEMM
 constexpr int kWgradSplits = 80;  // most split-K parts of a weight-gradient GEMM
-__global__ void loss_kernel(const float* __restrict__ Y, const float* __restrict__ T, int n,
-                            const float* __restrict__ mean, const float* __restrict__ istd,
-                            unsigned char* __restrict__ dY, float* __restrict__ dYf,
-                            double* __restrict__ loss)
-{
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    float l = 0.f;
-    if (i < n) {
-        const float scale = 2.0f / ((float)n * kOut);
-        float g[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-        for (int c = 0; c < kOut; c++) {
-            float r = Y[(size_t)i * kOut + c] - (T[(size_t)i * kOut + c] - mean[c]) * istd[c];
-            l += r * r;
-            g[c] = r * scale;
-            if (dYf) dYf[(size_t)i * kOut + c] = g[c];
-        }
-        // columns 8.. of dY stay zero from its allocation (mlp_reserve)
-        *reinterpret_cast<uint4*>(dY + tctrain::tile_offset(i, 0, 1)) =
-            make_uint4(pack_bf16(g[0], g[1]), pack_bf16(g[2], g[3]), pack_bf16(g[4], g[5]), pack_bf16(g[6], g[7]));
-    }
-    for (int off = 16; off > 0; off >>= 1) l += __shfl_down_sync(0xffffffffu, l, off);
-    if ((threadIdx.x & 31) == 0) atomicAdd(loss, (double)l);
-}
 
 // Partial sums of the output layer's gradients from the FP32 loss gradient dYf
 // [n][6] and the last hidden activations H3 [n][256]: part[block] holds
@@ -482,7 +456,7 @@ static bool mlp_reserve(int n)
               cuda_ok(cudaMalloc(&M.dYf, sizeof(float) * (size_t)n * kOut), "dYf");
     for (int l = 0; l < 4 && ok; l++)
         ok = cuda_ok(cudaMalloc(&M.Z[l], h), "Z") && cuda_ok(cudaMalloc(&M.H[l], h), "H");
-    // the padding columns of dY (beyond the 8 the loss kernel writes) stay zero
+    // the padding columns of dY (beyond the 8 that forward_loss writes) stay zero
     if (ok) ok = cuda_ok(cudaMemsetAsync(M.dY, 0, sizeof(__nv_bfloat16) * (size_t)n * kDYld, g.stream), "dY zero");
     if (ok) M.cap = n;
     return ok;
@@ -501,9 +475,9 @@ static bool mlp_refresh()
 }
 
 // forward of n samples from features X (rows up to the next multiple of 128
-// are computed too and ignored): fills Z/H and Y
-// (normalised outputs), on the tensor cores
-static bool mlp_forward(int n)
+// are computed too and ignored): fills Z/H and Y (normalised outputs), on the
+// tensor cores
+static bool mlp_hidden(int n)
 {
     cudaStream_t s = g.stream;
     const int np = (n + 127) / 128 * 128;
@@ -514,11 +488,36 @@ static bool mlp_forward(int n)
                      "fwd gemm")) return false;
         in = M.H[l];
     }
-    return cuda_ok(tctrain::forward_out(in, M.cp.wk[4], np, M.p + M.boff[4], M.Y, g.d_status, s), "out gemm");
+    return true;
 }
 
-// backward of n samples (a multiple of 128) after mlp_forward and the loss
-// kernel: the gradients into M.gr, or, with `step`, one AdamW step from them.
+static bool mlp_forward(int n)
+{
+    return mlp_hidden(n) && cuda_ok(tctrain::forward_out(M.H[3], M.cp.wk[4], (n + 127) / 128 * 128, M.p + M.boff[4],
+                                                         M.Y, g.d_status, g.stream),
+                                    "out gemm");
+}
+
+// the same for a multiple of 128 samples with targets T: the loss gradient and,
+// with loss_out, the mean loss; Y only with keep_y
+static bool mlp_forward_loss(int n, const float* T, bool keep_y, double* loss_out)
+{
+    cudaStream_t s = g.stream;
+    cudaMemsetAsync(M.loss, 0, sizeof(double), s);
+    const tctrain::Loss ls = {T, M.d_mean, M.d_istd, M.dY, M.dYf, M.loss};
+    if (!mlp_hidden(n) || !cuda_ok(tctrain::forward_loss(M.H[3], M.cp.wk[4], n, M.p + M.boff[4],
+                                                         keep_y ? M.Y : nullptr, ls, g.d_status, s),
+                                   "out gemm"))
+        return false;
+    if (loss_out) {
+        cudaMemcpyAsync(loss_out, M.loss, sizeof(double), cudaMemcpyDeviceToHost, s);
+        if (!cuda_ok(cudaStreamSynchronize(s), "loss")) return false;
+        *loss_out /= (double)n * kOut;
+    }
+    return true;
+}
+
+// backward of n samples (a multiple of 128) after mlp_forward_loss: the gradients into M.gr, or, with `step`, one AdamW step from them.
 // Data gradients and the hidden layers' weight gradients on the tensor cores;
 // bias gradients in the former's epilogue, the output layer's on the CUDA cores.
 static bool mlp_backward(int n, const Adam* step)
@@ -554,19 +553,6 @@ static bool mlp_backward(int n, const Adam* step)
     else
         update_kernel<false><<<kUpdateBlocks, 256, 0, s>>>(ps, M.gr, nullptr, nullptr, nullptr, Adam{}, M.cp);
     return cuda_ok(cudaGetLastError(), "update");
-}
-
-static bool mlp_loss(int n, const float* T, double* loss_out)
-{
-    cudaStream_t s = g.stream;
-    cudaMemsetAsync(M.loss, 0, sizeof(double), s);
-    loss_kernel<<<(n + 255) / 256, 256, 0, s>>>(M.Y, T, n, M.d_mean, M.d_istd, M.dY, M.dYf, M.loss);
-    if (loss_out) {
-        cudaMemcpyAsync(loss_out, M.loss, sizeof(double), cudaMemcpyDeviceToHost, s);
-        if (!cuda_ok(cudaStreamSynchronize(s), "loss")) return false;
-        *loss_out /= (double)n * kOut;
-    }
-    return cuda_ok(cudaGetLastError(), "loss");
 }
 
 bool mlp::mlp_model(Model& md)
@@ -663,7 +649,7 @@ extern "C" int tp_mlp_grad(int n, const unsigned int* u, const float* t, double*
     cudaMemcpyAsync(dU, u, sizeof(uint32_t) * 3 * n, cudaMemcpyHostToDevice, s);
     cudaMemcpyAsync(dT, t, sizeof(float) * 6 * n, cudaMemcpyHostToDevice, s);
     features_kernel<<<(n + 127) / 128, 128, 0, s>>>(dU, n, M.freq, M.X);
-    bool ok = mlp_forward(n) && mlp_loss(n, dT, loss) && mlp_backward(n, nullptr);
+    bool ok = mlp_forward_loss(n, dT, true, loss) && mlp_backward(n, nullptr);
     if (ok) {
         if (y) cudaMemcpyAsync(y, M.Y, sizeof(float) * 6 * n, cudaMemcpyDeviceToHost, s);
         if (grads) cudaMemcpyAsync(grads, M.gr, sizeof(float) * M.nparam, cudaMemcpyDeviceToHost, s);
@@ -749,8 +735,7 @@ extern "C" int tp_mlp_train(long long nsamples, int batch, int epochs, double lr
         a.wd = (float)wd;
         a.c1 = (float)(1.0 / (1.0 - std::pow(0.9, (double)step)));
         a.c2 = (float)(1.0 / (1.0 - std::pow(0.999, (double)step)));
-        ok = mlp_forward(batch) && mlp_loss(batch, dT + 6 * bi * batch, last ? &loss : nullptr) &&
-             mlp_backward(batch, &a);
+        ok = mlp_forward_loss(batch, dT + 6 * bi * batch, false, last ? &loss : nullptr) && mlp_backward(batch, &a);
         if (ok) M.step = step;
     }
     cudaEventRecord(e1, s);

@@ -266,6 +266,42 @@ struct EpiOut {
     __device__ void tail(uint32_t) {}
 };
 
+// The same in a training batch of n samples, with the loss: r = y - (t - mean) /
+// std, its gradient dY = 2 r / (n kOut) as FP32 rows and, in BF16, the first
+// eight columns of a block (the others stay zero), and the sum of r^2.  (As a
+// kernel of its own behind the GEMM this took 5.9 us for 65,536 samples.)
+struct EpiOutLoss {
+    const float* b;
+    float* Y;  // null: not kept
+    tctrain::Loss ls;
+    float scale;
+    __device__ void begin(const Warp&, int, int) {}
+    __device__ bool block(const Warp& w, int t, int, int, uint32_t acc)
+    {
+        const size_t m = (size_t)t * 128 + 32 * w.q + w.lane;
+        float tg[mlp::kOut], v[16];
+        for (int c = 0; c < mlp::kOut; c++) tg[c] = ls.T[m * mlp::kOut + c];
+        tc::tmem_ld16(acc, v);
+        float l = 0.f, g[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        for (int c = 0; c < mlp::kOut; c++) {
+            const float y = v[c] + b[c];
+            if (Y) Y[m * mlp::kOut + c] = y;
+            const float r = y - (tg[c] - ls.mean[c]) * ls.istd[c];
+            l += r * r;
+            g[c] = r * scale;
+            ls.dYf[m * mlp::kOut + c] = g[c];
+        }
+        *reinterpret_cast<uint4*>(ls.dY + tctrain::tile_offset(m, 0, 1)) =
+            make_uint4(mlp::pack_bf16(g[0], g[1]), mlp::pack_bf16(g[2], g[3]), mlp::pack_bf16(g[4], g[5]),
+                       mlp::pack_bf16(g[6], g[7]));
+        for (int off = 16; off > 0; off >>= 1) l += __shfl_down_sync(0xffffffffu, l, off);
+        if (w.lane == 0) atomicAdd(ls.sum, (double)l);
+        return true;
+    }
+    __device__ void finish(const Warp&) {}
+    __device__ void tail(uint32_t) {}
+};
+
 struct EpiStoreF32 {  // D[m][n] = acc (self-check)
     float* D;
     __device__ void begin(const Warp&, int, int) {}
@@ -632,6 +668,13 @@ cudaError_t forward_out(const void* H3, const void* W4, int M, const float* b, f
                         cudaStream_t s)
 {
     return launch_layer<mlp::kOutPad>(H3, W4, M, mlp::kHid, EpiOut{b, Y}, status, s);
+}
+
+cudaError_t forward_loss(const void* H3, const void* W4, int M, const float* b, float* Y, const Loss& ls, int* status,
+                         cudaStream_t s)
+{
+    return launch_layer<mlp::kOutPad>(H3, W4, M, mlp::kHid,
+                                      EpiOutLoss{b, Y, ls, 2.0f / ((float)M * mlp::kOut)}, status, s);
 }
 
 cudaError_t backward_data(const void* Gin, int kout, const void* WT, int M, const void* Zprev, void* G,

@@ -29,6 +29,18 @@ cudaError_t forward_hidden(const void* X, int kin, const void* W, int M, const f
 cudaError_t forward_out(const void* H3, const void* W4, int M, const float* b, float* Y, int* status,
                         cudaStream_t s);
 
+// The same with the loss of M samples against the targets T [M][6]: the gradient dYf
+// (FP32 rows) and dY (BF16 blocks of 64 columns, of which the first 8 are written), the
+// sum of the squares added to *sum; Y may be null.
+struct Loss {
+    const float *T, *mean, *istd;
+    unsigned char* dY;
+    float* dYf;
+    double* sum;
+};
+cudaError_t forward_loss(const void* H3, const void* W4, int M, const float* b, float* Y, const Loss& ls, int* status,
+                         cudaStream_t s);
+
 // G = (Gin WT^T) * silu'(Zprev): Gin [M][kout], WT [256][kout] (the layer's weights
 // transposed); G [M][256], its column sums over a block's samples in bpart [layer_blocks(M)][256].
 cudaError_t backward_data(const void* Gin, int kout, const void* WT, int M, const void* Zprev, void* G,
