@@ -7,7 +7,7 @@
 // in known ranges.  So each term is evaluated and summed in integers and one
 // conversion per component makes the double.  The FP64 cosine and sums took
 // about 2900 cycles a warp and mode; a run of 65,536 particles over 10 steps in
-// a 512-mode field (host buffers in and out) went from 49.8 to 5.6 ms, and a
+// a 512-mode field (host buffers in and out) went from 49.8 to 5.1 ms, and a
 // training run on 131,072 samples of such a field from 9.64 to 6.60 ms.  It is
 // bound by the issue of 126 instructions a mode (43 multiply-adds, 65 on the
 // half-rate integer pipe) and by four warps on one sub-partition where others
