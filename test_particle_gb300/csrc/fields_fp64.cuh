@@ -476,7 +476,7 @@ __device__ __forceinline__ uint64_t fixed_frac64(double u)
 __device__ __forceinline__ void mode_sum_fixed(const DevField& f, const int4* tab, const uint64_t u[3], double e[6])
 {
     int64_t s[6];
-    fx::mode_sum(f.fxm, f.nfx, tab, u, s);
+    fx::mode_sum<fx::kChunk>(f.fxm, f.nfx, tab, u, s);
 #pragma unroll
     for (int k = 0; k < 6; k++) e[k] = (double)s[k] * f.fxs[k];
 }

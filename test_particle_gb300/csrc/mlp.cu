@@ -99,7 +99,7 @@ __global__ void __launch_bounds__(128) samples_kernel(uint64_t seed, long long f
     if (f.fxm) {
         const uint64_t u64[3] = {(uint64_t)u[0] << 32, (uint64_t)u[1] << 32, (uint64_t)u[2] << 32};
         int64_t s[6];
-        fx::mode_sum(f.fxm, f.nfx, tab, u64, s);
+        fx::mode_sum<fx::kChunk>(f.fxm, f.nfx, tab, u64, s);
         for (int k = 0; k < 3; k++) {
             b[k] = (double)s[k] * f.fxs[k];
             e[k] = (double)s[3 + k] * f.fxs[3 + k];

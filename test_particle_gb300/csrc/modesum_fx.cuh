@@ -7,7 +7,7 @@
 // in known ranges.  So each term is evaluated and summed in integers and one
 // conversion per component makes the double.  The FP64 cosine and sums took
 // about 2900 cycles a warp and mode; a run of 65,536 particles over 10 steps in
-// a 512-mode field (host buffers in and out) went from 49.8 to 5.1 ms, and a
+// a 512-mode field (host buffers in and out) went from 49.8 to 4.8 ms, and a
 // training run on 131,072 samples of such a field from 9.64 to 6.60 ms.  It is
 // bound by the issue of 126 instructions a mode (43 multiply-adds, 65 on the
 // half-rate integer pipe) and by four warps on one sub-partition where others
@@ -100,7 +100,12 @@ __host__ __device__ __forceinline__ void cosine(uint64_t ph, const int4* tab, in
 // The six components at the point with box fractions u (64-bit fixed point),
 // as integers to be multiplied with the components' scales.  nm is a multiple
 // of kChunk (tables are padded with zero amplitudes).  Chunks first, first +
-// step, ... only: the sums of all of them add up exactly.
+// step, ... only: the sums of all of them add up exactly.  U modes are unrolled:
+// a whole chunk where a thread has a particle of its own (65,536 particles x 10
+// steps, 512 modes: 5.10 ms with four, 4.83 with eight; 30,000: 2.95 and 2.71;
+// only 30,000 with 2,000 modes, whose table leaves L1, loses 1.3 %), four where
+// four lanes share one and the warps are many (19,000: 1.70 and 1.72 ms).
+template <int U>
 __host__ __device__ __forceinline__ void mode_sum(const Mode* modes, int nm, const int4* tab, const uint64_t u[3],
                                                   int64_t out[6], int first = 0, int step = 1)
 {
@@ -114,7 +119,7 @@ __host__ __device__ __forceinline__ void mode_sum(const Mode* modes, int nm, con
     int64_t hh[6] = {0, 0, 0, 0, 0, 0}, mid[6] = {0, 0, 0, 0, 0, 0};
     for (int m0 = first * kChunk; m0 < nm; m0 += step * kChunk) {
 #ifdef __CUDA_ARCH__
-#pragma unroll 4
+#pragma unroll U
 #endif
         for (int m = m0; m < m0 + kChunk; m++) {
             int4 r[4];

@@ -71,7 +71,7 @@ __device__ __forceinline__ void small_field(const DevField& f, int c, double x, 
                                fixed_frac64((grp(x, 2) - f.zmin) / (f.zmax - f.zmin))};
         // every fourth chunk of modes; the integer sums of the chunks add in any order
         int64_t s[6];
-        fx::mode_sum(f.fxm, f.nfx, s_ctab, u, s, threadIdx.x & 3, 4);
+        fx::mode_sum<4>(f.fxm, f.nfx, s_ctab, u, s, threadIdx.x & 3, 4);
         int64_t b = 0, e = 0;
 #pragma unroll
         for (int k = 0; k < 3; k++) {
