@@ -238,8 +238,9 @@ __device__ __forceinline__ void mode_sum_mixed(const MixField& f, const uint64_t
     }
     const int npairs = (f.nmodes + 1) >> 1;
     // two positions: four pairs of modes in flight (8.69 against 8.97 ms with
-    // two, 262,144 particles x 50 steps, 512 modes); one position: two
-    constexpr int U = NP > 1 ? 4 : 2;
+    // two, 262,144 particles x 50 steps, 512 modes); one position: eight (1,000
+    // particles 0.75 ms, with two 1.01; 38,000: 1.31 and 1.41)
+    constexpr int U = NP > 1 ? 4 : 8;
 #pragma unroll U
     for (int q = 0; q < npairs; q++) {
         const int4 na = smodes[q].nph[0], nb = smodes[q].nph[1];

@@ -500,13 +500,13 @@ cudaError_t launch_emf_batch(const MixField& f, int n, const double* xyz, float*
 }
 
 // --------------------------------------------------------------- launchers
-// The mode sum with two particles a thread: from one 256-particle tile per SM
-// (152 of them) on -- below, half as many warps hide less latency than the
-// shared reads save (32,768 particles: 1.74 against 1.65 ms; 65,536: 2.80
-// against 2.97; 155,648: 5.27 against 5.91) -- and up to the modes whose
-// records leave room for two blocks (1,000 modes, 65,536 particles: 4.73
-// against 5.79 ms).
-constexpr int kPairParticles = 152 * 2 * kBlock;
+// The mode sum with two particles a thread: above three 128-particle blocks per
+// SM (152 of them) -- up to there a particle a thread needs no more rounds of
+// latency than pairs do (38,000 particles: 1.30 ms against 1.32; 50,000: 1.84
+// against 2.16; 60,000: 2.42 against 2.17; 262,144: 8.03 against 6.84) -- and up
+// to the modes whose records leave room for two blocks (1,000 modes, 65,536
+// particles: 4.73 against 5.79 ms).
+constexpr int kPairParticles = 152 * 3 * kBlock;
 constexpr int kPairModes = 1024;
 template <int SYS>
 static cudaError_t launch_sys(const MixField& f, const TrackBufs& b, const TrackParams& q, int grid,
@@ -543,7 +543,7 @@ cudaError_t launch_track(const MixField& f, const TrackBufs& b, const TrackParam
     case TP_SYS_FORCEFREE: return launch_sys<TP_SYS_FORCEFREE>(f, b, q, grid, s);
     case TP_SYS_PIC: return launch_sys<TP_SYS_PIC>(f, b, q, grid, s);
     case TP_SYS_MODESUM:
-        if (f.nmodes <= kPairModes && q.n >= kPairParticles) return launch_modes(f, b, q, grid, s);
+        if (f.nmodes <= kPairModes && q.n > kPairParticles) return launch_modes(f, b, q, grid, s);
         return launch_sys<TP_SYS_MODESUM>(f, b, q, grid, s);
     default: return cudaErrorInvalidValue;
     }

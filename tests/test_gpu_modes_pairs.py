@@ -1,4 +1,4 @@
-"""The mixed mode-sum run with two particles a thread (from 38,912 particles on)
+"""The mixed mode-sum run with two particles a thread (above 58,368 particles)
 against the one-particle kernel: the same particles in small runs, bit for bit."""
 import numpy as np
 import pytest
@@ -9,7 +9,9 @@ import test_particle_gb300.workloads as wl  # noqa: E402
 
 
 @pytest.mark.parametrize("n,nmodes,bc,nbins", [(38912, 33, 0, 200), (38913, 32, 1, 200), (39000 + 255, 1, 0, 5000),
-                                               (40001, 1024, 0, 200), (38912, 1025, 0, 3)])
+                                               (40001, 1024, 0, 200), (38912, 1025, 0, 3),
+                                               (58368, 33, 0, 200), (58369, 32, 1, 200), (58369 + 255, 1, 0, 5000),
+                                               (60001, 1024, 0, 200), (58369, 1025, 0, 3)])
 def test_pairs_match_single(n, nmodes, bc, nbins):
     modes = wl.kolmogorov_modes(nmodes, 1.0, 32.0, 0.5, 3, va=0.1)
     dom = tp.Domain()
