@@ -1,7 +1,7 @@
 // mlp.cu -- training and inference of the learned field model: the forward,
 // data-gradient and hidden weight-gradient GEMMs on the 5th-generation tensor
 // cores (tc_train.cu: tcgen05.mma, FP32 accumulation in tensor memory, fused
-// bias / SiLU / SiLU-derivative / bias-gradient epilogues), Fourier features, MSE
+// bias / SiLU / SiLU-derivative / loss epilogues), Fourier features, MSE
 // loss, the output layer's 6 x 256 weight gradient as a reduction on the CUDA
 // cores, and one kernel a batch that sums the partial gradients and takes the
 // AdamW step.
@@ -274,11 +274,10 @@ __global__ void copies_kernel(const float* __restrict__ p, const __grid_constant
 }
 
 // Partial sums of the gradients: the hidden layers' weights by split
-// (backward_weights), their biases by block of the data-gradient GEMM, the
-// output layer by block of out_grad_kernel.
+// (backward_weights), their biases in kBiasParts shares, the output layer by block of out_grad_kernel.
 struct Partials {
     const float *w[4], *b[4], *out;
-    int splits, bblocks, oblocks;
+    int splits, oblocks;
 };
 
 // The end of a batch in one launch: every gradient is summed from its partial
@@ -328,7 +327,7 @@ __global__ void __launch_bounds__(256) update_kernel(const __grid_constant__ Par
             const int e = (blk % (kHid / 32)) * 32 + lane;
             src = ps.b[l] + e;
             stride = kHid;
-            n = ps.bblocks;
+            n = tctrain::kBiasParts;
             idx = param_offset(l) + kHid * layer_in(l) + e;
             o = k = -1;
         } else {
@@ -519,7 +518,7 @@ static bool mlp_forward_loss(int n, const float* T, bool keep_y, double* loss_ou
 
 // backward of n samples (a multiple of 128) after mlp_forward_loss: the gradients into M.gr, or, with `step`, one AdamW step from them.
 // Data gradients and the hidden layers' weight gradients on the tensor cores;
-// bias gradients in the former's epilogue, the output layer's on the CUDA cores.
+// bias gradients beside the latter, the output layer's on the CUDA cores.
 static bool mlp_backward(int n, const Adam* step)
 {
     cudaStream_t s = g.stream;
@@ -532,11 +531,11 @@ static bool mlp_backward(int n, const Adam* step)
     unsigned char *gcur = M.G0, *gnext = M.G1;
     Partials ps;
     for (int l = 3; l >= 0; l--) {
-        if (!cuda_ok(tctrain::backward_data(gin, l == 3 ? kDYld : kHid, M.cp.wn[l + 1], n, M.Z[l], gcur, M.bpart[l],
-                                            g.d_status, s),
+        if (!cuda_ok(tctrain::backward_data(gin, l == 3 ? kDYld : kHid, M.cp.wn[l + 1], n, M.Z[l], gcur, g.d_status,
+                                            s),
                      "dH") ||
             !cuda_ok(tctrain::backward_weights(gcur, l == 0 ? M.X : M.H[l - 1], layer_in(l), n, M.wpart[l], splits,
-                                               g.d_status, s),
+                                               M.bpart[l], g.d_status, s),
                      "dW"))
             return false;
         ps.w[l] = M.wpart[l];
@@ -545,8 +544,7 @@ static bool mlp_backward(int n, const Adam* step)
         std::swap(gcur, gnext);
     }
     ps.out = M.opart;
-    ps.splits = splits;
-    ps.bblocks = tctrain::layer_blocks(n);
+    ps.splits = tctrain::used_splits(n / 64, splits);
     ps.oblocks = oblocks;
     if (step)
         update_kernel<true><<<kUpdateBlocks, 256, 0, s>>>(ps, nullptr, M.p, M.m, M.v, *step, M.cp);

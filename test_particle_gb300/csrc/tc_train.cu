@@ -1,7 +1,7 @@
 // tc_train.cu -- the GEMMs of the learned field model's training on the
 // 5th-generation tensor cores: BF16 operands, FP32 accumulation in tensor
 // memory, and a fused epilogue per use (bias + SiLU of the forward pass, the
-// SiLU derivative and the bias gradients of the backward pass).
+// SiLU derivative of the backward pass).
 //
 // Everything the GEMMs exchange lies in global memory the way shared memory
 // wants it: a matrix of samples [M][C] as blocks of 128 samples x 64 columns
@@ -133,17 +133,13 @@ struct EpiHidden {
     {
         if (w.lane == 0) tc::bulk_wait_all();
     }
-    __device__ void tail(uint32_t) {}
 };
 
-// g = acc * silu'(Z), and the sums of its columns over the block's samples (the
-// bias gradient's partial sums).  The strips of Z are fetched two blocks ahead,
+// g = acc * silu'(Z).  The strips of Z are fetched two blocks ahead,
 // each as soon as the strip of G that replaced it has been read back out.
 struct EpiBackSilu {
     const unsigned char* Z;
     unsigned char* G;
-    float* bpart;  // [gridDim.x][256]
-    float sum[4];
     uint32_t got[2];  // uses of each strip's mbarrier so far; loads in flight
     bool pend[2];
     __device__ void fetch(const Warp& w, int t, int h)
@@ -156,7 +152,6 @@ struct EpiBackSilu {
     }
     __device__ void begin(const Warp& w, int t, int ntiles)
     {
-        for (int k = 0; k < 4; k++) sum[k] = 0.f;
         for (int h = 0; h < 2; h++) {
             got[h] = 0;
             pend[h] = false;
@@ -194,22 +189,6 @@ struct EpiBackSilu {
             tc::bulk_s2g(G + strip_offset(t, w, w.c64 + h), strip, 4096);
             tc::bulk_commit();
         }
-        // the sums of columns 2 lane, 2 lane + 1 of the strip's 32 rows
-        float s0 = 0.f, s1 = 0.f;
-#pragma unroll
-        for (int r = 0; r < 32; r++) {
-            uint32_t g2;
-            asm volatile("ld.shared.b32 %0, [%1];"
-                         : "=r"(g2)
-                         : "r"(piece(strip, r, w.lane >> 2) + 4u * (w.lane & 3))
-                         : "memory");
-            const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&g2));
-            s0 += f.x;
-            s1 += f.y;
-        }
-        sum[2 * h] += s0;
-        sum[2 * h + 1] += s1;
-        __syncwarp();
         if (tnext >= 0) {
             if (w.lane == 0) tc::bulk_wait_read();
             fetch(w, tnext, h);
@@ -223,29 +202,6 @@ struct EpiBackSilu {
             for (int h = 0; h < 2; h++)  // after a give-up: a load in flight (bounded)
                 if (pend[h]) tc::mbar_wait(w.bar + 8u * h, got[h] & 1u, kLimit);
         }
-        __syncwarp();
-#pragma unroll
-        for (int h = 0; h < 2; h++)
-            asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(w.stage + 256u * h + 8u * w.lane),
-                         "r"(__float_as_uint(sum[2 * h])), "r"(__float_as_uint(sum[2 * h + 1]))
-                         : "memory");
-    }
-    // after a block barrier: column c is element c % 128 of the four warps of its half
-    __device__ void tail(uint32_t stage)
-    {
-        const int c = threadIdx.x;
-        if (c >= 256) return;
-        float t = 0.f;
-#pragma unroll
-        for (int q = 0; q < 4; q++) {
-            uint32_t u;
-            asm volatile("ld.shared.b32 %0, [%1];"
-                         : "=r"(u)
-                         : "r"(stage + (uint32_t)((c >> 7) * 4 + q) * 8192u + 4u * (c & 127))
-                         : "memory");
-            t += __uint_as_float(u);
-        }
-        bpart[(size_t)blockIdx.x * 256 + c] = t;
     }
 };
 
@@ -263,7 +219,6 @@ struct EpiOut {
         return true;
     }
     __device__ void finish(const Warp&) {}
-    __device__ void tail(uint32_t) {}
 };
 
 // The same in a training batch of n samples, with the loss: r = y - (t - mean) /
@@ -299,7 +254,6 @@ struct EpiOutLoss {
         return true;
     }
     __device__ void finish(const Warp&) {}
-    __device__ void tail(uint32_t) {}
 };
 
 struct EpiStoreF32 {  // D[m][n] = acc (self-check)
@@ -317,7 +271,6 @@ struct EpiStoreF32 {  // D[m][n] = acc (self-check)
         return true;
     }
     __device__ void finish(const Warp&) {}
-    __device__ void tail(uint32_t) {}
 };
 
 // ---------------------------------------------------------------- a layer
@@ -475,7 +428,6 @@ __global__ void __launch_bounds__(ws_threads(N), 1)
         epi.finish(me);
     }
     __syncthreads();
-    epi.tail(stage0);
     if (warp == 1) {
         if (lane == 0) {  // every MMA this block issued has completed (bounded)
             tc::mma_commit(fin);
@@ -505,31 +457,85 @@ static cudaError_t launch_layer(const void* A, const void* B, int M, int K, cons
 // P[split][x][n][m] = sum over the split's samples k of G[k][128 x + m] X[k][n]
 // (m < 128, n < 64 xatoms <= 256): both operands are read MN-major from their
 // blocks, 64 samples a stage (half a block of every 64 columns, 8 KB each).
-// 15.2 us at 65,536 samples (64 + 32 MB; 19.0 from transposed copies).
+// 15.2 us at 65,536 samples (64 + 32 MB; 19.0 from transposed copies) without the sums below.
 // One output tile per CTA, the samples split over gridDim.y so that the CTAs
 // fill the SMs.  Warp 0 copies, warp 1 issues the MMAs, warps 2..5 write the
 // accumulator, 32 consecutive m (128 bytes) a store.
+// Those four warps are idle until then: in the first 128 CTAs they take the bias
+// gradients, the sums of G's columns, 16 columns and one of eight shares of the
+// samples each.  The order of their sums and the shares of the weight gradients
+// are those of one thread block per feature and of equal steps per split: a few
+// AdamW steps turn the last place of a gradient into 1e-5 of the loss, so the
+// order is kept although sums in the data gradient's epilogue would be cheaper
+// (a batch of 65,536: this kernel 23 us with and 15 without the sums).
 constexpr int kDwThreads = 192;
 constexpr uint32_t kHalf = kBlk / 2;
+
+// part[w][c] for the 16 columns from 16 (unit % 16) and w = unit / 16: the samples in
+// groups of eight, group t + 256 k to running sum t (its pairs of samples one after
+// the other), the 32 sums t = 32 w .. added as a tree.  Thread = (t, 4 columns), four
+// groups' rows in flight.
+constexpr int kBiasUnits = 128;
+__device__ __forceinline__ void bias_unit(const unsigned char* __restrict__ G, int ngroups, int unit,
+                                          float* __restrict__ part, float (*sums)[17])
+{
+    const int th = threadIdx.x - 64, q = th & 3, tl = th >> 2, c0 = (unit & 15) * 16, w = unit >> 4;
+    float s[4] = {0.f, 0.f, 0.f, 0.f};
+    const int piece = ((c0 & 63) >> 3) + (q >> 1);
+    const unsigned char* base = G + (size_t)(c0 >> 6) * kBlk + 8u * (q & 1);
+#pragma unroll 4
+    for (int i = 32 * w + tl; i < ngroups; i += 256) {
+        const unsigned char* src = base + (size_t)(i >> 4) * 4 * kBlk + (size_t)(i & 15) * 1024u;
+        uint2 v[8];
+#pragma unroll
+        for (int r = 0; r < 8; r++) v[r] = __ldg(reinterpret_cast<const uint2*>(src + r * 128 + ((piece ^ r) << 4)));
+#pragma unroll
+        for (int r = 0; r < 8; r += 2) {
+            const uint32_t a[2] = {v[r].x, v[r].y}, b[2] = {v[r + 1].x, v[r + 1].y};
+#pragma unroll
+            for (int j = 0; j < 2; j++) {
+                const float2 fa = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&a[j]));
+                const float2 fb = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&b[j]));
+                s[2 * j] += fa.x + fb.x;
+                s[2 * j + 1] += fa.y + fb.y;
+            }
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < 4; j++) sums[tl][4 * q + j] = s[j];
+    asm volatile("bar.sync 1, 128;" ::: "memory");
+    if (th < 16) {
+        float t[32];
+#pragma unroll
+        for (int k = 0; k < 32; k++) t[k] = sums[k][th];
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1)
+#pragma unroll
+            for (int k = 0; k < off; k++) t[k] += t[k + off];
+        part[w * 256 + c0 + th] = t[0];
+    }
+    asm volatile("bar.sync 1, 128;" ::: "memory");
+}
 __host__ __device__ inline int dw_ring(int xatoms)
 {
-    const int n = (int)((kSmem - 1024) / ((2 + xatoms) * kHalf));
+    const int n = (int)((kSmem - 1024 - 8192) / ((2 + xatoms) * kHalf));
     return n < kMaxRing ? n : kMaxRing;
 }
 
 __global__ void __launch_bounds__(kDwThreads, 1)
     weights_kernel(const unsigned char* __restrict__ G, int gatoms, const unsigned char* __restrict__ X, int xatoms,
-                   int nsteps, float* __restrict__ P, int* __restrict__ status)
+                   int nsteps, int splits, float* __restrict__ P, float* __restrict__ bpart, int* __restrict__ status)
 {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t bars[2 * kMaxRing + 1];
+    __shared__ float sums[32][17];
     __shared__ uint32_t tmem_slot;
     __shared__ int abort_flag;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int ring = dw_ring(xatoms);
     const uint32_t stage = (uint32_t)(2 + xatoms) * kHalf;
-    const int k0 = (int)((long long)nsteps * blockIdx.y / gridDim.y);
-    const int k1 = (int)((long long)nsteps * (blockIdx.y + 1) / gridDim.y);
+    const int chunk = (nsteps + splits - 1) / splits;
+    const int k0 = blockIdx.y * chunk, k1 = min(nsteps, k0 + chunk);
     const uint32_t raw = tc::smem_addr(smem_raw);
     const uint32_t base = raw + ((1024u - (raw & 1023u)) & 1023u);
     const uint32_t bar0 = tc::smem_addr(&bars[0]);
@@ -594,6 +600,9 @@ __global__ void __launch_bounds__(kDwThreads, 1)
             if (!tc::mbar_wait(fin, 0, kLimit)) abort_flag = 1;
         }
         __syncwarp();
+    } else if (bpart) {
+        for (int u = blockIdx.y * gridDim.x + blockIdx.x; u < kBiasUnits; u += gridDim.x * gridDim.y)
+            bias_unit(G, nsteps * 8, u, bpart, sums);
     }
     __syncthreads();
     tc::tc_fence_after();
@@ -614,14 +623,15 @@ __global__ void __launch_bounds__(kDwThreads, 1)
 }
 
 static cudaError_t launch_weights(const void* G, int mtiles, const void* X, int xatoms, int nsteps, float* P,
-                                  int splits, int* status, cudaStream_t s)
+                                  int splits, float* bpart, int* status, cudaStream_t s)
 {
     if (splits < 1 || splits > nsteps || xatoms < 1 || xatoms > 4) return cudaErrorInvalidValue;
-    cudaError_t e = cudaFuncSetAttribute(weights_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem);
+    const uint32_t smem = 1024 + (uint32_t)dw_ring(xatoms) * (2 + xatoms) * kHalf;
+    cudaError_t e = cudaFuncSetAttribute(weights_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    weights_kernel<<<dim3(mtiles, splits), kDwThreads, kSmem, s>>>(
-        static_cast<const unsigned char*>(G), 2 * mtiles, static_cast<const unsigned char*>(X), xatoms, nsteps, P,
-        status);
+    weights_kernel<<<dim3(mtiles, tctrain::used_splits(nsteps, splits)), kDwThreads, smem, s>>>(
+        static_cast<const unsigned char*>(G), 2 * mtiles, static_cast<const unsigned char*>(X), xatoms, nsteps,
+        splits, P, bpart, status);
     return cudaGetLastError();
 }
 
@@ -655,6 +665,13 @@ namespace tctrain {
 
 using namespace tct;
 
+// splits of equal whole steps: the last ones may be empty and are not launched
+int used_splits(int nsteps, int splits)
+{
+    const int chunk = (nsteps + splits - 1) / splits;
+    return (nsteps + chunk - 1) / chunk;
+}
+
 int layer_blocks(int M) { return std::min(M / 128, g.num_sms > 0 ? g.num_sms : 148); }
 
 cudaError_t forward_hidden(const void* X, int kin, const void* W, int M, const float* b, void* Z, void* H,
@@ -678,19 +695,18 @@ cudaError_t forward_loss(const void* H3, const void* W4, int M, const float* b, 
 }
 
 cudaError_t backward_data(const void* Gin, int kout, const void* WT, int M, const void* Zprev, void* G,
-                          float* bpart, int* status, cudaStream_t s)
+                          int* status, cudaStream_t s)
 {
     EpiBackSilu e{};
     e.Z = static_cast<const unsigned char*>(Zprev);
     e.G = static_cast<unsigned char*>(G);
-    e.bpart = bpart;
     return launch_layer<256>(Gin, WT, M, kout, e, status, s);
 }
 
-cudaError_t backward_weights(const void* G, const void* X, int kin, int nsamp, float* P, int splits, int* status,
-                             cudaStream_t s)
+cudaError_t backward_weights(const void* G, const void* X, int kin, int nsamp, float* P, int splits, float* bpart,
+                             int* status, cudaStream_t s)
 {
-    return launch_weights(G, mlp::kHid / 128, X, kin / 64, nsamp / 64, P, splits, status, s);
+    return launch_weights(G, mlp::kHid / 128, X, kin / 64, nsamp / 64, P, splits, bpart, status, s);
 }
 
 // the shapes of the layer GEMMs go through the kernel those use, the others
@@ -706,7 +722,7 @@ static cudaError_t gemm_f32(const __nv_bfloat16* A, const __nv_bfloat16* B, int 
     to_blocks_kernel<<<grid((size_t)N * K), 256, 0, s>>>(B, N, K, layer ? 1 : 2, layer ? K / 64 : npad / 64, wb);
     if (layer) return launch_layer<256>(wa, wb, M, K, EpiStoreF32{D}, status, s);
     float* P = reinterpret_cast<float*>(wb + 2 * (size_t)npad * kpad);
-    cudaError_t e = launch_weights(wa, M / 128, wb, npad / 64, K / 64, P, 1, status, s);
+    cudaError_t e = launch_weights(wa, M / 128, wb, npad / 64, K / 64, P, 1, nullptr, status, s);
     if (e != cudaSuccess) return e;
     from_split_kernel<<<grid((size_t)M * N), 256, 0, s>>>(P, M, N, npad, D);
     return cudaGetLastError();

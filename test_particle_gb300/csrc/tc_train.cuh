@@ -17,7 +17,7 @@ __host__ __device__ __forceinline__ size_t tile_offset(size_t m, int c, int atom
 
 // Weights are k-atoms of all rows: element (n, k) of [N][K] at sw128_offset(N, n, k).
 
-// Blocks of a layer kernel over M samples (the rows of backward_data's bpart).
+// Blocks of a layer kernel over M samples.
 int layer_blocks(int M);
 
 // Z, H = silu(X W^T + b) of a hidden layer: X [M][kin], W [256][kin]; Z, H [M][256].
@@ -42,14 +42,18 @@ cudaError_t forward_loss(const void* H3, const void* W4, int M, const float* b, 
                          cudaStream_t s);
 
 // G = (Gin WT^T) * silu'(Zprev): Gin [M][kout], WT [256][kout] (the layer's weights
-// transposed); G [M][256], its column sums over a block's samples in bpart [layer_blocks(M)][256].
+// transposed); G [M][256].
 cudaError_t backward_data(const void* Gin, int kout, const void* WT, int M, const void* Zprev, void* G,
-                          float* bpart, int* status, cudaStream_t s);
+                          int* status, cudaStream_t s);
 
 // The gradient G^T X [256][kin] over nsamp samples, G [nsamp][256], X [nsamp][kin],
-// as `splits` (at most nsamp / 64) partial sums: P[split][m / 128][k][m % 128] FP32.
+// as used_splits(nsamp / 64, splits) partial sums (splits at most nsamp / 64), each over
+// the next nsamp / 64 / splits, rounded up, steps of 64 samples: P[split][m / 128][k][m % 128].
+// G's column sums as kBiasParts partial sums in bpart [kBiasParts][256].
+constexpr int kBiasParts = 8;
+int used_splits(int nsteps, int splits);
 cudaError_t backward_weights(const void* G, const void* X, int kin, int nsamp, float* P, int splits,
-                             int* status, cudaStream_t s);
+                             float* bpart, int* status, cudaStream_t s);
 
 }  // namespace tctrain
 }  // namespace tp
