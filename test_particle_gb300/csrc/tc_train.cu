@@ -606,7 +606,7 @@ __global__ void __launch_bounds__(kDwThreads, 1)
     }
     __syncthreads();
     tc::tc_fence_after();
-    if (warp >= 2 && !*abort) {
+    if (warp >= 2 && k0 < k1 && !*abort) {
         const int q = warp & 3;
         float* dst = P + ((size_t)blockIdx.y * gridDim.x + blockIdx.x) * (64 * xatoms) * 128 + 32 * q + lane;
         for (int c = 0; c < 64 * xatoms; c += 32) {
@@ -629,7 +629,11 @@ static cudaError_t launch_weights(const void* G, int mtiles, const void* X, int 
     const uint32_t smem = 1024 + (uint32_t)dw_ring(xatoms) * (2 + xatoms) * kHalf;
     cudaError_t e = cudaFuncSetAttribute(weights_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    weights_kernel<<<dim3(mtiles, tctrain::used_splits(nsteps, splits)), kDwThreads, smem, s>>>(
+    // with few splits, CTAs without samples of their own for the column sums (a
+    // training in batches of some 2,000 samples 0.79 -> 0.60 ms)
+    const int used = tctrain::used_splits(nsteps, splits);
+    const int rows = bpart ? std::max(used, (kBiasUnits + mtiles - 1) / mtiles) : used;
+    weights_kernel<<<dim3(mtiles, rows), kDwThreads, smem, s>>>(
         static_cast<const unsigned char*>(G), 2 * mtiles, static_cast<const unsigned char*>(X), xatoms, nsteps,
         splits, P, bpart, status);
     return cudaGetLastError();
