@@ -286,7 +286,7 @@ struct Partials {
 // A block takes 32 x 8 of a hidden layer's weights (thread = one, 128-byte reads
 // of every split, turned through shared memory for the row-major parameters), 32
 // biases, or 32 of the output layer's parameters (eight threads each).  17.8
-// us for 76 splits (68 MB read); a kernel per layer and purpose (four sums of
+// us for 74 splits (66 MB read); a kernel per layer and purpose (four sums of
 // splits, four of biases, AdamW, six of copies) took 137 us.
 constexpr int kPatches0 = (kHid / 32) * (kIn / 8), kPatches = (kHid / 32) * (kHid / 8);
 constexpr int kBiasBlocks = 4 * kHid / 32, kOutBlocks = (kOutGrad + 31) / 32;

@@ -15,7 +15,7 @@
 // activations and gradients exists, and the epilogues write 4 KB at a time.
 // With row-major activations, 16-byte cp.async and a transposed copy of each
 // for the weight gradients, a layer of 65,536 samples took 33 us forward and
-// 33 us backward; now 20.6 and 22.1 (96 MB each, 4.5 TB/s).
+// 33 us backward; now 20.4 and 21.2 (96 MB each, 4.5 TB/s).
 //
 // Every wait is bounded; one that runs out sets the block's abort flag, every
 // other wait then gives up, the block waits (bounded) for its copies and MMAs
