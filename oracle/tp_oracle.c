@@ -798,7 +798,7 @@ int or_track_fixed(const or_field *f, const or_spectrum *s, int nptl, double dt,
             int ntp = (int)floor(1 / (double)einterval);
             int tstep = 1;
             double sg[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-            if (esc_pre) my_rem[1] -= 1;
+            if (esc_pre && nsdc > 1) my_rem[1] -= 1;
             for (int j = 1; j <= estep; j++) {
                 sg[0] = 0.0; sg[4] = 0.0; sg[5] = 0.0; /* drr, dpp, duu reset (:334-336) */
                 if (esc_pre == 0 || f->bc_flag == 0) {

@@ -262,7 +262,7 @@ __global__ void __launch_bounds__(kBlock, track_min_blocks(SYS)) track_kernel(De
 #pragma unroll
             for (int c = 0; c < 8; c++) sg[c] = b.sg_carry[(size_t)i * kSegCarry + c];
         }
-        if (active && esc_pre && !q.resumed) atomicSub(&b.remain[1], 1);
+        if (active && esc_pre && !q.resumed && q.nsdc > 1) atomicSub(&b.remain[1], 1);
         double* slot_base = b.dpart + (size_t)blockIdx.x * q.nsdc * 8;
         int npts = 1;
         long toff = 0;

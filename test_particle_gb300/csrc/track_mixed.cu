@@ -164,7 +164,7 @@ __global__ void __launch_bounds__(kBlock, SYS == TP_SYS_PIC ? TP_MIXED_PIC_MINBL
         int esc_pre = esc ? 1 : 0;
         int esc_after = esc_pre;
         int ntp = q.ntp0, tstep = 1 + q.row0;
-        if (active && esc_pre && !q.resumed) atomicSub(&b.remain[1], 1);
+        if (active && esc_pre && !q.resumed && q.nsdc > 1) atomicSub(&b.remain[1], 1);
         double* slot_base = b.dpart + (size_t)blockIdx.x * q.nsdc * 8;
         int done = 0;
         if (active && q.resumed && b.sg_carry) done = (int)b.sg_carry[(size_t)i * kSegCarry + 15];
@@ -336,7 +336,7 @@ __global__ void __launch_bounds__(kBlock, 4) track_modes_kernel(MixField f, Trac
             }
             esc_pre[r] = esc;
             esc_after[r] = esc;
-            if (active[r] && esc && !q.resumed) atomicSub(&b.remain[1], 1);
+            if (active[r] && esc && !q.resumed && q.nsdc > 1) atomicSub(&b.remain[1], 1);
             done[r] = 0;
             if (active[r] && q.resumed && b.sg_carry) done[r] = (int)b.sg_carry[(size_t)i * kSegCarry + 15];
         }

@@ -223,7 +223,7 @@ __global__ void __launch_bounds__(128) track_small_kernel(DevField f, TrackBufs 
     bool esc_pre = group_any(out), esc_after = esc_pre;
     int ntp = q.ntp0, tstep = 1;
     double sg[8] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-    if (active && lead && esc_pre) atomicSub(&b.remain[1], 1);
+    if (active && lead && esc_pre && q.nsdc > 1) atomicSub(&b.remain[1], 1);
     double* slot_base = b.dpart + (size_t)blockIdx.x * q.nsdc * 8;
     // countdowns to the next diagnostic steps (j % einterval, j % 100)
     int to_frame = (q.einterval - q.sstep % q.einterval) % q.einterval;

@@ -469,7 +469,7 @@ __global__ void __launch_bounds__(kThreads, 1) track_surrogate_kernel(
         int esc_after = esc_pre;
         int ntp = q.ntp0, tstep = 1;
         double sg[8] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-        if (active && esc_pre) atomicSub(&b.remain[1], 1);
+        if (active && esc_pre && q.nsdc > 1) atomicSub(&b.remain[1], 1);
         double* slot_base = b.dpart + (size_t)blockIdx.x * q.nsdc * 8;
         int done = 0;
         int to_frame = q.einterval - q.sstep % q.einterval;
