@@ -235,7 +235,8 @@ __global__ void __launch_bounds__(128) track_small_kernel(DevField f, TrackBufs 
         const bool moves = !esc_pre || f.bc_flag == 0;
         sg[0] = 0.0; sg[4] = 0.0; sg[5] = 0.0;  // src/tracking.c:334-336
         double xn = x, un = u, tn = t, xsn = xs;
-        small_wirz<SYS>(f, c, xn, un, tn, q.dt, sh, active ? b.status : nullptr);
+        // (one that no longer moves reports nothing)
+        small_wirz<SYS>(f, c, xn, un, tn, q.dt, sh, active && moves ? b.status : nullptr);
         const bool left = small_bc(f, c, xn, xsn);
         const bool any = group_any(left);
         if (moves) {
