@@ -656,6 +656,10 @@ extern "C" int tp_get_emf_batch(int n, const double* xyzt, double* emf6)
     DevField f;
     if (!build_field(system_type, f)) return -1;
     if (n <= 0) return 0;
+    if (!xyzt || !emf6) {
+        set_error(6, "tp_get_emf_batch: null buffer");
+        return -1;
+    }
     if (in_place(xyzt, 8) && in_place(emf6, 8)) {
         if (!cuda_ok(fp64::launch_emf_batch(f, n, xyzt, emf6, g.d_status, g.stream), "emf")) return -1;
         return cuda_ok(cudaStreamSynchronize(g.stream), "emf sync") ? 0 : -1;

@@ -174,6 +174,10 @@ extern "C" int tp_get_emf_mixed_batch(int n, const double* xyz, float* emf6)
     mixed::MixField mf;
     if (!build_mixfield(system_type, mf, nullptr)) return -1;
     if (n <= 0) return 0;
+    if (!xyz || !emf6) {
+        set_error(6, "tp_get_emf_mixed_batch: null buffer");
+        return -1;
+    }
     if (in_place(xyz, 8) && in_place(emf6, 4)) {
         if (!cuda_ok(mixed::launch_emf_batch(mf, n, xyz, emf6, g.stream), "emf mixed")) return -1;
         return cuda_ok(cudaStreamSynchronize(g.stream), "emf mixed sync") ? 0 : -1;

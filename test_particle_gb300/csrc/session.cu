@@ -192,6 +192,10 @@ bool Session::reserve(int n)
 bool Session::load(const particles* ptl_init, const particles* ptl, int n_)
 {
     if (!reserve(n_)) return false;
+    if (n_ > 0 && (!ptl_init || !ptl)) {
+        set_error(6, "particle records: null buffer");
+        return false;
+    }
     n = n_;
     cudaStream_t s = g.stream;
     double *S = (double*)soa.ptr, *S0 = (double*)soa0.ptr;
@@ -600,7 +604,8 @@ extern "C" int tp_track_host_to(int precision, int nptl, double dt, int nt_out, 
     rs.nbins = nbins;
     if (!s.load(ptl_init, ptl, nptl)) return -1;
     auto meanwhile = [&] {
-        if (nptl > 0 && ptl_out != ptl && ptl_out != ptl_init) touch_pages(ptl_out, sizeof(particles) * (size_t)nptl);
+        if (nptl > 0 && ptl_out && ptl_out != ptl && ptl_out != ptl_init)
+            touch_pages(ptl_out, sizeof(particles) * (size_t)nptl);
         if (nptl > 0 && nsteps_ptl) touch_pages(nsteps_ptl, sizeof(int) * (size_t)nptl);
     };
     if (!s.run(rs, info, meanwhile)) {

@@ -91,7 +91,10 @@ bool compute_thresholds(int nbins, double lmin, double lde, std::vector<double>&
 // A host buffer that kernels may read or write in place: the device walks the
 // host's page tables, and elements are aligned.  Work on it has to be waited
 // for before the caller gets its buffer back.
-inline bool in_place(const void* host, size_t align) { return g.direct && ((uintptr_t)host & (align - 1)) == 0; }
+inline bool in_place(const void* host, size_t align)
+{
+    return g.direct && host && ((uintptr_t)host & (align - 1)) == 0;
+}
 // particles records to columns (both when soa2 is given) and back
 void aos_to_soa(const double* aos, int n, double* d_soa, double* d_soa2, long stride, cudaStream_t s);
 void soa_to_aos(const double* d_soa, int n, long stride, double* aos, cudaStream_t s);

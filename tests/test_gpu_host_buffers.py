@@ -1,0 +1,51 @@
+"""Host buffers that kernels read and write in place or through staged copies
+(field batches, particle records): what is refused, and that every way gives
+the same bytes."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+tp = pytest.importorskip("test_particle_gb300")
+import test_particle_gb300.workloads as wl  # noqa: E402
+
+DT = 0.02
+
+
+def _setup(steps=20):
+    dom = tp.Domain()
+    dom.xmax = dom.ymax = dom.zmax = 1.0
+    dom.tmax = (steps + 0.5) * DT
+    tp.configure(system_type=tp.SYS_FORCEFREE, dom=dom, abc=(1.0, 0.7, 0.4), lambda0=2 * np.pi)
+    tp.set_spectrum(50, 1e-3, 1e2)
+
+
+def _track(prec, n, p0, p, out, nst=None, steps=20):
+    esp, ese, ds, rem = np.zeros(50), np.zeros(50), np.zeros(8), np.zeros(1, np.int32)
+    return tp.lib().tp_track_host_to(C.c_int(prec), C.c_int(n), C.c_double(DT), C.c_int(1), C.c_int(50), tp._ptr(p0),
+                                     tp._ptr(p), tp._ptr(out), tp._ptr(nst), tp._ptr(esp), tp._ptr(ese), tp._ptr(ds),
+                                     tp._ptr(rem), None)
+
+
+def test_null_buffers_are_refused():
+    """Refused on the host, with a message and no error left for the next call."""
+    _setup()
+    L = tp.lib()
+    x, e, f = np.zeros((4, 4)), np.zeros((4, 6)), np.zeros((4, 6), np.float32)
+    p = wl.shell_particles(4, 0.5, (0, 0, 0), (1, 1, 1), 1)
+    s = tp.Session(4)
+    h = C.c_void_p(s.h)
+    for call in (lambda: L.tp_get_emf_batch(4, None, tp._ptr(e)), lambda: L.tp_get_emf_batch(4, tp._ptr(x), None),
+                 lambda: L.tp_get_emf_mixed_batch(4, None, tp._ptr(f)),
+                 lambda: L.tp_get_emf_mixed_batch(4, tp._ptr(x), None),
+                 lambda: L.tp_session_load(h, None, tp._ptr(p)), lambda: L.tp_session_load(h, tp._ptr(p), None),
+                 lambda: L.tp_session_load(h, None, None), lambda: _track(tp.PREC_FP64, 4, None, None, p),
+                 lambda: _track(tp.PREC_FP64, 4, p, None, p), lambda: _track(tp.PREC_FP64, 4, None, p, p)):
+        assert call() == -1
+        assert b"null" in L.tp_last_error()
+        L.tp_clear_status()
+    assert np.isfinite(tp.get_emf(x)).all()
+    s.load(p)
+    assert _track(tp.PREC_FP64, 4, p, p, None) == 0  # no particles wanted back
+    assert tp.device_status() == 0
