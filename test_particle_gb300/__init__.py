@@ -238,7 +238,10 @@ def track(ptl_init, dt, nt_out, nbins, precision=PREC_FP64, ptl=None):
     p0 = np.ascontiguousarray(ptl_init, dtype=PARTICLE_DTYPE)
     start = p0 if ptl is None else np.ascontiguousarray(ptl, dtype=PARTICLE_DTYPE)
     n = len(p0)
-    p = np.empty(n, dtype=PARTICLE_DTYPE)
+    if len(start) < n:
+        raise ValueError("track: %d current particles for %d initial ones" % (len(start), n))
+    # (records behind the n tracked ones are returned as they came)
+    p = np.empty(n, dtype=PARTICLE_DTYPE) if start.shape == (n,) else start.copy()
     estep = int(Domain.in_dll(L, "simul_domain").tmax / dt)
     nsdc = estep // 100 + 1
     esp = np.zeros(nt_out * nbins)
@@ -349,6 +352,8 @@ class Session:
     def load(self, ptl_init, ptl=None):
         p0 = np.ascontiguousarray(ptl_init, dtype=PARTICLE_DTYPE)
         p = p0 if ptl is None else np.ascontiguousarray(ptl, dtype=PARTICLE_DTYPE)
+        if p0.size < self.n or p.size < self.n:
+            raise ValueError("session load: fewer records than the session's %d particles" % self.n)
         check(self.L.tp_session_load(C.c_void_p(self.h), _ptr(p0), _ptr(p)), "session load")
 
     def track(self, dt, nt_out, nbins, precision=PREC_FP64):

@@ -49,3 +49,21 @@ def test_null_buffers_are_refused():
     s.load(p)
     assert _track(tp.PREC_FP64, 4, p, p, None) == 0  # no particles wanted back
     assert tp.device_status() == 0
+
+
+def test_record_arrays_of_other_lengths():
+    """Fewer records than particles are refused (the device would read past the
+    array); more are returned behind the tracked ones as they came."""
+    _setup()
+    p = wl.shell_particles(8, 0.5, (0, 0, 0), (1, 1, 1), 1)
+    with pytest.raises(ValueError):
+        tp.track(p, DT, 1, 50, ptl=p[:7])
+    s = tp.Session(8)
+    with pytest.raises(ValueError):
+        s.load(p[:7])
+    with pytest.raises(ValueError):
+        s.load(p, p[:7])
+    few = tp.track(p[:5], DT, 1, 50, ptl=p)
+    assert few["ptl"].shape == (8,) and len(few["nsteps"]) == 5
+    assert few["ptl"][5:].tobytes() == p[5:].tobytes()
+    assert few["ptl"][:5].tobytes() == tp.track(p[:5], DT, 1, 50)["ptl"].tobytes()
