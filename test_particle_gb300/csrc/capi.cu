@@ -660,17 +660,19 @@ extern "C" int tp_get_emf_batch(int n, const double* xyzt, double* emf6)
         set_error(6, "tp_get_emf_batch: null buffer");
         return -1;
     }
-    if (in_place(xyzt, 8) && in_place(emf6, 8)) {
-        if (!cuda_ok(fp64::launch_emf_batch(f, n, xyzt, emf6, g.d_status, g.stream), "emf")) return -1;
-        return cuda_ok(cudaStreamSynchronize(g.stream), "emf sync") ? 0 : -1;
+    const size_t nin = sizeof(double) * 4 * (size_t)n, nout = sizeof(double) * 6 * (size_t)n;
+    const double* in = xyzt;
+    double* out = emf6;
+    if (!in_place(xyzt, 8)) {
+        double* d = (double*)g.s_batch_a.get(nin);
+        if (!d || !cuda_ok(cudaMemcpyAsync(d, xyzt, nin, cudaMemcpyHostToDevice, g.stream), "emf points")) return -1;
+        in = d;
     }
-    double* d_in = (double*)g.s_batch_a.get(sizeof(double) * 4 * (size_t)n);
-    double* d_out = (double*)g.s_batch_b.get(sizeof(double) * 6 * (size_t)n);
-    if (!d_in || !d_out) return -1;
-    cudaMemcpyAsync(d_in, xyzt, sizeof(double) * 4 * n, cudaMemcpyHostToDevice, g.stream);
-    if (!cuda_ok(fp64::launch_emf_batch(f, n, d_in, d_out, g.d_status, g.stream), "emf")) return -1;
-    cudaMemcpyAsync(emf6, d_out, sizeof(double) * 6 * n, cudaMemcpyDeviceToHost, g.stream);
-    return cuda_ok(cudaStreamSynchronize(g.stream), "emf sync") ? 0 : -1;
+    if (!result_in_place(emf6, nout, 8, xyzt, nin) && !(out = (double*)g.s_batch_b.get(nout))) return -1;
+    bool ok = cuda_ok(fp64::launch_emf_batch(f, n, in, out, g.d_status, g.stream), "emf");
+    if (ok && out != emf6)
+        ok = cuda_ok(cudaMemcpyAsync(emf6, out, nout, cudaMemcpyDeviceToHost, g.stream), "emf fields");
+    return cuda_ok(cudaStreamSynchronize(g.stream), "emf sync") && ok ? 0 : -1;
 }
 
 extern "C" int tp_wirz_steps(int n, particles* ptl, double dt, int nsteps, int* iescape)

@@ -178,15 +178,17 @@ extern "C" int tp_get_emf_mixed_batch(int n, const double* xyz, float* emf6)
         set_error(6, "tp_get_emf_mixed_batch: null buffer");
         return -1;
     }
-    if (in_place(xyz, 8) && in_place(emf6, 4)) {
-        if (!cuda_ok(mixed::launch_emf_batch(mf, n, xyz, emf6, g.stream), "emf mixed")) return -1;
-        return cuda_ok(cudaStreamSynchronize(g.stream), "emf mixed sync") ? 0 : -1;
+    const size_t nin = sizeof(double) * 3 * (size_t)n, nout = sizeof(float) * 6 * (size_t)n;
+    const double* in = xyz;
+    float* out = emf6;
+    if (!in_place(xyz, 8)) {
+        double* d = (double*)g.s_batch_a.get(nin);
+        if (!d || !cuda_ok(cudaMemcpyAsync(d, xyz, nin, cudaMemcpyHostToDevice, g.stream), "emf points")) return -1;
+        in = d;
     }
-    double* d_in = (double*)g.s_batch_a.get(sizeof(double) * 3 * (size_t)n);
-    float* d_out = (float*)g.s_batch_b.get(sizeof(float) * 6 * (size_t)n);
-    if (!d_in || !d_out) return -1;
-    cudaMemcpyAsync(d_in, xyz, sizeof(double) * 3 * (size_t)n, cudaMemcpyHostToDevice, g.stream);
-    if (!cuda_ok(mixed::launch_emf_batch(mf, n, d_in, d_out, g.stream), "emf mixed")) return -1;
-    cudaMemcpyAsync(emf6, d_out, sizeof(float) * 6 * (size_t)n, cudaMemcpyDeviceToHost, g.stream);
-    return cuda_ok(cudaStreamSynchronize(g.stream), "emf mixed sync") ? 0 : -1;
+    if (!result_in_place(emf6, nout, 4, xyz, nin) && !(out = (float*)g.s_batch_b.get(nout))) return -1;
+    bool ok = cuda_ok(mixed::launch_emf_batch(mf, n, in, out, g.stream), "emf mixed");
+    if (ok && out != emf6)
+        ok = cuda_ok(cudaMemcpyAsync(emf6, out, nout, cudaMemcpyDeviceToHost, g.stream), "emf fields");
+    return cuda_ok(cudaStreamSynchronize(g.stream), "emf mixed sync") && ok ? 0 : -1;
 }

@@ -95,6 +95,13 @@ inline bool in_place(const void* host, size_t align)
 {
     return g.direct && host && ((uintptr_t)host & (align - 1)) == 0;
 }
+// The same for a result that is computed from `input`: where the two overlap it
+// goes through a copy, which follows the last read of the input.
+inline bool result_in_place(const void* host, size_t bytes, size_t align, const void* input, size_t input_bytes)
+{
+    const uintptr_t a = (uintptr_t)host, b = (uintptr_t)input;
+    return in_place(host, align) && (a + bytes <= b || b + input_bytes <= a);
+}
 // particles records to columns (both when soa2 is given) and back
 void aos_to_soa(const double* aos, int n, double* d_soa, double* d_soa2, long stride, cudaStream_t s);
 void soa_to_aos(const double* d_soa, int n, long stride, double* aos, cudaStream_t s);

@@ -67,3 +67,24 @@ def test_record_arrays_of_other_lengths():
     assert few["ptl"].shape == (8,) and len(few["nsteps"]) == 5
     assert few["ptl"][5:].tobytes() == p[5:].tobytes()
     assert few["ptl"][:5].tobytes() == tp.track(p[:5], DT, 1, 50)["ptl"].tobytes()
+
+
+@pytest.mark.parametrize("n", [1, 129, 20000])
+@pytest.mark.parametrize("shift", [0, 3])
+def test_fields_written_over_their_points(n, shift):
+    """A result that overlaps the points is what one in its own buffer is."""
+    _setup()
+    rng = np.random.default_rng(n)
+    pts = rng.random((n, 4))
+    want = tp.get_emf(pts)
+    for at, to in ((0, shift), (shift, 0)):
+        buf = np.zeros(6 * n + 8)
+        buf[at:at + 4 * n] = pts.ravel()
+        tp.check(tp.lib().tp_get_emf_batch(C.c_int(n), tp._ptr(buf[at:]), tp._ptr(buf[to:])))
+        assert buf[to:to + 6 * n].tobytes() == want.tobytes()
+    want = tp.get_emf_mixed(pts[:, :3])
+    buf = np.zeros(3 * n + 8)
+    buf[:3 * n] = pts[:, :3].ravel()
+    out = buf.view(np.float32)[shift:shift + 6 * n]
+    tp.check(tp.lib().tp_get_emf_mixed_batch(C.c_int(n), tp._ptr(buf), tp._ptr(out)))
+    assert out.tobytes() == want.tobytes()
