@@ -209,15 +209,13 @@ bool Session::load(const particles* ptl_init, const particles* ptl, int n_)
         aos_to_soa(src, n, to, also, cap, s);
         return true;
     };
-    if (n > 0) {
-        if (ptl == ptl_init) {
-            if (!records(ptl, S, S0)) return false;
-        } else if (!records(ptl_init, S0, nullptr) || !records(ptl, S, nullptr)) {
-            return false;
-        }
-    }
-    loaded = true;
-    return cuda_ok(cudaGetLastError(), "load");
+    bool ok = true;
+    if (n > 0)
+        ok = ptl == ptl_init ? records(ptl, S, S0) : records(ptl_init, S0, nullptr) && records(ptl, S, nullptr);
+    ok = ok && cuda_ok(cudaGetLastError(), "load");
+    if (ok) loaded = true;
+    else cudaStreamSynchronize(s);  // the records are the caller's again: nothing may read them any more
+    return ok;
 }
 
 bool Session::run(const RunSpec& rs, tp_run_info* info, const std::function<void()>& meanwhile)
