@@ -348,7 +348,8 @@ int tp_track_host(int precision, int nptl, double dt, int nt_out, int nbins,
                   double *espect, double *espect_escape, double *dsum, int *remain,
                   tp_run_info *info);
 /* The same with the final particles in a buffer of their own (ptl is read
- * only; ptl_out may be fresh memory: its pages are mapped during the run). */
+ * only; ptl_out may be fresh memory: its pages are mapped during the run, with
+ * their contents kept, so that a run that fails leaves every output as it was). */
 int tp_track_host_to(int precision, int nptl, double dt, int nt_out, int nbins,
                      const particles *ptl_init, const particles *ptl, particles *ptl_out, int *nsteps_ptl,
                      double *espect, double *espect_escape, double *dsum, int *remain,

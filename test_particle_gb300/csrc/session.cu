@@ -581,11 +581,14 @@ extern "C" int tp_session_fetch(tp_session* s, particles* ptl, int* nsteps_ptl, 
 
 // Maps the pages of a buffer that is about to be written: a fresh allocation's
 // pages are zeroed one by one at their first touch, 10 GB/s on one core, which
-// the tracking kernel's time hides.
+// the tracking kernel's time hides.  The contents stay: a run that fails leaves
+// its caller's arrays as they were.
 static void touch_pages(void* p, size_t bytes)
 {
     const size_t page = (size_t)sysconf(_SC_PAGESIZE);
-    for (size_t i = 0; i < bytes; i += page) ((volatile char*)p)[i] = 0;
+    volatile char* c = (volatile char*)p;
+    for (size_t i = 0; i < bytes; i += page) c[i] = c[i];
+    if (bytes > 0) c[bytes - 1] = c[bytes - 1];  // (the first byte need not start a page)
 }
 
 extern "C" int tp_track_host_to(int precision, int nptl, double dt, int nt_out, int nbins,

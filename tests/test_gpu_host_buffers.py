@@ -88,3 +88,26 @@ def test_fields_written_over_their_points(n, shift):
     out = buf.view(np.float32)[shift:shift + 6 * n]
     tp.check(tp.lib().tp_get_emf_mixed_batch(C.c_int(n), tp._ptr(buf), tp._ptr(out)))
     assert out.tobytes() == want.tobytes()
+
+
+def test_failed_run_leaves_the_outputs():
+    """A refused run leaves the records and step counts as they were, and an
+    output that lies over part of the inputs is written after they are read
+    (its pages are mapped, but not changed, while the run is going)."""
+    _setup()
+    n = 5000
+    p = wl.shell_particles(n, 0.5, (0, 0, 0), (1, 1, 1), 1)
+    out = np.frombuffer(np.random.default_rng(1).bytes(88 * n), dtype=tp.PARTICLE_DTYPE).copy()
+    nst = np.arange(n, dtype=np.int32) + 1000
+    keep = out.copy(), nst.copy()
+    assert _track(7, n, p, p, out, nst) == -1  # no such precision
+    tp.lib().tp_clear_status()
+    assert out.tobytes() == keep[0].tobytes() and nst.tobytes() == keep[1].tobytes()
+    # the same outputs over part of the inputs: read before they are written
+    both = np.zeros(2 * n, dtype=tp.PARTICLE_DTYPE)
+    both[:n] = p
+    want = np.zeros(n, dtype=tp.PARTICLE_DTYPE)
+    assert _track(tp.PREC_MIXED, n, p, p, want, nst) == 0
+    shifted = both[n // 2:n // 2 + n]
+    assert _track(tp.PREC_MIXED, n, both, both, shifted, nst) == 0
+    assert shifted.tobytes() == want.tobytes()
