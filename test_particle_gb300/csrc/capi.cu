@@ -56,6 +56,7 @@ void set_error(int code, const char* fmt, ...)
 bool cuda_ok(cudaError_t e, const char* what)
 {
     if (e == cudaSuccess) return true;
+    cudaGetLastError();  // reported here: not to be taken for the next launch's
     set_error(2, "%s: %s", what, cudaGetErrorString(e));
     return false;
 }
@@ -473,6 +474,8 @@ void* Scratch::get(size_t b)
     ptr = nullptr;
     cap = 0;
     if (cudaMalloc(&ptr, b) != cudaSuccess) {
+        cudaGetLastError();
+        ptr = nullptr;
         set_error(7, "device allocation of %zu bytes failed", b);
         return nullptr;
     }

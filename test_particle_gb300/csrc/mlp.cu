@@ -371,7 +371,7 @@ __global__ void __launch_bounds__(256) update_kernel(const __grid_constant__ Par
 using namespace mlp;
 
 struct MlpState {
-    bool ready = false;
+    bool ready = false, have_params = false;
     int freq_h[kFeat * 3];
     // parameters (FP32 master), gradients, Adam moments: one flat buffer each
     size_t nparam = 0;
@@ -401,9 +401,17 @@ static MlpState M;
 // most blocks of a kernel whose partial sums are kept by block
 static int max_blocks() { return 2 * tctrain::layer_blocks(INT_MAX / 128 * 128); }
 
+template <class T>
+static void drop(T*& p)
+{
+    if (p) cudaFree(p);
+    p = nullptr;
+}
+
+// Everything of the model itself, or nothing of it.
 static bool mlp_alloc_params()
 {
-    if (M.p) return true;
+    if (M.have_params) return true;
     size_t off = 0;
     for (int l = 0; l < kLayers; l++) {
         M.woff[l] = off;
@@ -412,41 +420,58 @@ static bool mlp_alloc_params()
         off += layer_out(l);
     }
     M.nparam = off;  // = kParams
-    size_t b = sizeof(float) * off;
-    if (!cuda_ok(cudaMalloc(&M.p, b), "mlp params") || !cuda_ok(cudaMalloc(&M.gr, b), "mlp grads") ||
-        !cuda_ok(cudaMalloc(&M.m, b), "mlp m") || !cuda_ok(cudaMalloc(&M.v, b), "mlp v"))
-        return false;
+    const size_t b = sizeof(float) * off;
+    bool ok = cuda_ok(cudaMalloc(&M.p, b), "mlp params") && cuda_ok(cudaMalloc(&M.gr, b), "mlp grads") &&
+              cuda_ok(cudaMalloc(&M.m, b), "mlp m") && cuda_ok(cudaMalloc(&M.v, b), "mlp v");
     // the rows and columns that pad the output layer's copies stay zero
     auto zeroed = [](unsigned char*& d, size_t n, const char* what) {
         return cuda_ok(cudaMalloc(&d, n), what) && cuda_ok(cudaMemsetAsync(d, 0, n, g.stream), what);
     };
-    for (int l = 0; l < kLayers; l++) {
-        if (!zeroed(M.cp.wk[l], sizeof(__nv_bfloat16) * layer_out_pad(l) * layer_in(l), "mlp wk") ||
-            (l > 0 && !zeroed(M.cp.wn[l],
-                              sizeof(__nv_bfloat16) * (size_t)layer_in(l) * (l == kLayers - 1 ? kDYld : kHid), "mlp wn")))
-            return false;
+    for (int l = 0; l < kLayers && ok; l++) {
+        ok = zeroed(M.cp.wk[l], sizeof(__nv_bfloat16) * layer_out_pad(l) * layer_in(l), "mlp wk") &&
+             (l == 0 || zeroed(M.cp.wn[l],
+                               sizeof(__nv_bfloat16) * (size_t)layer_in(l) * (l == kLayers - 1 ? kDYld : kHid),
+                               "mlp wn"));
         if (l == kLayers - 1) continue;
-        if (!cuda_ok(cudaMalloc(&M.wpart[l], sizeof(float) * (size_t)kWgradSplits * kHid * layer_in(l)),
-                     "mlp weight partial") ||
-            !cuda_ok(cudaMalloc(&M.bpart[l], sizeof(float) * (size_t)max_blocks() * kHid), "mlp bias partial"))
-            return false;
+        ok = ok &&
+             cuda_ok(cudaMalloc(&M.wpart[l], sizeof(float) * (size_t)kWgradSplits * kHid * layer_in(l)),
+                     "mlp weight partial") &&
+             cuda_ok(cudaMalloc(&M.bpart[l], sizeof(float) * (size_t)max_blocks() * kHid), "mlp bias partial");
     }
-    return zeroed(M.cp.pack, kPackBytes, "mlp wpack") &&
-           cuda_ok(cudaMalloc(&M.opart, sizeof(float) * (size_t)max_blocks() * kOutGrad), "mlp output partial") &&
-           cuda_ok(cudaMalloc(&M.freq, sizeof(int) * 3 * kFeat), "mlp freq") &&
-           cuda_ok(cudaMalloc(&M.d_mean, sizeof(float) * kOut), "mlp mean") &&
-           cuda_ok(cudaMalloc(&M.d_istd, sizeof(float) * kOut), "mlp std") &&
-           cuda_ok(cudaMalloc(&M.loss, sizeof(double)), "mlp loss");
+    ok = ok && zeroed(M.cp.pack, kPackBytes, "mlp wpack") &&
+         cuda_ok(cudaMalloc(&M.opart, sizeof(float) * (size_t)max_blocks() * kOutGrad), "mlp output partial") &&
+         cuda_ok(cudaMalloc(&M.freq, sizeof(int) * 3 * kFeat), "mlp freq") &&
+         cuda_ok(cudaMalloc(&M.d_mean, sizeof(float) * kOut), "mlp mean") &&
+         cuda_ok(cudaMalloc(&M.d_istd, sizeof(float) * kOut), "mlp std") &&
+         cuda_ok(cudaMalloc(&M.loss, sizeof(double)), "mlp loss");
+    if (!ok) {
+        drop(M.p); drop(M.gr); drop(M.m); drop(M.v);
+        for (int l = 0; l < kLayers; l++) { drop(M.cp.wk[l]); drop(M.cp.wn[l]); }
+        for (int l = 0; l < 4; l++) { drop(M.wpart[l]); drop(M.bpart[l]); }
+        drop(M.cp.pack); drop(M.opart); drop(M.freq); drop(M.d_mean); drop(M.d_istd); drop(M.loss);
+    }
+    M.have_params = ok;
+    return ok;
 }
 
-// workspaces for batches of up to n samples (rounded up to a whole 128-row tile)
+static void mlp_drop_batch()
+{
+    M.cap = 0;
+    drop(M.X); drop(M.G0); drop(M.G1); drop(M.dY); drop(M.Y); drop(M.dYf);
+    for (int l = 0; l < 4; l++) { drop(M.Z[l]); drop(M.H[l]); }
+}
+
+// workspaces for batches of up to n samples (rounded up to a whole 128-row tile);
+// none are left when they cannot all be had
 static bool mlp_reserve(int n)
 {
+    if (n > INT_MAX / 128 * 128) {
+        set_error(12, "batches of up to %d samples", INT_MAX / 128 * 128);
+        return false;
+    }
     n = (n + 127) / 128 * 128;
     if (n <= M.cap) return true;
-    auto fr = [](void* p) { if (p) cudaFree(p); };
-    fr(M.X); fr(M.G0); fr(M.G1); fr(M.dY); fr(M.Y); fr(M.dYf);
-    for (int l = 0; l < 4; l++) { fr(M.Z[l]); fr(M.H[l]); }
+    mlp_drop_batch();
     size_t h = sizeof(__nv_bfloat16) * (size_t)n * kHid;
     bool ok = cuda_ok(cudaMalloc(&M.X, sizeof(__nv_bfloat16) * (size_t)n * kIn), "X") &&
               cuda_ok(cudaMalloc(&M.G0, h), "G0") && cuda_ok(cudaMalloc(&M.G1, h), "G1") &&
@@ -458,6 +483,7 @@ static bool mlp_reserve(int n)
     // the padding columns of dY (beyond the 8 that forward_loss writes) stay zero
     if (ok) ok = cuda_ok(cudaMemsetAsync(M.dY, 0, sizeof(__nv_bfloat16) * (size_t)n * kDYld, g.stream), "dY zero");
     if (ok) M.cap = n;
+    else mlp_drop_batch();
     return ok;
 }
 
