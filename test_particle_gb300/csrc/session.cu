@@ -183,6 +183,8 @@ bool Session::reserve(int n)
     }
     if (n <= cap) return true;
     size_t rec = sizeof(double) * 11 * (size_t)n;
+    cap = 0;  // until all of them are there
+    loaded = false;
     if (!soa.get(rec) || !soa0.get(rec) || !aos.get(rec) || !nsteps.get(sizeof(int) * (size_t)n))
         return false;
     cap = n;
