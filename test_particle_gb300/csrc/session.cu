@@ -4,6 +4,7 @@
 #include <climits>
 #include <cmath>
 #include <cstring>
+#include <sys/mman.h>
 #include <unistd.h>
 
 #include "../../include/tp_gpu.h"
@@ -584,13 +585,18 @@ extern "C" int tp_session_fetch(tp_session* s, particles* ptl, int* nsteps_ptl, 
 // Maps the pages of a buffer that is about to be written: a fresh allocation's
 // pages are zeroed one by one at their first touch, 10 GB/s on one core, which
 // the tracking kernel's time hides.  The contents stay: a run that fails leaves
-// its caller's arrays as they were.
+// its caller's arrays as they were.  (Where the kernel does not take the advice,
+// an atomic addition of nothing to each page: a load and a store would fault
+// twice on a page that is not there, 92 MB 33 ms a run in place of 13.)
 static void touch_pages(void* p, size_t bytes)
 {
-    const size_t page = (size_t)sysconf(_SC_PAGESIZE);
-    volatile char* c = (volatile char*)p;
-    for (size_t i = 0; i < bytes; i += page) c[i] = c[i];
-    if (bytes > 0) c[bytes - 1] = c[bytes - 1];  // (the first byte need not start a page)
+    if (bytes == 0) return;
+    const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE), a = (uintptr_t)p, end = a + bytes;
+    const uintptr_t first = a & ~(page - 1);
+#ifdef MADV_POPULATE_WRITE
+    if (madvise((void*)first, end - first, MADV_POPULATE_WRITE) == 0) return;
+#endif
+    for (uintptr_t q = first; q < end; q += page) __atomic_fetch_add((unsigned char*)(q < a ? a : q), 0, __ATOMIC_RELAXED);
 }
 
 extern "C" int tp_track_host_to(int precision, int nptl, double dt, int nt_out, int nbins,
