@@ -462,7 +462,7 @@ bool Session::fetch(particles* ptl, int* nsteps_ptl, double* espect, double* esp
 {
     cudaStream_t s = g.stream;
     if (ptl && n > 0) {
-        const bool direct = in_place(ptl, 8);
+        const bool direct = result_in_place(ptl, sizeof(particles) * (size_t)n, 8);
         soa_to_aos((const double*)soa.ptr, n, cap, direct ? (double*)ptl : (double*)aos.ptr, s);
         if (!direct) cudaMemcpyAsync(ptl, aos.ptr, sizeof(particles) * n, cudaMemcpyDeviceToHost, s);
     }

@@ -111,3 +111,33 @@ def test_failed_run_leaves_the_outputs():
     shifted = both[n // 2:n // 2 + n]
     assert _track(tp.PREC_MIXED, n, both, both, shifted, nst) == 0
     assert shifted.tobytes() == want.tobytes()
+
+
+@pytest.mark.parametrize("n", [87381, 87382])
+def test_field_batches_around_the_size_of_results_in_place(n):
+    """48 bytes a point: 4 MB of results and one more point."""
+    _setup()
+    rng = np.random.default_rng(7)
+    pts = rng.random((n, 4))
+    out = tp.get_emf(pts)
+    pick = np.r_[0:300, n - 300:n]
+    assert np.array_equal(tp.get_emf(pts[pick]), out[pick])
+    mixed = tp.get_emf_mixed(np.r_[pts, pts][:, :3])  # 24 bytes a point
+    assert mixed[:n].tobytes() == mixed[n:].tobytes()
+    assert np.array_equal(tp.get_emf_mixed(pts[pick, :3]), mixed[pick])
+
+
+@pytest.mark.parametrize("n", [47662, 47663])
+def test_records_around_the_size_of_results_in_place(n):
+    """88 bytes a particle, fetched from a session and from a whole run."""
+    _setup()
+    p = wl.shell_particles(n, 0.5, (0, 0, 0), (1, 1, 1), 1)
+    r = tp.track(p, DT, 1, 50, precision=tp.PREC_MIXED)
+    s = tp.Session(n)
+    s.load(p)
+    s.track(DT, 1, 50, tp.PREC_MIXED)
+    f = s.fetch(1, 50, 1)
+    assert f["ptl"].tobytes() == r["ptl"].tobytes()
+    assert np.array_equal(f["nsteps"], r["nsteps"])
+    few = tp.track(p[n - 100:], DT, 1, 50, precision=tp.PREC_MIXED)
+    assert few["ptl"].tobytes() == r["ptl"][n - 100:].tobytes()
