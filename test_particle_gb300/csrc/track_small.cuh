@@ -64,7 +64,7 @@ __device__ __forceinline__ void small_field(const DevField& f, int c, double x, 
         const double as = c == 0 ? f.ffA : c == 1 ? f.ffB : f.ffC, ac = c == 0 ? f.ffC : c == 1 ? f.ffA : f.ffB;
         B = as * sp + ac * cp;
         B *= f.B0;
-    } else if (SYS == TP_SYS_MODESUM && f.fxm) {
+    } else if (SYS == TP_SYS_MODESUM) {
         extern __shared__ int4 s_ctab[];
         const uint64_t u[3] = {fixed_frac64((grp(x, 0) - f.xmin) / (f.xmax - f.xmin)),
                                fixed_frac64((grp(x, 1) - f.ymin) / (f.ymax - f.ymin)),
@@ -119,7 +119,7 @@ __device__ __forceinline__ void small_field(const DevField& f, int c, double x, 
         if (c == 2) B = B + 0.0;
     } else {
         double e[6];
-        emf64<SYS, SYS == TP_SYS_MODESUM>(f, grp(x, 0), grp(x, 1), grp(x, 2), t, e, status);
+        emf64<SYS>(f, grp(x, 0), grp(x, 1), grp(x, 2), t, e, status);
         B = c == 0 ? e[0] : c == 1 ? e[1] : e[2];
         E = c == 0 ? e[3] : c == 1 ? e[4] : e[5];
     }
@@ -201,7 +201,7 @@ __global__ void __launch_bounds__(128) track_small_kernel(DevField f, TrackBufs 
 {
     __shared__ double red[(128 / 32) * 8];
     __shared__ SmallShared sh;
-    if (SYS == TP_SYS_MODESUM && f.fxm) {
+    if (SYS == TP_SYS_MODESUM) {
         extern __shared__ int4 s_ctab[];
         for (int k = threadIdx.x; k <= fx::kTab; k += blockDim.x) s_ctab[k] = f.ctab[k];
         __syncthreads();
@@ -316,6 +316,10 @@ int track_small_blocks(const DevField& f, int n, int num_sms)
     const int blocks = (n + kSmallTile - 1) / kSmallTile;
     if (n < 1 || blocks > per_sm * num_sms) return 0;
     if (f.system_type == TP_SYS_WLCS && f.nwlcs > kSmallSystems) return 0;
+    // a mode table that stays in FP64 is not split over the lanes: every lane
+    // would sum all of it (17,000 modes, 9,000 particles x 2 steps: 159 ms, 92 in
+    // track_kernel; one particle: 92 and 84)
+    if (f.system_type == TP_SYS_MODESUM && !f.fxm) return 0;
     return blocks;
 }
 
