@@ -279,6 +279,36 @@ __device__ __noinline__ void interp_exact(const DevField& f, double x, double y,
     for (int a = 0; a < NF; a++) interp_f3(f, r, g[a], ga[a], gb[a], out[a], status);
 }
 
+// The same for component c alone of each field.
+template <int NF>
+__device__ __noinline__ void interp_exact_lane(const DevField& f, double x, double y, double z, double t,
+                                               const float* const g[NF], const float* const ga[NF],
+                                               const float* const gb[NF], int c, float out[NF], int* status)
+{
+    Tri64 r;
+    trilinear64(f, x, y, z, t, r);
+#pragma unroll
+    for (int a = 0; a < NF; a++) {
+        if (f.multi_tframe == 0) {
+            float v = 0.0f;
+#pragma unroll
+            for (int i = 0; i < 8; i++)
+                if (corner_ok(f, r.c[i], status))
+                    v = (float)((double)v + (double)__ldg(g[a] + 3 * r.c[i] + c) * r.w[i]);
+            out[a] = v;
+        } else {
+            double p = 0.0, q = 0.0;
+#pragma unroll
+            for (int i = 0; i < 8; i++)
+                if (corner_ok(f, r.c[i], status)) {
+                    p += (double)__ldg(ga[a] + 3 * r.c[i] + c) * r.w[i];
+                    q += (double)__ldg(gb[a] + 3 * r.c[i] + c) * r.w[i];
+                }
+            out[a] = (float)(r.dt * p + (1.0 - r.dt) * q);
+        }
+    }
+}
+
 template <int NF>
 __device__ __forceinline__ void interp_grids(const DevField& f, double x, double y, double z, double t,
                                              const float* const g[NF], const float* const ga[NF],

@@ -10,7 +10,8 @@
 // scalars come from the group by shuffles.  The fields split likewise: one
 // sine and cosine a lane (force-free), a quarter of the modes a lane (mode
 // sum), and one wire or loop a warp for the block's 32 particles (current
-// systems), through shared memory; gridded fields are evaluated by every lane.
+// systems), through shared memory; gridded fields are evaluated by every lane
+// where the filtered sums hold and by component where they do not.
 // Every particle's operations and their order are those of track_kernel.
 // Whole runs: 256 particles x 200 steps, ABC, 3.11 -> 1.79 ms; 4,096 x 200, two
 // wires and loops, 23.2 -> 9.2 ms (4.5 with the integrals of ellint_fx.cuh).
@@ -117,6 +118,29 @@ __device__ __forceinline__ void small_field(const DevField& f, int c, double x, 
             if (!(p & 1) && f.iBessel != 0) E += sh.part[p][3 + c][q];
         }
         if (c == 2) B = B + 0.0;
+    } else if (SYS == TP_SYS_MHD || SYS == TP_SYS_PIC) {
+        // every lane evaluates the whole grid sample where the filtered sums are
+        // certain; where they are not, the reference's arithmetic on its own
+        // component only (two time frames, 9,000 particles x 110 steps: 7.8 ms with
+        // all components in every lane, 4.6 so, 5.5 with a lane a particle)
+        const bool mhd = SYS == TP_SYS_MHD;
+        const float *g[2] = {mhd ? f.vc_f : f.ec_f, f.bc_f}, *ga[2] = {mhd ? f.va_f : f.ea_f, f.ba_f},
+                    *gb[2] = {mhd ? f.vb_f : f.eb_f, f.bb_f};
+        const double px = grp(x, 0), py = grp(x, 1), pz = grp(x, 2);
+        float all[2][3], own[2];
+        if (f.multi_tframe == 0 && interp_filtered<2>(f, px, py, pz, g, all)) {
+            own[0] = c == 0 ? all[0][0] : c == 1 ? all[0][1] : all[0][2];
+            own[1] = c == 0 ? all[1][0] : c == 1 ? all[1][1] : all[1][2];
+        } else {
+            interp_exact_lane<2>(f, px, py, pz, t, g, ga, gb, c, own, status);
+        }
+        B = own[1];
+        E = own[0];
+        if (mhd) {  // E = B x v (src/emfields.c:107-120), the next two components of each
+            const int c1 = c == 2 ? 0 : c + 1, c2 = c == 0 ? 2 : c - 1;
+            const double v = own[0];
+            E = grp(B, c1) * grp(v, c2) - grp(B, c2) * grp(v, c1);
+        }
     } else {
         double e[6];
         emf64<SYS>(f, grp(x, 0), grp(x, 1), grp(x, 2), t, e, status);
