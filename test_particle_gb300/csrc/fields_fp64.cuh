@@ -42,19 +42,16 @@ __device__ __forceinline__ void trilinear64(const DevField& f, double x, double 
                                             double t, Tri64& r)
 {
     int nx = f.nx, ny = f.ny, nz = f.nz;
-    int ix1 = (int)floor((x - f.xmin) / f.gdx);
-    int iy1 = (int)floor((y - f.ymin) / f.gdy);
-    int iz1 = (int)floor((z - f.zmin) / f.gdz);
+    // (quotients in integers, soft64.cuh: the same doubles)
+    const bool ox = x > f.xmax || x < f.xmin, oy = y > f.ymax || y < f.ymin, oz = z > f.zmax || z < f.zmin;
+    const double qx = sd::div(ox ? x : x - f.xmin, f.d_gdx), qy = sd::div(oy ? y : y - f.ymin, f.d_gdy),
+                 qz = sd::div(oz ? z : z - f.zmin, f.d_gdz);
+    int ix1 = (int)floor(qx), iy1 = (int)floor(qy), iz1 = (int)floor(qz);
     int ix2 = ix1 + 1, iy2 = iy1 + 1, iz2 = iz1 + 1;
-    double dx = (x - f.xmin) / f.gdx - ix1;
-    double dy = (y - f.ymin) / f.gdy - iy1;
-    double dz = (z - f.zmin) / f.gdz - iz1;
-    if (x > f.xmax) { ix1 = nx - 1; ix2 = 0; dx = x / f.gdx - (nx - 1); }
-    if (y > f.ymax) { iy1 = ny - 1; iy2 = 0; dy = y / f.gdy - (ny - 1); }
-    if (z > f.zmax) { iz1 = nz - 1; iz2 = 0; dz = z / f.gdz - (nz - 1); }
-    if (x < f.xmin) { ix1 = nx - 1; ix2 = 0; dx = x / f.gdx + 1.0; }
-    if (y < f.ymin) { iy1 = ny - 1; iy2 = 0; dy = y / f.gdy + 1.0; }
-    if (z < f.zmin) { iz1 = nz - 1; iz2 = 0; dz = z / f.gdz + 1.0; }
+    double dx = qx - ix1, dy = qy - iy1, dz = qz - iz1;
+    if (ox) { ix1 = nx - 1; ix2 = 0; dx = x < f.xmin ? qx + 1.0 : qx - (nx - 1); }
+    if (oy) { iy1 = ny - 1; iy2 = 0; dy = y < f.ymin ? qy + 1.0 : qy - (ny - 1); }
+    if (oz) { iz1 = nz - 1; iz2 = 0; dz = z < f.zmin ? qz + 1.0 : qz - (nz - 1); }
     if (f.multi_tframe == 0) {
         r.dt = 0.0;
     } else {
@@ -268,15 +265,27 @@ __device__ __forceinline__ bool interp_filtered(const DevField& f, double x, dou
     return !bad;
 }
 
-// NF fields on float grids in the reference's own arithmetic (any time frames).
+// NF fields on float grids in the reference's own arithmetic (any time frames): a
+// call in the loops of the push, whose instruction cache it would fill, inline
+// (INL below) in the diffusion terms of a batch, which evaluate it twice and where
+// the call made a pair in two time frames 71 us instead of 59.
+template <int NF>
+__device__ __forceinline__ void interp_exact_inline(const DevField& f, double x, double y, double z, double t,
+                                                    const float* const g[NF], const float* const ga[NF],
+                                                    const float* const gb[NF], float out[NF][3], int* status)
+{
+    Tri64 r;
+    trilinear64(f, x, y, z, t, r);
+#pragma unroll
+    for (int a = 0; a < NF; a++) interp_f3(f, r, g[a], ga[a], gb[a], out[a], status);
+}
+
 template <int NF>
 __device__ __noinline__ void interp_exact(const DevField& f, double x, double y, double z, double t, const float* const g[NF],
                                           const float* const ga[NF], const float* const gb[NF], float out[NF][3],
                                           int* status)
 {
-    Tri64 r;
-    trilinear64(f, x, y, z, t, r);
-    for (int a = 0; a < NF; a++) interp_f3(f, r, g[a], ga[a], gb[a], out[a], status);
+    interp_exact_inline<NF>(f, x, y, z, t, g, ga, gb, out, status);
 }
 
 // The same for component c alone of each field.
@@ -309,13 +318,15 @@ __device__ __noinline__ void interp_exact_lane(const DevField& f, double x, doub
     }
 }
 
-template <int NF>
+template <int NF, bool INL = false>
 __device__ __forceinline__ void interp_grids(const DevField& f, double x, double y, double z, double t,
                                              const float* const g[NF], const float* const ga[NF],
                                              const float* const gb[NF], float out[NF][3], int* status)
 {
-    if (f.multi_tframe != 0 || !interp_filtered<NF>(f, x, y, z, g, out))
-        interp_exact<NF>(f, x, y, z, t, g, ga, gb, out, status);
+    if (f.multi_tframe != 0 || !interp_filtered<NF>(f, x, y, z, g, out)) {
+        if (INL) interp_exact_inline<NF>(f, x, y, z, t, g, ga, gb, out, status);
+        else interp_exact<NF>(f, x, y, z, t, g, ga, gb, out, status);
+    }
 }
 
 // ---------------------------------------------------------------- WLCS
@@ -514,7 +525,7 @@ __device__ __forceinline__ void mode_sum_fixed(const DevField& f, const int4* ta
 // get_emf, src/emfields.c:32-60, specialised per system type (0..5).  TAB: the
 // cosine table of the mode sum lies at the start of the block's dynamic shared
 // memory, else it is read from global memory.
-template <int SYS, bool TAB = false>
+template <int SYS, bool TAB = false, bool INL = false>
 __device__ __forceinline__ void emf64(const DevField& f, double x, double y, double z, double t,
                                       double e[6], int* status)
 {
@@ -574,7 +585,7 @@ __device__ __forceinline__ void emf64(const DevField& f, double x, double y, dou
         // getemf_mhd_test_particle, src/emfields.c:107-120
         const float *g[2] = {f.vc_f, f.bc_f}, *ga[2] = {f.va_f, f.ba_f}, *gb[2] = {f.vb_f, f.bb_f};
         float vb[2][3];
-        interp_grids<2>(f, x, y, z, t, g, ga, gb, vb, status);
+        interp_grids<2, INL>(f, x, y, z, t, g, ga, gb, vb, status);
         const float *v = vb[0], *b = vb[1];
         e[0] = b[0]; e[1] = b[1]; e[2] = b[2];
         e[3] = e[1] * v[2] - e[2] * v[1];
@@ -585,7 +596,7 @@ __device__ __forceinline__ void emf64(const DevField& f, double x, double y, dou
         // computes the same corners and weights twice, once is enough
         const float *g[2] = {f.ec_f, f.bc_f}, *ga[2] = {f.ea_f, f.ba_f}, *gb[2] = {f.eb_f, f.bb_f};
         float eb[2][3];
-        interp_grids<2>(f, x, y, z, t, g, ga, gb, eb, status);
+        interp_grids<2, INL>(f, x, y, z, t, g, ga, gb, eb, status);
         const float *ev = eb[0], *b = eb[1];
         e[3] = ev[0]; e[4] = ev[1]; e[5] = ev[2];
         e[0] = b[0]; e[1] = b[1]; e[2] = b[2];

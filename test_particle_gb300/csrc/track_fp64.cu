@@ -147,7 +147,7 @@ __device__ __forceinline__ int energy_bin(const double* thr, int nbins, double u
 
 // calc_diff_coeff, src/diagnostics.c:659-705 (pow(v, 2) taken as v * v).
 // Output order: drr, dxx, dyy, dzz, dpp, duu, daa, dee.
-template <int SYS, bool TAB = false>
+template <int SYS, bool TAB = false, bool INL = false>
 __device__ __forceinline__ void calc_diff(const DevField& f, const P64& p0, const P64& p,
                                           double dt, double o[8], int* status)
 {
@@ -162,8 +162,8 @@ __device__ __forceinline__ void calc_diff(const DevField& f, const P64& p0, cons
     double dg = gamma - gamma0;
     double dee = dg * dg / t;
     double e[6], e0[6];
-    emf64<SYS, TAB>(f, p.x, p.y, p.z, p.t, e, status);
-    emf64<SYS, TAB>(f, p0.x, p0.y, p0.z, p0.t, e0, status);
+    emf64<SYS, TAB, INL>(f, p.x, p.y, p.z, p.t, e, status);
+    emf64<SYS, TAB, INL>(f, p0.x, p0.y, p0.z, p0.t, e0, status);
     double abs_b = sqrt(e[0] * e[0] + e[1] * e[1] + e[2] * e[2]);
     double abs_u = sqrt(p.ux * p.ux + p.uy * p.uy + p.uz * p.uz);
     double mu = (e[0] * p.ux + e[1] * p.uy + e[2] * p.uz) / (abs_b * abs_u);
@@ -424,7 +424,7 @@ __global__ void diffc_kernel(DevField f, int n, const double* st0, const double*
     P64 p = {r[0], r[1], r[2], r[4], r[5], r[6], r[7], r[8], r[9], r[10]};
     P64 p0 = {r0[0], r0[1], r0[2], r0[4], r0[5], r0[6], r0[7], r0[8], r0[9], r0[10]};
     double o[8];
-    calc_diff<SYS>(f, p0, p, dt, o, status);
+    calc_diff<SYS, false, true>(f, p0, p, dt, o, status);
     for (int k = 0; k < 8; k++) out[8 * i + k] = o[k];
 }
 
@@ -597,7 +597,8 @@ __global__ void poincare_kernel(DevField f, int n, const double* __restrict__ se
 // eight weights two a lane, exchanged as float pairs by shuffles.  Operations
 // and order are those of poincare_kernel.  256^3 grid, 4 crossings, against
 // that kernel: 1,024 seeds 13.8 -> 7.2 ms, 4,000 14.1 -> 7.4, 16,000 14.0 ->
-// 12.9; 30,000 seeds 18.9 -> 26.2, so it stops at kPoincareSmall.
+// 12.9; 30,000 seeds 18.9 -> 26.2, so it stops at kPoincareSmall.  (16 blocks an SM
+// let the compiler take 112 registers; by itself it took 96 and spilled, 2 % slower.)
 constexpr int kPoincareSmall = 16384;
 __device__ __forceinline__ double sgrp(double v, int k) { return __shfl_sync(0xffffffffu, v, (threadIdx.x & 28) | k); }
 __device__ __forceinline__ float sgrp(float v, int k) { return __shfl_sync(0xffffffffu, v, (threadIdx.x & 28) | k); }
@@ -644,16 +645,16 @@ __device__ __forceinline__ double pm_unit_lane(const DevField& f, int c, double 
     const double px = sgrp(x, 0), py = sgrp(x, 1), pz = sgrp(x, 2);
     if (any & 15u) {  // the whole group: not certain
         const float *g[1] = {f.bc_f}, *ga[1] = {f.ba_f}, *gb[1] = {f.bb_f};
-        float w[1][3];
-        interp_exact<1>(f, px, py, pz, 0.0, g, ga, gb, w, status);
-        v = c == 0 ? w[0][0] : c == 1 ? w[0][1] : w[0][2];
+        float w[1];
+        interp_exact_lane<1>(f, px, py, pz, 0.0, g, ga, gb, c, w, status);
+        v = w[0];
     }
     const double b = v, b2 = b * b;
     const double ib = sd::div(1.0, sd::sqrt_rn(sgrp(b2, 0) + sgrp(b2, 1) + sgrp(b2, 2)));
     return b * ib;
 }
 
-__global__ void __launch_bounds__(32) poincare_small_kernel(DevField f, int n, const double* __restrict__ seeds,
+__global__ void __launch_bounds__(32, 16) poincare_small_kernel(DevField f, int n, const double* __restrict__ seeds,
                                                             int face, double h, double lmax, int ncross, double* xo,
                                                             double* yo, double* zo, int* found, int* status)
 {
