@@ -650,17 +650,23 @@ __global__ void from_split_kernel(const float* __restrict__ P, int M, int N, int
 
 // Self-check: row-major A [rows][K] into blocks (kind 0), k-atoms of R rows
 // (kind 1), or transposed, K the samples, into blocks of `atoms` 64-column
-// atoms (kind 2).
-__global__ void to_blocks_kernel(const __nv_bfloat16* __restrict__ A, int rows, int K, int kind, int atoms,
-                                 unsigned char* __restrict__ out)
+// atoms (kind 2); both operands in one launch (blockIdx.y).
+struct PackOp {
+    const __nv_bfloat16* A;
+    int rows, kind, atoms;
+    unsigned char* out;
+};
+
+__global__ void to_blocks_kernel(PackOp a, PackOp b, int K)
 {
+    const PackOp p = blockIdx.y == 0 ? a : b;
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (size_t)rows * K) return;
+    if (i >= (size_t)p.rows * K) return;
     const int r = (int)(i / K), k = (int)(i % K);
-    const size_t o = kind == 0   ? tctrain::tile_offset(r, k, atoms)
-                     : kind == 1 ? (size_t)tc::sw128_offset(rows, r, k)
-                                 : tctrain::tile_offset(k, r, atoms);
-    *reinterpret_cast<__nv_bfloat16*>(out + o) = A[i];
+    const size_t o = p.kind == 0   ? tctrain::tile_offset(r, k, p.atoms)
+                     : p.kind == 1 ? (size_t)tc::sw128_offset(p.rows, r, k)
+                                   : tctrain::tile_offset(k, r, p.atoms);
+    *reinterpret_cast<__nv_bfloat16*>(p.out + o) = p.A[i];
 }
 
 }  // namespace tct
@@ -722,8 +728,9 @@ static cudaError_t gemm_f32(const __nv_bfloat16* A, const __nv_bfloat16* B, int 
     const bool layer = N == 256 && K <= 256;
     const int kpad = (K + 127) / 128 * 128, npad = (N + 63) / 64 * 64;
     unsigned char *wa = work, *wb = work + 2 * (size_t)M * kpad;
-    to_blocks_kernel<<<grid((size_t)M * K), 256, 0, s>>>(A, M, K, layer ? 0 : 2, layer ? K / 64 : M / 64, wa);
-    to_blocks_kernel<<<grid((size_t)N * K), 256, 0, s>>>(B, N, K, layer ? 1 : 2, layer ? K / 64 : npad / 64, wb);
+    to_blocks_kernel<<<dim3(grid((size_t)std::max(M, N) * K), 2), 256, 0, s>>>(
+        PackOp{A, M, layer ? 0 : 2, layer ? K / 64 : M / 64, wa},
+        PackOp{B, N, layer ? 1 : 2, layer ? K / 64 : npad / 64, wb}, K);
     if (layer) return launch_layer<256>(wa, wb, M, K, EpiStoreF32{D}, status, s);
     float* P = reinterpret_cast<float*>(wb + 2 * (size_t)npad * kpad);
     cudaError_t e = launch_weights(wa, M / 128, wb, npad / 64, K / 64, P, 1, nullptr, status, s);
@@ -757,27 +764,20 @@ extern "C" int tp_tc_gemm_train_bf16(int m, int n, int k, const unsigned short* 
     cudaStream_t s = g.stream;
     const size_t sa = sizeof(uint16_t) * (size_t)m * k, sb = sizeof(uint16_t) * (size_t)n * k,
                  sd = sizeof(float) * (size_t)m * n;
-    const size_t sw = tctrain::gemm_work_bytes(m, n, k);
-    void *dA = nullptr, *dB = nullptr, *dD = nullptr, *dW = nullptr;
-    bool ok = cuda_ok(cudaMalloc(&dA, sa), "A") && cuda_ok(cudaMalloc(&dB, sb), "B") &&
-              cuda_ok(cudaMalloc(&dD, sd), "D") && cuda_ok(cudaMalloc(&dW, sw), "work");
-    if (ok) {
-        cudaMemcpyAsync(dA, a, sa, cudaMemcpyHostToDevice, s);
-        cudaMemcpyAsync(dB, b, sb, cudaMemcpyHostToDevice, s);
-        cudaMemsetAsync(dD, 0, sd, s);
-        cudaMemsetAsync(dW, 0, sw, s);
-        ok = cuda_ok(tctrain::gemm_f32(static_cast<const __nv_bfloat16*>(dA), static_cast<const __nv_bfloat16*>(dB),
-                                       m, n, k, static_cast<unsigned char*>(dW), static_cast<float*>(dD),
-                                       g.d_status, s),
-                     "train gemm");
-    }
-    if (ok) {
-        cudaMemcpyAsync(d, dD, sd, cudaMemcpyDeviceToHost, s);
-        ok = cuda_ok(cudaStreamSynchronize(s), "train gemm sync");
-    }
-    if (dA) cudaFree(dA);
-    if (dB) cudaFree(dB);
-    if (dD) cudaFree(dD);
-    if (dW) cudaFree(dW);
-    return ok ? 0 : -1;
+    // all of it in the batch calls' buffer (allocations of its own cost as much as
+    // the kernels); the padding of the packed operands is zero
+    auto whole = [](size_t b) { return (b + 1023) / 1024 * 1024; };
+    const size_t sw = tctrain::gemm_work_bytes(m, n, k), oB = whole(sa), oD = oB + whole(sb), oW = oD + whole(sd);
+    unsigned char* d0 = static_cast<unsigned char*>(g.s_batch_a.get(oW + sw));
+    if (!d0) return -1;
+    cudaMemcpyAsync(d0, a, sa, cudaMemcpyHostToDevice, s);
+    cudaMemcpyAsync(d0 + oB, b, sb, cudaMemcpyHostToDevice, s);
+    cudaMemsetAsync(d0 + oD, 0, oW + sw - oD, s);
+    if (!cuda_ok(tctrain::gemm_f32(reinterpret_cast<const __nv_bfloat16*>(d0),
+                                   reinterpret_cast<const __nv_bfloat16*>(d0 + oB), m, n, k, d0 + oW,
+                                   reinterpret_cast<float*>(d0 + oD), g.d_status, s),
+                 "train gemm"))
+        return -1;
+    cudaMemcpyAsync(d, d0 + oD, sd, cudaMemcpyDeviceToHost, s);
+    return cuda_ok(cudaStreamSynchronize(s), "train gemm sync") ? 0 : -1;
 }
