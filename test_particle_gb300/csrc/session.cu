@@ -375,6 +375,7 @@ bool Session::run(const RunSpec& rs, tp_run_info* info, const std::function<void
     q.sstep = rs.sstep;
     q.traj_every = rs.traj_every;
     q.dt = rs.dt;
+    q.num_sms = g.num_sms;
     auto launch = [&](const TrackParams& qq, int gr) {
         if (small > 0)
             return rs.precision == TP_PREC_FP64 ? fp64::launch_track_small(f, b, qq, g.num_sms, s)

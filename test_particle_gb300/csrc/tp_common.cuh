@@ -100,6 +100,7 @@ struct TrackParams {
     int ntiles;
     int sstep;       // first step index (the reference starts at 1)
     int traj_every;  // nsteps_output when trajectory diagnostics are on, else 0
+    int num_sms;     // of the device (the mixed mode sum's choice of kernel)
     double dt;
     // a segment of an open-boundary run (all zero for a whole run): diffusion
     // rows used before it, whether it continues a run (no initial escape

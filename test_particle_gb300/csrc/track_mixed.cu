@@ -501,12 +501,12 @@ cudaError_t launch_emf_batch(const MixField& f, int n, const double* xyz, float*
 
 // --------------------------------------------------------------- launchers
 // The mode sum with two particles a thread: above three 128-particle blocks per
-// SM (152 of them) -- up to there a particle a thread needs no more rounds of
+// SM (58,368 particles on 152 SMs) -- up to there a particle a thread needs no more rounds of
 // latency than pairs do (38,000 particles: 1.30 ms against 1.32; 50,000: 1.84
 // against 2.16; 60,000: 2.42 against 2.17; 262,144: 8.03 against 6.84) -- and up
 // to the modes whose records leave room for two blocks (1,000 modes, 65,536
 // particles: 4.73 against 5.79 ms).
-constexpr int kPairParticles = 152 * 3 * kBlock;
+constexpr int kPairBlocks = 3;
 constexpr int kPairModes = 1024;
 template <int SYS>
 static cudaError_t launch_sys(const MixField& f, const TrackBufs& b, const TrackParams& q, int grid,
@@ -543,7 +543,7 @@ cudaError_t launch_track(const MixField& f, const TrackBufs& b, const TrackParam
     case TP_SYS_FORCEFREE: return launch_sys<TP_SYS_FORCEFREE>(f, b, q, grid, s);
     case TP_SYS_PIC: return launch_sys<TP_SYS_PIC>(f, b, q, grid, s);
     case TP_SYS_MODESUM:
-        if (f.nmodes <= kPairModes && q.n > kPairParticles) return launch_modes(f, b, q, grid, s);
+        if (f.nmodes <= kPairModes && q.n > kPairBlocks * kBlock * q.num_sms) return launch_modes(f, b, q, grid, s);
         return launch_sys<TP_SYS_MODESUM>(f, b, q, grid, s);
     default: return cudaErrorInvalidValue;
     }
