@@ -266,7 +266,7 @@ static bool run_range(int nptl, const RunSpec& rs, particles* ptl_init, particle
     o.dsum.assign((size_t)8 * s.nsdc, 0.0);
     o.remain.assign(s.nsdc, 0);
     if (!s.fetch(ptl, nsteps_ptl, o.espect.data(), o.espect_esc.data(), o.dsum.data(),
-                 o.remain.data())) return fail();
+                 o.remain.data(), true)) return fail();
     if (rs.traj_every > 0 && !s.get_traj(ptl_time, traj_points)) return false;
     if (wall_ms) *wall_ms = info.kernel_ms;
     return true;

@@ -459,11 +459,11 @@ bool Session::run(const RunSpec& rs, tp_run_info* info, const std::function<void
 }
 
 bool Session::fetch(particles* ptl, int* nsteps_ptl, double* espect, double* espect_escape,
-                    double* dsum_out, int* remain)
+                    double* dsum_out, int* remain, bool mapped)
 {
     cudaStream_t s = g.stream;
     if (ptl && n > 0) {
-        const bool direct = result_in_place(ptl, sizeof(particles) * (size_t)n, 8);
+        const bool direct = result_in_place(ptl, sizeof(particles) * (size_t)n, 8, mapped);
         soa_to_aos((const double*)soa.ptr, n, cap, direct ? (double*)ptl : (double*)aos.ptr, s);
         if (!direct) cudaMemcpyAsync(ptl, aos.ptr, sizeof(particles) * n, cudaMemcpyDeviceToHost, s);
     }
@@ -622,7 +622,7 @@ extern "C" int tp_track_host_to(int precision, int nptl, double dt, int nt_out, 
         cudaStreamSynchronize(g.stream);  // the records may still be read in place
         return -1;
     }
-    if (!s.fetch(ptl_out, nsteps_ptl, espect, espect_escape, dsum, remain)) return -1;
+    if (!s.fetch(ptl_out, nsteps_ptl, espect, espect_escape, dsum, remain, true)) return -1;
     if (remain)  // the kernel counts departures; the reference starts from nptl
         for (int k = 0; k < s.nsdc; k++) remain[k] += nptl;
     return 0;

@@ -95,24 +95,27 @@ inline bool in_place(const void* host, size_t align)
 {
     return g.direct && host && ((uintptr_t)host & (align - 1)) == 0;
 }
-// The same for a result, up to kResultInPlace bytes.  Reading in place is the
+// The same for a result, by its size.  Reading in place is the
 // faster way at any size (particle records: 88 KB 33 us against 50 with copies,
 // 23 MB 150 and 340, 92 MB 0.6 and 1.3 ms, warm or fresh).  Writing is where the
 // pages are there already (0.09 MB 13 us against 19, 5.8 MB 42 and 57, 92 MB 0.5 to
 // 0.6 ms either way), but pages that the device is the first to touch cost it
 // more than they cost the copy: 0.35 MB 80 us against 175, 2.8 MB 255 and 286,
-// 5.8 MB 480 and 400, 23 MB 1.7 and 1.1 ms, 92 MB 6 to 24 and 4 ms.
-constexpr size_t kResultInPlace = (size_t)4 << 20;
-inline bool result_in_place(const void* host, size_t bytes, size_t align)
+// 5.8 MB 480 and 400, 23 MB 1.7 and 1.1 ms, 92 MB 6 to 24 and 4 ms.  So pages that
+// may be new are written up to kNewInPlace bytes, those that the caller's input or
+// touch_pages has mapped up to kMappedInPlace (11.5 MB just mapped: 92 us and 99;
+// 23 MB 165 and 157).
+constexpr size_t kNewInPlace = (size_t)4 << 20, kMappedInPlace = (size_t)16 << 20;
+inline bool result_in_place(const void* host, size_t bytes, size_t align, bool mapped = false)
 {
-    return bytes <= kResultInPlace && in_place(host, align);
+    return bytes <= (mapped ? kMappedInPlace : kNewInPlace) && in_place(host, align);
 }
 // A result that is computed from `input`: where the two overlap it goes through a
 // copy, which follows the last read of the input.
 inline bool result_in_place(const void* host, size_t bytes, size_t align, const void* input, size_t input_bytes)
 {
     const uintptr_t a = (uintptr_t)host, b = (uintptr_t)input;
-    return result_in_place(host, bytes, align) && (a + bytes <= b || b + input_bytes <= a);
+    return result_in_place(host, bytes, align, false) && (a + bytes <= b || b + input_bytes <= a);
 }
 // particles records to columns (both when soa2 is given) and back
 void aos_to_soa(const double* aos, int n, double* d_soa, double* d_soa2, long stride, cudaStream_t s);

@@ -39,9 +39,10 @@ struct Session {
     bool load(const particles* ptl_init, const particles* ptl, int n);
     // meanwhile: host work done once the first kernel is launched
     bool run(const RunSpec& rs, tp_run_info* info, const std::function<void()>& meanwhile = nullptr);
-    // remain: departures counted on the device (negative numbers)
+    // remain: departures counted on the device (negative numbers); mapped: the
+    // pages of ptl are there
     bool fetch(particles* ptl, int* nsteps_ptl, double* espect, double* espect_escape,
-               double* dsum, int* remain);
+               double* dsum, int* remain, bool mapped = false);
     bool set_traj(const int* ntraj_accum, const particles* ptl_time, int* points);
     bool get_traj(particles* ptl_time, int* points);
 };

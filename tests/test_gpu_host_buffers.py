@@ -141,3 +141,13 @@ def test_records_around_the_size_of_results_in_place(n):
     assert np.array_equal(f["nsteps"], r["nsteps"])
     few = tp.track(p[n - 100:], DT, 1, 50, precision=tp.PREC_MIXED)
     assert few["ptl"].tobytes() == r["ptl"][n - 100:].tobytes()
+
+
+@pytest.mark.parametrize("n", [190650, 190651])
+def test_records_around_the_size_of_mapped_results_in_place(n):
+    """A run's own result: 16 MB and one more particle."""
+    _setup()
+    p = wl.shell_particles(n, 0.5, (0, 0, 0), (1, 1, 1), 1)
+    r = tp.track(p, DT, 1, 50, precision=tp.PREC_MIXED)
+    for a in (0, n - 500):
+        assert tp.track(p[a:a + 500], DT, 1, 50, precision=tp.PREC_MIXED)["ptl"].tobytes() == r["ptl"][a:a + 500].tobytes()
