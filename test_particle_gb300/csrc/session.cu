@@ -312,7 +312,8 @@ bool Session::run(const RunSpec& rs, tp_run_info* info, const std::function<void
     const int nslot = grid + (segs ? 1 : 0);  // the last slot takes the departed particles' rows
     size_t nspec = (size_t)nt_out * nbins;
     unsigned* d_spec = (unsigned*)spec.get(sizeof(unsigned) * 2 * nspec);
-    int* d_rem = (int*)rem.get(sizeof(int) * nsdc);
+    const size_t nrem = std::max(nsdc, 2);  // entry 1 takes the particles outside at the start, read or not
+    int* d_rem = (int*)rem.get(sizeof(int) * nrem);
     double* d_dpart = (double*)dpart.get(sizeof(double) * 8 * (size_t)nsdc * nslot);
     double* d_dsum = (double*)dsum.get(sizeof(double) * 8 * (size_t)nsdc);
     if (!d_spec || !d_rem || !d_dpart || !d_dsum) return false;
@@ -335,7 +336,7 @@ bool Session::run(const RunSpec& rs, tp_run_info* info, const std::function<void
     }
     cudaEventRecord(evb, s);
     cudaMemsetAsync(d_spec, 0, sizeof(unsigned) * 2 * nspec, s);
-    cudaMemsetAsync(d_rem, 0, sizeof(int) * nsdc, s);
+    cudaMemsetAsync(d_rem, 0, sizeof(int) * nrem, s);
     cudaMemsetAsync(d_dpart, 0, sizeof(double) * 8 * (size_t)nsdc * nslot, s);
     if (rs.reset_nsteps) fill_int((int*)nsteps.ptr, n, 1, s);
 

@@ -71,7 +71,7 @@ struct TrackBufs {
     const double *ebin_thr;       // nbins - 1 ascending energy thresholds
     unsigned int *espect;         // nt_out * nbins counts
     unsigned int *espect_esc;     // nt_out * nbins counts (open boundary)
-    int *remain;                  // nsdc
+    int *remain;                  // nsdc; track_kernel: 2 entries at least
     double *dpart;                // gridDim.x * nsdc * 8 per-block partial sums (scratch)
     // open-boundary runs in segments (null otherwise): per-particle state
     // carried from one segment to the next (kSegCarry doubles: the diffusion

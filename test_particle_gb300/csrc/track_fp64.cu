@@ -219,8 +219,9 @@ __device__ __forceinline__ void block_diff_sum(const double sg[8], double* red, 
 // Resident blocks per SM the kernel is compiled for (3: at most 168 registers,
 // no spills).  Two blocks (up to 228 registers) left the gridded run of 131,072
 // particles 8 % slower, four (128, 120-316 bytes of spills) 4 %.
-// The mode sum: four blocks (5.62 ms on 65,536 particles x 10 steps against
-// 5.82 with three), its loop unrolled four times (5.77 with two, 5.92 with one).
+// The mode sum: four blocks, with some 100 bytes of spills (kernel time of 10 steps,
+// 512 modes, 65,536 particles 4.63 ms against 4.91 with three and none; 262,144
+// 16.0 and 15.7; in between it depends on the last wave: 131,072 9.25 and 7.97).
 constexpr int track_min_blocks(int sys) { return sys == TP_SYS_MODESUM ? 4 : 3; }
 
 // Persistent fixed-step tracking, restating particle_tracking_multi_steps_openmp
@@ -262,7 +263,9 @@ __global__ void __launch_bounds__(kBlock, track_min_blocks(SYS)) track_kernel(De
 #pragma unroll
             for (int c = 0; c < 8; c++) sg[c] = b.sg_carry[(size_t)i * kSegCarry + c];
         }
-        if (active && esc_pre && !q.resumed && q.nsdc > 1) atomicSub(&b.remain[1], 1);
+        // (remain has two entries at least; a test of q.nsdc here costs the mode
+        // sum 0.6 %, its registers being full)
+        if (active && esc_pre && !q.resumed) atomicSub(&b.remain[1], 1);
         double* slot_base = b.dpart + (size_t)blockIdx.x * q.nsdc * 8;
         int npts = 1;
         long toff = 0;
