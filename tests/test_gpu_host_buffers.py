@@ -151,3 +151,44 @@ def test_records_around_the_size_of_mapped_results_in_place(n):
     r = tp.track(p, DT, 1, 50, precision=tp.PREC_MIXED)
     for a in (0, n - 500):
         assert tp.track(p[a:a + 500], DT, 1, 50, precision=tp.PREC_MIXED)["ptl"].tobytes() == r["ptl"][a:a + 500].tobytes()
+
+
+def _at(nbytes, off):
+    """A byte array of nbytes that starts `off` bytes past a 64-byte boundary."""
+    raw = np.zeros(nbytes + 128, np.uint8)
+    a = -raw.ctypes.data % 64 + off
+    return raw[a:a + nbytes]
+
+
+@pytest.mark.parametrize("n", [1, 129, 60001])
+@pytest.mark.parametrize("src,dst", [(4, 0), (0, 4), (4, 4)])
+def test_misaligned_buffers_take_the_copies(n, src, dst):
+    """Doubles on 4-byte boundaries (and floats on 2-byte ones), which no kernel
+    reads or writes: the same bytes through staged copies."""
+    _setup()
+    L = tp.lib()
+    rng = np.random.default_rng(n)
+    pts = rng.random((n, 4))
+    x, e = _at(32 * n, src), _at(48 * n, dst)
+    x[:] = pts.view(np.uint8).ravel()
+    tp.check(L.tp_get_emf_batch(C.c_int(n), tp._ptr(x), tp._ptr(e)))
+    assert e.tobytes() == tp.get_emf(pts).tobytes()
+    xm, em = _at(24 * n, src), _at(24 * n, dst // 2)
+    xm[:] = np.ascontiguousarray(pts[:, :3]).view(np.uint8).ravel()
+    tp.check(L.tp_get_emf_mixed_batch(C.c_int(n), tp._ptr(xm), tp._ptr(em)))
+    assert em.tobytes() == tp.get_emf_mixed(pts[:, :3]).tobytes()
+    p = wl.shell_particles(n, 0.5, (0, 0, 0), (1, 1, 1), 1)
+    other = p.copy()
+    other["t"] = 0.5
+    want = tp.track(p, DT, 1, 50, precision=tp.PREC_MIXED, ptl=other)
+    p0, p1, out = _at(88 * n, src), _at(88 * n, src), _at(88 * n, dst)
+    p0[:], p1[:] = p.view(np.uint8), other.view(np.uint8)
+    assert _track(tp.PREC_MIXED, n, p0, p1, out) == 0
+    assert out.tobytes() == want["ptl"].tobytes()
+    # one buffer in and out, initial and current records the same
+    want = tp.track(p, DT, 1, 50, precision=tp.PREC_MIXED)
+    esp, ese, ds, rem, nst = np.zeros(50), np.zeros(50), np.zeros(8), np.zeros(1, np.int32), np.zeros(n, np.int32)
+    tp.check(L.tp_track_host(C.c_int(tp.PREC_MIXED), C.c_int(n), C.c_double(DT), C.c_int(1), C.c_int(50), tp._ptr(p0),
+                             tp._ptr(p0), tp._ptr(nst), tp._ptr(esp), tp._ptr(ese), tp._ptr(ds), tp._ptr(rem), None))
+    assert p0.tobytes() == want["ptl"].tobytes() and np.array_equal(nst, want["nsteps"])
+    assert np.array_equal(esp, want["espect"].ravel())
