@@ -1,10 +1,19 @@
-// fields_fp64.cuh -- FP64 field evaluation on the device, reference arithmetic.
+// fields_fp64.cuh -- FP64 field evaluation on the device.
 //
-// Each function follows the reference function named in its comment with the
-// same operation order; the translation unit is compiled with -fmad=false so
-// no multiply-add is fused, and sqrt / division are IEEE correctly rounded, so
-// results differ from the reference only where CUDA's sin/cos/acos/log differ
-// from glibc's by an ulp.
+// Each function follows the reference function named in its comment.  In the
+// parity build (-fmad=false: no multiply-add is fused) a field differs from the
+// reference's by:
+//   gridded fields   nothing: the same roundings, in FP32 with carried errors
+//                    where those are certain (interp_filtered), else in double;
+//   analytic ABC     sine and cosine in fixed point (soft64.cuh, 0.513 units of
+//                    the last place), the sums in the reference's order;
+//   wires            the same sine and cosine, CUDA's arc cosine and Bessel terms;
+//   loops            K and E in fixed point (ellint_fx.cuh, 6.5e-16 and 4.1e-15 of
+//                    their value at most), CUDA's logarithm, the rest in order;
+//                    the adaptive stepper keeps the FP64 series;
+//   mode sum         the whole sum in fixed point (modesum_fx.cuh; its header has
+//                    the errors by number of modes), in FP64 outside its range.
+// Divisions and square roots are correctly rounded throughout.
 #pragma once
 #include "ellint_fx.cuh"
 #include "tp_common.cuh"

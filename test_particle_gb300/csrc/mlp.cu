@@ -162,7 +162,7 @@ __global__ void __launch_bounds__(128) moments_kernel(const float* __restrict__ 
 
 // ---------------------------------------------------------------- loss, output layer, AdamW
 constexpr int kDYld = 64;         // columns of dY: one k-atom of the output layer's data-gradient GEMM
-constexpr int kWgradSplits = 80;  // most split-K parts of a weight-gradient GEMM
+constexpr int kWgradSplits = 76;  // most split-K parts of a weight-gradient GEMM: two CTAs each, one an SM
 
 // Partial sums of the output layer's gradients from the FP32 loss gradient dYf
 // [n][6] and the last hidden activations H3 [n][256]: part[block] holds
@@ -436,7 +436,7 @@ static bool mlp_alloc_params()
         ok = ok &&
              cuda_ok(cudaMalloc(&M.wpart[l], sizeof(float) * (size_t)kWgradSplits * kHid * layer_in(l)),
                      "mlp weight partial") &&
-             cuda_ok(cudaMalloc(&M.bpart[l], sizeof(float) * (size_t)max_blocks() * kHid), "mlp bias partial");
+             cuda_ok(cudaMalloc(&M.bpart[l], sizeof(float) * (size_t)tctrain::kBiasParts * kHid), "mlp bias partial");
     }
     ok = ok && zeroed(M.cp.pack, kPackBytes, "mlp wpack") &&
          cuda_ok(cudaMalloc(&M.opart, sizeof(float) * (size_t)max_blocks() * kOutGrad), "mlp output partial") &&
@@ -552,7 +552,7 @@ static bool mlp_backward(int n, const Adam* step)
     out_grad_kernel<<<oblocks, 256, 0, s>>>(M.dYf, M.H[3], n / 128, M.opart);
     // split the samples so that the two 128-row tiles fill the SMs, at least
     // four steps of 64 per split
-    const int splits = std::max(1, std::min({kWgradSplits, 76, n / 256}));
+    const int splits = std::max(1, std::min(kWgradSplits, n / 256));
     const unsigned char* gin = M.dY;
     unsigned char *gcur = M.G0, *gnext = M.G1;
     Partials ps;
@@ -719,8 +719,8 @@ extern "C" int tp_mlp_train(long long nsamples, int batch, int epochs, double lr
     {
         const int cnt = (int)std::min<long long>(nsamples, 1 << 20);
         const int blocks = std::min((cnt + 127) / 128, max_blocks());
-        static_assert(2 * sizeof(double) * kOut <= sizeof(float) * kHid, "the moments fit the bias partial sums");
-        double* part = reinterpret_cast<double*>(M.bpart[0]);
+        static_assert(2 * sizeof(double) * kOut <= sizeof(float) * kOutGrad, "the moments fit a block's partial gradients");
+        double* part = reinterpret_cast<double*>(M.opart);
         std::vector<double> hp((size_t)blocks * 2 * kOut);
         moments_kernel<<<blocks, 128, 0, s>>>(dT, cnt, part);
         cudaMemcpyAsync(hp.data(), part, sizeof(double) * hp.size(), cudaMemcpyDeviceToHost, s);

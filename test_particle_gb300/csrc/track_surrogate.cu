@@ -160,7 +160,6 @@ __device__ __noinline__ void mma_issuer(const Pipe& pp, int* status)
             ok = wait_or_abort(aready, nready & 1, abort, lim);
             nready++;
             if (ok && *stop) {
-
                 stopped = true;
                 ok = false;
             }
@@ -226,7 +225,7 @@ __device__ __noinline__ void field_tile(const Model& md, const Pipe& pp, Cons& c
     const uint32_t accf = pp.accf, aready = pp.aready, lim = pp.lim;
     int* const abort = pp.abort;
     const float *const hbias = pp.hbias, *const bias = pp.bias;
-    // (a lattice vector is one 16-byte load: 8.84 against 8.70 ms a pass)
+    // (a lattice vector is one 16-byte load: 8.70 ms a pass, 8.84 with three of 4 bytes)
     const int4* freq = reinterpret_cast<const int4*>(pp.freq);
     // Fourier features of this thread's particle: inputs 0..63 sin, 64..127 cos
     {
