@@ -177,7 +177,8 @@ extern double emin, emax, logemin, logemax, logde;
 
 enum {
     TP_PREC_FP64 = 0,       /* reference arithmetic (no FMA contraction): parity path */
-    TP_PREC_FP64_FAST = 1,  /* FP64 with FMA contraction */
+    TP_PREC_FP64_FAST = 1,  /* FP64 with FMA contraction; a particle's last places depend on whether
+                             * the run is small enough for the kernel of few particles */
     TP_PREC_MIXED = 2,      /* FP32 push and field, 64-bit fixed-point positions */
     TP_PREC_SURROGATE = 3   /* as MIXED with the learned field model (mode-sum field) */
 };
