@@ -101,7 +101,8 @@ inline bool in_place(const void* host, size_t align)
 // pages are there already (0.09 MB 13 us against 19, 5.8 MB 42 and 57, 92 MB 0.5 to
 // 0.6 ms either way), but pages that the device is the first to touch cost it
 // more than they cost the copy: 0.35 MB 80 us against 175, 2.8 MB 255 and 286,
-// 5.8 MB 480 and 400, 23 MB 1.7 and 1.1 ms, 92 MB 6 to 24 and 4 ms.  So pages that
+// 5.8 MB 480 and 400, 23 MB 1.7 and 1.1 ms, 92 MB 6 to 24 and 4 ms.  (The host
+// reads either at the same speed afterwards: 92 MB in 4.8 ms.)  So pages that
 // may be new are written up to kNewInPlace bytes, those that the caller's input or
 // touch_pages has mapped up to kMappedInPlace (11.5 MB just mapped: 92 us and 99;
 // 23 MB 165 and 157).
